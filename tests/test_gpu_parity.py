@@ -369,3 +369,32 @@ def test_index_ops_wide_structs(cuda, width):
     ok = bad >= 0
     e[ok] = src_h[bad[ok]]
     assert np.array_equal(to_host(dst), e.reshape(-1))
+
+
+@pytest.mark.parametrize("width", WIDTHS)
+def test_index_ops_default_route(cuda, width):
+    """The one-chunk row-form kernels as a plain call takes them: the last
+    struct of a chunk, the length where the unroll changes (2^16), a source
+    longer and one shorter than the indices, and out-of-range indices at
+    every position of a chunk."""
+    torch = cuda
+    for n, bound in [(1, 1), (31, 40), (65, 33), ((1 << 16), 5000), ((1 << 16) + 1, 70001), ((1 << 16) + 300, 1 << 16)]:
+        src_h = oracle.random_structs(max(n, bound), width, seed=width + n)
+        idx_h = oracle.uniform_indices(n, bound, n + 5).copy()
+        idx_h[::37] = [-1, bound, 0x7FFFFFFF, -0x80000000][n % 4]
+        ok = (idx_h >= 0) & (idx_h < bound)
+        expect = np.full((n, width), SENTINEL, np.uint8)
+        expect[ok] = src_h[idx_h[ok]]
+        src = to_dev(torch, src_h)
+        idx = torch.from_numpy(idx_h).cuda()
+        buf, start = guarded(torch, n * width)
+        tg.gather(buf[start:], src, bound, idx, n, width)
+        assert np.array_equal(check_guards(buf, start, n * width), expect.reshape(-1)), ("gather", n, bound)
+        perm_h = oracle.permutation(max(n, bound), 7)[:n].copy()
+        perm_h[::41] = bound + 1 if bound < n else -7
+        ok = (perm_h >= 0) & (perm_h < bound)
+        expect = np.full((bound, width), SENTINEL, np.uint8)
+        expect[perm_h[ok]] = src_h[:n][ok]
+        buf, start = guarded(torch, bound * width)
+        tg.scatter(buf[start:], bound, src, torch.from_numpy(perm_h).cuda(), n, width)
+        assert np.array_equal(check_guards(buf, start, bound * width), expect.reshape(-1)), ("scatter", n, bound)

@@ -346,12 +346,37 @@ static bool blocked_scatter_pays(uint32_t width, uint64_t n, uint64_t dst_n) {
     return width <= 16 && (long long)(dst_n * width) > kScatterPassBytes && 2 * n >= dst_n;
 }
 
-// Without a tuned entry, struct gathers and scatters take the row-form path
-// with 2 structs per lane, streaming index and contiguous side, and (gather)
-// random loads with the 64-byte L2 prefetch hint (policy 4): measured on
-// GB300 with L2 flushed, the best or within 1 % of the best at every width
-// from 8 to 64 bytes on permutations, runs of 32 and the identity.  Narrow
-// scatters onto large destinations run in destination passes (policy 6).
+// Structs per lane of the row-form kernels when the caller gives none.  A call
+// of at most 2^16 structs does not fill the GPU (2048 warps at one struct per
+// lane): more structs per lane only lengthen each warp (4096 structs of 28
+// bytes: 1.79 us at 1, 1.93 at 2, 2.43 at 4).  Above, one or two 4- or 8-byte
+// words in flight per lane are too few (2^24 structs of 4 bytes: gather 99 us
+// at 1, 80 at 2, 79 at 4; 2^20 of 8 bytes: 8.7 / 8.1 / 8.0 us; 2^20 of 12 to
+// 24 bytes: 2-6 % faster at 2 than at 1), while from 28 bytes up one struct
+// per lane is as fast or faster (2^20 of 36 bytes: 16.1 us at 1, 17.0 at 2).
+// Scatters gain from 2 up to 8 bytes only (2^20 of 8 bytes: 8.8 / 7.8 us; of
+// 24 bytes: 23.3 / 23.8).
+static int rows_unroll(bool gather, uint32_t width, uint64_t n) {
+    if (n <= (uint64_t(1) << 16)) return 1;
+    if (gather) return width <= 8 ? 4 : width <= 24 ? 2 : 1;
+    return width <= 8 ? 2 : 1;
+}
+
+// L2 fetch hint of a gather's random loads.  A source larger than L2 holds
+// (64 MiB and more) is fetched by 64-byte halves (policy 4): the rest of a
+// 128-byte line would leave L2 before another row of it is asked for.  A
+// source that fits and most of whose rows are read is fetched by whole lines
+// (policy 5), which brings the neighbouring rows in early: 2^20 rows of 64
+// bytes 25.0 us against 28.3 with 64-byte fetches, of 48 bytes 19.1 against
+// 20.0; below 32 bytes the two are within 3 %, and narrow rows keep policy 4.
+constexpr uint64_t kL2SourceBytes = uint64_t(64) << 20;
+static int gather_policy(uint32_t width, uint64_t n, uint64_t src_n) {
+    return width >= 32 && src_n * width <= kL2SourceBytes && 2 * n >= src_n ? 5 : 4;
+}
+
+// Without a tuned entry, struct gathers and scatters take the row-form path,
+// streaming the index and contiguous side.  Narrow scatters onto large
+// destinations run in destination passes (policy 6).
 static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound, const int32_t* idx, uint64_t n,
                         uint32_t width, const trv_launch* cfg, void* stream) {
     if (!size_ok(n, width) || !size_ok(bound, width)) return TRV_ERR_INVALID_ARGUMENT;
@@ -370,7 +395,9 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
                                    &t))
             c = trv_launch{t.path, t.unroll, 0, t.grid, 0, t.cache_policy};
         else if (structs)
-            c = trv_launch{TRV_PATH_WARP, 2, 0, 0, 0, gather ? 4 : blocked_scatter_pays(width, n, bound) ? 6 : 1};
+            c = gather                                    ? trv_launch{TRV_PATH_WARP, 0, 0, 0, 0, gather_policy(width, n, bound)}
+                : blocked_scatter_pays(width, n, bound) ? trv_launch{TRV_PATH_WARP, 2, 0, 0, 0, 6}
+                                                        : trv_launch{TRV_PATH_WARP, 0, 0, 0, 0, 1};
         else
             c.path = wide_words ? TRV_PATH_WARP : TRV_PATH_VECTOR;
     }
@@ -401,7 +428,9 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
     }
     if (!struct_width(width)) return TRV_ERR_UNSUPPORTED;
     if (!aligned(dst, 4) || !aligned(src, 4)) return TRV_ERR_MISALIGNED;
-    const int u = c.unroll > 0 ? c.unroll : default_unroll(width);
+    const int u = c.unroll > 0                ? c.unroll
+                  : path == TRV_PATH_WARP ? rows_unroll(gather, width, n)
+                                          : default_unroll(width);
     const int slot = unroll_slot(u);
     if (slot < 0) return TRV_ERR_INVALID_ARGUMENT;
     const WidthOps* ops = ops_for_words(int(width / 4));
@@ -415,7 +444,9 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
         kp = gather ? &ops->gather[mode][slot] : &ops->scatter[mode][slot];
     }
     const IndexKernel& k = *kp;
-    const int grid = grid_for(k.func, (long long)n, 256 * ops->built_unroll[slot], 256, grid_req);
+    int grid = 0;
+    const bool once = one_chunk_per_warp((long long)n, ops->built_unroll[slot], grid_req, &grid);
+    if (!once) grid = grid_for(k.func, (long long)n, 256 * ops->built_unroll[slot], 256, grid_req);
     if (!gather && path == TRV_PATH_WARP && c.cache_policy == 6) {  // destination passes
         const long long dst_bytes = (long long)bound * (long long)width;
         long long passes = (dst_bytes + kScatterPassBytes - 1) / kScatterPassBytes;
@@ -423,11 +454,12 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
         for (long long p = 0; p < passes; ++p) {
             IndexArgs a{src, dst, idx, (long long)n, (long long)bound * (p + 1) / passes, 1};
             a.lo = (long long)bound * p / passes;
+            a.once = once;
             k.launch(a, grid, 256, st);
         }
         return check_launch();
     }
-    k.launch(IndexArgs{src, dst, idx, (long long)n, (long long)bound, c.cache_policy}, grid, 256, st);
+    k.launch(IndexArgs{src, dst, idx, (long long)n, (long long)bound, c.cache_policy, 0, once}, grid, 256, st);
     return check_launch();
 }
 

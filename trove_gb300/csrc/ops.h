@@ -25,6 +25,7 @@ struct IndexArgs {
     long long bound;  // src_n for gather, dst_n for scatter
     int policy;       // cache policy of the row-form kernels
     long long lo = 0; // row-form scatter: only destinations in [lo, bound) are written
+    bool once = false; // the grid covers every 32*unroll-struct chunk with one warp
 };
 
 template <typename Args>

@@ -62,14 +62,43 @@ struct word_of<4> {
     typedef unsigned type;
 };
 
+// The random side's length as the unsigned bound of the one-chunk kernels.
+unsigned index_bound(long long n) { return n > 0x80000000ll ? 0x80000000u : unsigned(n); }
+
+// Default grids run the one-chunk kernels, built for the cache policies that
+// calls use in earnest; requested grids and policies 2 and 3 the grid-stride form.
+template <typename V, int U, int POL>
+void launch_gather_once(const IndexArgs& a, int grid, int block, cudaStream_t st) {
+    gather_rows_once_kernel<S, V, U, POL><<<grid, block, 0, st>>>(
+        static_cast<const V*>(a.src), index_bound(a.bound), a.idx, static_cast<V*>(a.dst), a.n);
+}
+
 template <typename V, int U>
 void launch_gather_rows(const IndexArgs& a, int grid, int block, cudaStream_t st) {
+    if (a.once) {
+        switch (a.policy) {
+            case 0: return launch_gather_once<V, U, 0>(a, grid, block, st);
+            case 1: return launch_gather_once<V, U, 1>(a, grid, block, st);
+            case 4: return launch_gather_once<V, U, 4>(a, grid, block, st);
+            case 5: return launch_gather_once<V, U, 5>(a, grid, block, st);
+        }
+    }
     gather_rows_kernel<S, V, U><<<grid, block, 0, st>>>(static_cast<const V*>(a.src), a.bound, a.idx,
                                                         static_cast<V*>(a.dst), a.n, a.policy);
 }
 
+template <typename V, int U, int POL>
+void launch_scatter_once(const IndexArgs& a, int grid, int block, cudaStream_t st) {
+    scatter_rows_once_kernel<S, V, U, POL><<<grid, block, 0, st>>>(
+        static_cast<const V*>(a.src), a.idx, static_cast<V*>(a.dst), index_bound(a.bound), a.n);
+}
+
 template <typename V, int U>
 void launch_scatter_rows(const IndexArgs& a, int grid, int block, cudaStream_t st) {
+    if (a.once && a.lo == 0) {
+        if (a.policy == 0) return launch_scatter_once<V, U, 0>(a, grid, block, st);
+        if (a.policy != 2 && a.policy != 3) return launch_scatter_once<V, U, 1>(a, grid, block, st);
+    }
     scatter_rows_kernel<S, V, U><<<grid, block, 0, st>>>(static_cast<const V*>(a.src), a.idx,
                                                          static_cast<V*>(a.dst), a.lo, a.bound, a.n, a.policy);
 }
