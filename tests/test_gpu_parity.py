@@ -398,3 +398,45 @@ def test_index_ops_default_route(cuda, width):
         buf, start = guarded(torch, bound * width)
         tg.scatter(buf[start:], bound, src, torch.from_numpy(perm_h).cuda(), n, width)
         assert np.array_equal(check_guards(buf, start, bound * width), expect.reshape(-1)), ("scatter", n, bound)
+
+
+@pytest.mark.parametrize("width,offset", [(4, 0), (8, 0), (12, 0), (28, 4), (32, 16), (36, 0), (48, 0), (60, 8)])
+def test_scatter_in_parts(cuda, width, offset):
+    """Scatters onto destinations that take two parts (64 MiB and a little
+    more) and one (just above 22 MiB): random and sorted indices, skipped ones
+    among them, a last slab of one struct, rows that nothing is written to."""
+    torch = cuda
+    for bound in ((64 << 20) // width + 77, (22 << 20) // width + 1):
+        n = (bound - 5) // 4096 * 4096 + 1
+        src_h = oracle.random_structs(n, width, seed=width)
+        src = torch.zeros(n * width + 64, dtype=torch.uint8, device="cuda")
+        src[offset:offset + n * width] = to_dev(torch, src_h)
+        perm = oracle.permutation(bound, width + 9)[:n].copy()
+        for idx_h in (perm, np.sort(perm)):
+            idx_h = idx_h.copy()
+            idx_h[::4099] = -1
+            idx_h[7::8191] = bound
+            ok = (idx_h >= 0) & (idx_h < bound)
+            expect = np.full((bound, width), SENTINEL, np.uint8)
+            expect[idx_h[ok]] = src_h[ok]
+            idx = torch.from_numpy(idx_h).cuda()
+            for kw in ({}, {"path": "warp", "policy": 6}):
+                buf, start = guarded(torch, bound * width, offset=offset)
+                tg.scatter(buf[start:], bound, src[offset:], idx, n, width, **kw)
+                assert np.array_equal(check_guards(buf, start, bound * width), expect.reshape(-1)), (bound, kw)
+
+
+@pytest.mark.parametrize("n", [1, 2, 33, 4097])
+def test_scatter_in_parts_short(cuda, n):
+    """The same policy asked for on arrays of any size, onto one row too."""
+    torch = cuda
+    for width, bound in [(12, n), (20, n + 9), (4, 1)]:
+        src_h = oracle.random_structs(n, width, seed=n)
+        idx_h = oracle.permutation(n, 3) if bound >= n else np.where(np.arange(n) == n // 2, 0, -1).astype(np.int32)
+        ok = (idx_h >= 0) & (idx_h < bound)
+        expect = np.full((bound, width), SENTINEL, np.uint8)
+        expect[idx_h[ok]] = src_h[ok]
+        buf, start = guarded(torch, bound * width)
+        tg.scatter(buf[start:], bound, to_dev(torch, src_h), torch.from_numpy(idx_h).cuda(), n, width, path="warp",
+                   policy=6)
+        assert np.array_equal(check_guards(buf, start, bound * width), expect.reshape(-1)), (n, width)

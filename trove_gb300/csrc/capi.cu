@@ -329,21 +329,39 @@ int32_t trv_copy_exit(void* dst, const void* src, uint64_t n, uint32_t width, ui
     return trv_copy_exit_ex(dst, src, n, width, modulus, &cfg, stream);
 }
 
-// Destination bytes one pass of a blocked scatter (cache policy 6) covers.
-// A random store of a struct narrower than a 32-byte sector is a partial-sector
-// write; when the destination is much larger than L2, the sector leaves L2
-// before its other structs arrive and DRAM must read, merge and write it.
-// Taking only the indices that land in one L2-sized part of the destination
-// per pass lets the partial writes merge in L2 (each pass re-reads the index
-// and source arrays).  Measured on 2^24-struct permutation scatters of the
-// row-form kernel: +53 / +33 / +23 % at 8 / 12 / 16 bytes (2-4 passes);
-// at 20 and 24 bytes the 5-6 passes cost more than they save (-25 / -16 %).
-constexpr long long kScatterPassBytes = 64ll << 20;
+// In how many parts a scatter writes its destination (scatter_parts.cu): 0, as
+// one plain pass; 1, one pass after the destination has been fetched into L2;
+// more, a pass for each part.  Measured on GB300 with random permutations:
+//  - rows that fill whole 32-byte sectors need no fill: one plain pass;
+//  - up to about 22 MiB of destination L2 absorbs the partial sectors (2^20 rows
+//    of 20 bytes, 20 MiB: 15.1 us, 18.4 with the fetch; of 24 bytes, 24 MiB:
+//    23.1 against 18.8), and 4-byte rows gain nothing from the fetch alone (2^24:
+//    103 against 104 us);
+//  - up to 64 MiB one pass is still best (2^24 rows of 4 bytes, 64 MiB: 104 us,
+//    114 in two; 3 * 2^20 of 20 bytes, 60 MiB: 49.4 and 55.0);
+//  - parts of 48, 56 and 64 MiB: 2^24 rows of 24 bytes 406 / 409 / 429 us, of 60
+//    bytes 931 / 916 / 927, 5 * 2^24 of 16 bytes 2921 / 2820 / 2848;
+//  - a pass costs about 1 ns per index whatever it writes, so many parts lose
+//    again: 5 * 2^24 rows of 20 bytes in 29 parts 3548 us against 3812 plain, of
+//    24 bytes in 35 parts 4053 against 3853;
+//  - a destination most of whose rows are not written would be fetched for
+//    nothing.
+constexpr uint64_t kPlainScatterBytes = uint64_t(22) << 20;
+constexpr uint64_t kOnePassBytes = uint64_t(64) << 20;
+constexpr uint64_t kPartBytes = uint64_t(56) << 20;
+constexpr uint64_t kMostParts = 24;
 
-// The blocked scatter pays for narrow structs whose destination exceeds a
-// pass and that most of the destination's rows receive.
-static bool blocked_scatter_pays(uint32_t width, uint64_t n, uint64_t dst_n) {
-    return width <= 16 && (long long)(dst_n * width) > kScatterPassBytes && 2 * n >= dst_n;
+static uint64_t parts_of(uint64_t bytes) {
+    return bytes <= kOnePassBytes ? 1 : (bytes + kPartBytes - 1) / kPartBytes;
+}
+
+static int scatter_parts(uint32_t width, uint64_t n, uint64_t dst_n, const void* dst) {
+    const uint64_t bytes = dst_n * width;
+    if (bytes <= kPlainScatterBytes || 2 * n < dst_n) return 0;
+    if (width % 32 == 0 && aligned(dst, 32)) return 0;
+    const uint64_t parts = parts_of(bytes);
+    if (parts > kMostParts || (parts == 1 && width < 8)) return 0;
+    return int(parts);
 }
 
 // Structs per lane of the row-form kernels when the caller gives none.  A call
@@ -375,8 +393,8 @@ static int gather_policy(uint32_t width, uint64_t n, uint64_t src_n) {
 }
 
 // Without a tuned entry, struct gathers and scatters take the row-form path,
-// streaming the index and contiguous side.  Narrow scatters onto large
-// destinations run in destination passes (policy 6).
+// streaming the index and contiguous side; scatters onto large destinations
+// run in parts (policy 6).
 static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound, const int32_t* idx, uint64_t n,
                         uint32_t width, const trv_launch* cfg, void* stream) {
     if (!size_ok(n, width) || !size_ok(bound, width)) return TRV_ERR_INVALID_ARGUMENT;
@@ -396,8 +414,8 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
             c = trv_launch{t.path, t.unroll, 0, t.grid, 0, t.cache_policy};
         else if (structs)
             c = gather                                    ? trv_launch{TRV_PATH_WARP, 0, 0, 0, 0, gather_policy(width, n, bound)}
-                : blocked_scatter_pays(width, n, bound) ? trv_launch{TRV_PATH_WARP, 2, 0, 0, 0, 6}
-                                                        : trv_launch{TRV_PATH_WARP, 0, 0, 0, 0, 1};
+                                                          : trv_launch{TRV_PATH_WARP, 0, 0, 0, 0,
+                                                                       scatter_parts(width, n, bound, dst) ? 6 : 1};
         else
             c.path = wide_words ? TRV_PATH_WARP : TRV_PATH_VECTOR;
     }
@@ -447,19 +465,19 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
     int grid = 0;
     const bool once = one_chunk_per_warp((long long)n, ops->built_unroll[slot], grid_req, &grid);
     if (!once) grid = grid_for(k.func, (long long)n, 256 * ops->built_unroll[slot], 256, grid_req);
-    if (!gather && path == TRV_PATH_WARP && c.cache_policy == 6) {  // destination passes
-        const long long dst_bytes = (long long)bound * (long long)width;
-        long long passes = (dst_bytes + kScatterPassBytes - 1) / kScatterPassBytes;
-        passes = passes < 1 ? 1 : passes > 16 ? 16 : passes;
-        for (long long p = 0; p < passes; ++p) {
-            IndexArgs a{src, dst, idx, (long long)n, (long long)bound * (p + 1) / passes, 1};
-            a.lo = (long long)bound * p / passes;
-            a.once = once;
+    if (!gather && path == TRV_PATH_WARP && c.cache_policy == 6 && n >= 2 && bound >= 1) {  // in parts
+        const IndexArgs a{src, dst, idx, (long long)n, (long long)bound, 1, once};
+        const uint64_t parts = std::min<uint64_t>(parts_of(bound * width), 64);
+        if (parts > 1) {
+            const int wb = kp == &ops->scatter_rows[0][slot] ? ops->rows_word_bytes : 4;
+            launch_scatter_passes(wb, a, int(width) / wb, int(parts), st);
+        } else {
+            launch_fetch_destination(a, int(width), st);
             k.launch(a, grid, 256, st);
         }
         return check_launch();
     }
-    k.launch(IndexArgs{src, dst, idx, (long long)n, (long long)bound, c.cache_policy, 0, once}, grid, 256, st);
+    k.launch(IndexArgs{src, dst, idx, (long long)n, (long long)bound, c.cache_policy, once}, grid, 256, st);
     return check_launch();
 }
 

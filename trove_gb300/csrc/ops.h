@@ -24,8 +24,7 @@ struct IndexArgs {
     long long n;
     long long bound;  // src_n for gather, dst_n for scatter
     int policy;       // cache policy of the row-form kernels
-    long long lo = 0; // row-form scatter: only destinations in [lo, bound) are written
-    bool once = false; // the grid covers every 32*unroll-struct chunk with one warp
+    bool once = false; // row-form kernels: the grid covers every 32*unroll-struct chunk with one warp
 };
 
 template <typename Args>
@@ -64,6 +63,12 @@ struct WidthOps {
 // width that is a multiple of 4 bytes.  word_bytes: 16, 8 or 4.
 void launch_index_rows_rt(bool gather, int word_bytes, const IndexArgs& a, int m, int grid, cudaStream_t st);
 const void* index_rows_rt_func(bool gather, int word_bytes);
+
+// Scatter onto a large destination (rows_rt.cu), any width that is a multiple
+// of 4 bytes, n >= 2: in `passes` parts of the destination (one launch), or the
+// fetch of the destination into L2 ahead of a scatter in one pass.
+void launch_scatter_passes(int word_bytes, const IndexArgs& a, int m, int passes, cudaStream_t st);
+void launch_fetch_destination(const IndexArgs& a, int row_bytes, cudaStream_t st);
 
 // Defined in width_ops.cu, one specialisation per translation unit.
 template <int S>

@@ -1,0 +1,226 @@
+// Scatters onto large destinations.
+//
+// A row that does not fill whole 32-byte sectors is a partial-sector write.
+// Scattered over a destination of more than about 22 MiB, each one makes L2
+// fill the rest of its sector from DRAM at the rate of random accesses, and
+// over one larger than L2 the sector leaves before its other rows arrive and
+// is filled and written again.  Two remedies:
+//  - the destination (or the part at hand) is fetched into L2 first, in
+//    address order at the full DRAM rate, so that the writes find their
+//    sectors (2^21 rows of 24 bytes: 52 -> 25 us plus the fetch);
+//  - a destination larger than L2 is written in parts that fit, one pass each.
+#include <cuda_runtime.h>
+
+#include "ops.h"
+
+namespace trv {
+namespace {
+
+// Loads of what a kernel reads once: 64-byte fetches, first to leave L2.
+__device__ __forceinline__ unsigned long long l2_evict_first_policy() {
+    unsigned long long pol;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+    return pol;
+}
+__device__ __forceinline__ uint4 ld_once(const uint4* p, unsigned long long pol) {
+    uint4 v;
+    asm volatile("ld.global.nc.L2::cache_hint.L2::64B.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p), "l"(pol));
+    return v;
+}
+__device__ __forceinline__ uint2 ld_once(const uint2* p, unsigned long long pol) {
+    uint2 v;
+    asm volatile("ld.global.nc.L2::cache_hint.L2::64B.v2.u32 {%0, %1}, [%2], %3;"
+                 : "=r"(v.x), "=r"(v.y)
+                 : "l"(p), "l"(pol));
+    return v;
+}
+__device__ __forceinline__ unsigned ld_once(const unsigned* p, unsigned long long pol) {
+    unsigned v;
+    asm volatile("ld.global.nc.L2::cache_hint.L2::64B.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));
+    return v;
+}
+__device__ __forceinline__ int ld_once(const int* p, unsigned long long pol) {
+    return int(ld_once(reinterpret_cast<const unsigned*>(p), pol));
+}
+
+// Whether indices mostly step from one row to the next (sorted, runs): then
+// the writes of neighbouring rows meet in L2 by themselves, and neither remedy
+// is needed.  Every warp takes the same 32 pairs of the index array, so every
+// warp of a launch comes to the same answer.
+struct IndexSample {
+    int a, b;
+    __device__ __forceinline__ IndexSample(const int* __restrict__ idx, long long n, int lane) {
+        const long long p = (long long)lane * (n - 1) >> 5;  // n >= 2
+        a = __ldg(idx + p);
+        b = __ldg(idx + p + 1);
+    }
+    __device__ __forceinline__ bool local(int row_bytes) const {
+        const long long d = (long long)b - a;
+        const bool near = (d < 0 ? -d : d) * row_bytes <= 256;
+        return __popc(__ballot_sync(0xFFFFFFFFu, near)) >= 20;
+    }
+};
+
+// Fetches [p0, p1) into L2: block c of `blocks`, 4 KiB an instruction.
+__device__ __forceinline__ void fetch_part(unsigned long long p0, unsigned long long p1, unsigned c, unsigned blocks) {
+    p0 = (p0 + 15) & ~15ull;
+    p1 &= ~15ull;
+    const unsigned long long step = (unsigned long long)blocks * blockDim.x * 4096;
+    for (unsigned long long p = p0 + ((unsigned long long)c * blockDim.x + threadIdx.x) * 4096; p < p1; p += step) {
+        const unsigned bytes = p1 - p < 4096 ? unsigned(p1 - p) : 4096u;
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+    }
+}
+
+// Ahead of a one-pass scatter: the whole destination.
+__global__ void __launch_bounds__(256)
+fetch_destination_kernel(const unsigned char* dst, long long bytes, const int* __restrict__ idx, long long n,
+                         int row_bytes) {
+    if (IndexSample(idx, n, int(threadIdx.x & 31u)).local(row_bytes)) return;
+    const unsigned long long p = reinterpret_cast<unsigned long long>(dst);
+    fetch_part(p, p + (unsigned long long)bytes, blockIdx.x, gridDim.x);
+}
+
+// Scatter in passes: pass p moves the rows whose index lies in the p-th part
+// of the destination.  One launch, the passes' blocks in order, so a pass
+// starts as the one before it drains; between two passes come the blocks that
+// fetch the next part.
+//
+// A warp reads the indices of a slab of kSlab structs (all loads in flight at
+// once), compacts the ones of its pass into a list in shared memory, and moves
+// the listed structs with every lane busy: word q = l + 32k of the list's
+// words is word q % m of struct list[q / m].  A pass so reads the index array
+// and its own share of the source, not the whole of both, and both are first
+// to leave L2, which keeps the part being written.
+//
+// Bound by DRAM: 2^24 random rows of 12 bytes in four passes move about 1.35 GB
+// in 233 us (one pass of the row-form kernel 544 us, three passes of it over
+// 64 MiB parts 380 us); of 24 bytes 406 us (one pass 717), of 48 bytes 682 us
+// (1147), of 60 bytes 916 us (1358).
+constexpr int kSlabRounds = 16;
+constexpr int kSlab = 32 * kSlabRounds;
+constexpr int kPassWarps = 8;
+
+struct PassPlan {
+    unsigned bound;          // rows of the destination
+    unsigned rows_per_pass;
+    unsigned passes;
+    unsigned body;           // blocks that move a pass's structs
+    unsigned fetch;          // blocks that fetch a part
+};
+
+template <typename V, int G>
+__global__ void __launch_bounds__(32 * kPassWarps)
+scatter_passes_kernel(const V* __restrict__ src, const int* __restrict__ idx, V* __restrict__ dst, long long n, int m,
+                      PassPlan plan) {
+    __shared__ int s_to[kPassWarps][kSlab];
+    __shared__ unsigned short s_at[kPassWarps][kSlab];
+    const int lane = int(threadIdx.x & 31u), warp = int(threadIdx.x >> 5);
+    const unsigned long long row = (unsigned long long)m * sizeof(V);
+    const IndexSample sample(idx, n, lane);
+    const unsigned pass = blockIdx.x / (plan.fetch + plan.body);
+    unsigned c = blockIdx.x - pass * (plan.fetch + plan.body);
+    unsigned lo = pass * plan.rows_per_pass;
+    unsigned rows = plan.bound - lo < plan.rows_per_pass ? plan.bound - lo : plan.rows_per_pass;
+    const bool local = sample.local(int(row));
+    if (local) {  // one pass over everything
+        if (pass != 0) return;
+        rows = plan.bound;
+    }
+    if (c < plan.fetch) {
+        const unsigned long long p = reinterpret_cast<unsigned long long>(dst) + lo * row;
+        if (!local) fetch_part(p, p + rows * row, c, plan.fetch);
+        return;
+    }
+    c -= plan.fetch;
+    const unsigned long long pol = l2_evict_first_policy();
+    const int step_j = 32 / m, step_r = 32 % m;
+    int* to = s_to[warp];
+    unsigned short* at = s_at[warp];
+    for (long long base = ((long long)c * kPassWarps + warp) * kSlab; base < n;
+         base += (long long)plan.body * kPassWarps * kSlab) {
+        const int rem = n - base < kSlab ? int(n - base) : kSlab;
+        int v[kSlabRounds];
+#pragma unroll
+        for (int t = 0; t < kSlabRounds; ++t) v[t] = t * 32 + lane < rem ? ld_once(idx + base + t * 32 + lane, pol) : -1;
+        int cnt = 0;
+        __syncwarp();  // the previous slab's list has been read
+#pragma unroll
+        for (int t = 0; t < kSlabRounds; ++t) {
+            const bool mine = unsigned(v[t]) - lo < rows;  // a negative index is 2^31 or more, lo + rows at most 2^31
+            const unsigned b = __ballot_sync(0xFFFFFFFFu, mine);
+            if (mine) {
+                const int k = cnt + __popc(b & ((1u << lane) - 1u));
+                to[k] = v[t];
+                at[k] = (unsigned short)(t * 32 + lane);
+            }
+            cnt += __popc(b);
+        }
+        __syncwarp();
+        const V* from = src + base * m;
+        const int words = cnt * m;
+        int j = lane / m, r = lane % m;
+        for (int q = lane; q < words; q += 32 * G) {
+            V val[G];
+            V* out[G];
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                out[g] = nullptr;
+                if (q + 32 * g < words) {
+                    val[g] = ld_once(from + unsigned(at[j]) * unsigned(m) + r, pol);
+                    out[g] = dst + (long long)to[j] * m + r;
+                }
+                j += step_j;
+                r += step_r;
+                if (r >= m) {
+                    r -= m;
+                    ++j;
+                }
+            }
+#pragma unroll
+            for (int g = 0; g < G; ++g)
+                if (out[g]) *out[g] = val[g];
+        }
+    }
+}
+
+constexpr int kFetchBlocks = 64;
+// Blocks that move a pass's structs, at most (more slabs run in a loop): few
+// enough to leave quickly where the indices are local, enough that two passes
+// overlap only briefly.  2^24 / 3 * 2^24 random rows of 24 bytes: 458 / 2073 us
+// at 608 (one resident wave), 406 / 1840 at 2048, 395 / 1793 at 4096; 2^24
+// sorted rows of 48 bytes: 264 / 277 / 331 us.
+constexpr int kBodyBlocks = 2048;
+
+template <typename V, int G>
+void launch_passes(const IndexArgs& a, int m, int passes, cudaStream_t st) {
+    const unsigned bound = a.bound > 0x80000000ll ? 0x80000000u : unsigned(a.bound);
+    PassPlan p;
+    p.bound = bound;
+    p.rows_per_pass = unsigned((bound + (long long)passes - 1) / passes);
+    p.passes = (bound + p.rows_per_pass - 1) / p.rows_per_pass;
+    const long long slabs = (a.n + kSlab * kPassWarps - 1) / (kSlab * kPassWarps);
+    p.body = unsigned(slabs < kBodyBlocks ? slabs : kBodyBlocks);
+    p.fetch = kFetchBlocks;
+    scatter_passes_kernel<V, G><<<p.passes * (p.fetch + p.body), 32 * kPassWarps, 0, st>>>(
+        static_cast<const V*>(a.src), a.idx, static_cast<V*>(a.dst), a.n, m, p);
+}
+}  // namespace
+
+void launch_fetch_destination(const IndexArgs& a, int row_bytes, cudaStream_t st) {
+    fetch_destination_kernel<<<kFetchBlocks, 256, 0, st>>>(static_cast<const unsigned char*>(a.dst),
+                                                           a.bound * row_bytes, a.idx, a.n, row_bytes);
+}
+
+void launch_scatter_passes(int word_bytes, const IndexArgs& a, int m, int passes, cudaStream_t st) {
+    if (word_bytes == 16)
+        launch_passes<uint4, 4>(a, m, passes, st);
+    else if (word_bytes == 8)
+        launch_passes<uint2, 8>(a, m, passes, st);
+    else
+        launch_passes<unsigned, 8>(a, m, passes, st);
+}
+
+}  // namespace trv

@@ -95,12 +95,12 @@ void launch_scatter_once(const IndexArgs& a, int grid, int block, cudaStream_t s
 
 template <typename V, int U>
 void launch_scatter_rows(const IndexArgs& a, int grid, int block, cudaStream_t st) {
-    if (a.once && a.lo == 0) {
+    if (a.once) {
         if (a.policy == 0) return launch_scatter_once<V, U, 0>(a, grid, block, st);
         if (a.policy != 2 && a.policy != 3) return launch_scatter_once<V, U, 1>(a, grid, block, st);
     }
     scatter_rows_kernel<S, V, U><<<grid, block, 0, st>>>(static_cast<const V*>(a.src), a.idx,
-                                                         static_cast<V*>(a.dst), a.lo, a.bound, a.n, a.policy);
+                                                         static_cast<V*>(a.dst), a.bound, a.n, a.policy);
 }
 
 template <typename V, int k>
