@@ -440,3 +440,12 @@ def test_scatter_in_parts_short(cuda, n):
         tg.scatter(buf[start:], bound, to_dev(torch, src_h), torch.from_numpy(idx_h).cuda(), n, width, path="warp",
                    policy=6)
         assert np.array_equal(check_guards(buf, start, bound * width), expect.reshape(-1)), (n, width)
+
+
+def test_default_stream_is_torchs_current_one(cuda):
+    torch = cuda
+    assert tg._stream(None) == torch.cuda.current_stream().cuda_stream
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        assert tg._stream(None) == side.cuda_stream != 0
+    assert tg._stream(None) == torch.cuda.current_stream().cuda_stream

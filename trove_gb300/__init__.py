@@ -184,9 +184,12 @@ def _addr(x) -> int:
 
 def _stream(stream) -> int:
     if stream is None:
+        # The current stream's handle alone: asking whether CUDA is available and
+        # building a Stream object took 4.7 of the 8.1 us of a call (an
+        # initialised torch.cuda is an available one).
         torch = sys.modules.get("torch")
-        if torch is not None and torch.cuda.is_available() and torch.cuda.is_initialized():
-            return int(torch.cuda.current_stream().cuda_stream)
+        if torch is not None and torch.cuda.is_initialized():
+            return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
         return 0
     if isinstance(stream, int):
         return stream
