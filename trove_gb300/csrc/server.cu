@@ -123,14 +123,26 @@ struct Slot {
     size_t n_small = 0;                // ids[0, n_small) complete at done_small (0: one launch)
     bool small_done = false;
     cudaError_t small_q = cudaErrorNotReady, done_q = cudaErrorNotReady;  // what the last poll saw
-    BatchTask* d_tasks = nullptr;
-    long long* d_prefix = nullptr;
-    unsigned long long* d_counter = nullptr;
-    BatchTask* h_tasks = nullptr;  // pinned staging
-    long long* h_prefix = nullptr;
+    unsigned char* d_tables = nullptr;
+    unsigned char* h_tables = nullptr;  // pinned staging
     std::vector<uint64_t> ids;
     std::vector<std::pair<trv_request, uint64_t>> todo;  // the batch's requests, offset of each one's output
     bool busy = false;
+};
+
+// A batch's tables lie in one block, so that one copy brings them to the
+// device: two work counters (zero), the small and the large requests' tile
+// prefixes, the task table.
+struct Tables {
+    unsigned long long* counter;
+    long long* prefix;  // of the small requests; the large ones' follows
+    BatchTask* tasks;
+    static size_t tasks_at(size_t take) { return (16 + (take + 2) * sizeof(long long) + 15) / 16 * 16; }
+    static size_t bytes(size_t take) { return tasks_at(take) + take * sizeof(BatchTask); }
+    Tables(unsigned char* p, size_t take)
+        : counter(reinterpret_cast<unsigned long long*>(p)),
+          prefix(reinterpret_cast<long long*>(p + 16)),
+          tasks(reinterpret_cast<BatchTask*>(p + tasks_at(take))) {}
 };
 
 uint64_t request_bytes(const trv_request& r) {
@@ -253,7 +265,6 @@ struct trv_server {
     // its tables are written and its copies and kernels are launched (about 20
     // microseconds that every submission used to wait for).
     void launch_ready() {
-        const size_t stride = size_t(cfg.max_batch_requests) + 1;  // second prefix array
         for (Slot& s : slots) {
             if (s.busy) continue;
             size_t take, ns;
@@ -282,6 +293,7 @@ struct trv_server {
                 }
                 ++batches;
             }
+            const Tables h(s.h_tables, take), d(s.d_tables, take);
             long long tiles[2] = {0, 0};
             for (size_t k = 0; k < take; ++k) {
                 const trv_request& r = s.todo[k].first;
@@ -296,34 +308,27 @@ struct trv_server {
                 p.scatter_policy = 5;
                 p.copy_bulk = 1;
                 const long long nt = plan_task(r.op, r.width, r.n, r.src_n, r.src, arena.base() + s.todo[k].second,
-                                               r.idx, p, &s.h_tasks[k]);
+                                               r.idx, p, &h.tasks[k]);
                 const int grp = k < ns ? 0 : 1;
-                long long* pre = s.h_prefix + (grp ? stride : 0);
-                pre[grp ? k - ns : k] = tiles[grp];
+                h.prefix[k + size_t(grp)] = tiles[grp];
                 tiles[grp] += nt;
             }
-            s.h_prefix[ns] = tiles[0];
-            s.h_prefix[stride + (take - ns)] = tiles[1];
-            cudaError_t e = cudaMemcpyAsync(s.d_tasks, s.h_tasks, sizeof(BatchTask) * take, cudaMemcpyHostToDevice,
+            h.prefix[ns] = tiles[0];
+            h.prefix[take + 1] = tiles[1];
+            h.counter[0] = h.counter[1] = 0;
+            cudaError_t e = cudaMemcpyAsync(s.d_tables, s.h_tables, Tables::bytes(take), cudaMemcpyHostToDevice,
                                             s.stream);
-            if (e == cudaSuccess)
-                e = cudaMemcpyAsync(s.d_prefix, s.h_prefix, sizeof(long long) * (ns + 1), cudaMemcpyHostToDevice,
-                                    s.stream);
-            if (e == cudaSuccess)
-                e = cudaMemcpyAsync(s.d_prefix + stride, s.h_prefix + stride, sizeof(long long) * (take - ns + 1),
-                                    cudaMemcpyHostToDevice, s.stream);
-            if (e == cudaSuccess) e = cudaMemsetAsync(s.d_counter, 0, 2 * sizeof(unsigned long long), s.stream);
             const bool two = ns > 0 && ns < take;
             int launches = 0;
             if (e == cudaSuccess && ns > 0 && tiles[0] > 0) {
                 const int g = tiles[0] < grid ? int(tiles[0]) : grid;
-                e = launch_batch_kernel(s.d_tasks, int(ns), s.d_prefix, s.d_counter, g, kServerBlocksPerSm, s.stream);
+                e = launch_batch_kernel(d.tasks, int(ns), d.prefix, d.counter, g, kServerBlocksPerSm, s.stream);
                 ++launches;
             }
             if (e == cudaSuccess && two) e = cudaEventRecord(s.done_small, s.stream);
             if (e == cudaSuccess && ns < take && tiles[1] > 0) {
                 const int g = tiles[1] < grid_large ? int(tiles[1]) : grid_large;
-                e = launch_batch_kernel(s.d_tasks + ns, int(take - ns), s.d_prefix + stride, s.d_counter + 1, g,
+                e = launch_batch_kernel(d.tasks + ns, int(take - ns), d.prefix + ns + 1, d.counter + 1, g,
                                         kServerBlocksPerSm, s.stream);
                 ++launches;
             }
@@ -382,11 +387,8 @@ void free_slot(Slot& s) {
     if (s.stream) cudaStreamDestroy(s.stream);
     if (s.done) cudaEventDestroy(s.done);
     if (s.done_small) cudaEventDestroy(s.done_small);
-    if (s.d_tasks) cudaFree(s.d_tasks);
-    if (s.d_prefix) cudaFree(s.d_prefix);
-    if (s.d_counter) cudaFree(s.d_counter);
-    if (s.h_tasks) cudaFreeHost(s.h_tasks);
-    if (s.h_prefix) cudaFreeHost(s.h_prefix);
+    if (s.d_tables) cudaFree(s.d_tables);
+    if (s.h_tables) cudaFreeHost(s.h_tables);
     s = Slot();
 }
 
@@ -449,12 +451,8 @@ static int32_t server_create_impl(const trv_server_config* cfg, trv_server** out
         cudaError_t e = cudaStreamCreateWithFlags(&sl.stream, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sl.done_small, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaMalloc(&sl.d_tasks, sizeof(BatchTask) * nt);
-        // two prefix arrays and two work counters: a batch's small and large requests
-        if (e == cudaSuccess) e = cudaMalloc(&sl.d_prefix, 2 * sizeof(long long) * (nt + 1));
-        if (e == cudaSuccess) e = cudaMalloc(&sl.d_counter, 2 * sizeof(unsigned long long));
-        if (e == cudaSuccess) e = cudaMallocHost(&sl.h_tasks, sizeof(BatchTask) * nt);
-        if (e == cudaSuccess) e = cudaMallocHost(&sl.h_prefix, 2 * sizeof(long long) * (nt + 1));
+        if (e == cudaSuccess) e = cudaMalloc(&sl.d_tables, Tables::bytes(nt));
+        if (e == cudaSuccess) e = cudaMallocHost(&sl.h_tables, Tables::bytes(nt));
         if (e != cudaSuccess) {
             cudaGetLastError();
             for (Slot& x : s->slots) free_slot(x);
