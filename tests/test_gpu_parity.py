@@ -449,3 +449,39 @@ def test_default_stream_is_torchs_current_one(cuda):
     with torch.cuda.stream(side):
         assert tg._stream(None) == side.cuda_stream != 0
     assert tg._stream(None) == torch.cuda.current_stream().cuda_stream
+
+
+@pytest.mark.parametrize("width", [5, 6, 7, 12, 13, 20, 31, 47, 64, 65, 217])
+def test_index_ops_packed(cuda, width):
+    """Rows of any width at any alignment: chunk and array ends, skipped rows,
+    the lengths and widths where the route changes, source and destination at
+    every offset from a word boundary; bytes around the arrays stay."""
+    torch = cuda
+    lengths = [1, 9, 33, 131, 70001] + ([(1 << 19) + 77] if width < 20 else [])
+    for n in lengths:
+        for bound in (n + 3, max(1, n - n // 3)):
+            rows = max(n, bound)
+            src_h = np.frombuffer(oracle.random_words((rows * width + 3) // 4, n).tobytes()[:rows * width], np.uint8)
+            src_h = src_h.reshape(rows, width)
+            uni = oracle.uniform_indices(n, bound, n + 1).copy()
+            perm = oracle.permutation(rows, 3)[:n].copy()
+            for soff, doff in [(1, 0), (0, 3), (2, 1), (3, 2)] if n < 1000 else [(1, 3)]:
+                src = torch.zeros(rows * width + 8, dtype=torch.uint8, device="cuda")
+                src[soff:soff + rows * width] = to_dev(torch, src_h)
+                for skip in (False, True):
+                    if skip:
+                        uni[::5] = -1
+                        perm[::5] = bound
+                    buf, start = guarded(torch, n * width, offset=doff)
+                    tg.gather(buf[start:], src[soff:], bound, torch.from_numpy(uni).cuda(), n, width)
+                    ok = uni >= 0
+                    expect = np.full((n, width), SENTINEL, np.uint8)
+                    expect[ok] = src_h[uni[ok]]
+                    assert np.array_equal(check_guards(buf, start, n * width), expect.reshape(-1)), (n, bound, soff, doff)
+                    buf, start = guarded(torch, bound * width, offset=doff)
+                    tg.scatter(buf[start:], bound, src[soff:], torch.from_numpy(perm).cuda(), n, width)
+                    ok = perm < bound
+                    expect = np.full((bound, width), SENTINEL, np.uint8)
+                    expect[perm[ok]] = src_h[:n][ok]
+                    assert np.array_equal(check_guards(buf, start, bound * width), expect.reshape(-1)), (n, bound, soff,
+                                                                                                         doff)

@@ -33,6 +33,13 @@ void launch_flat_copy(const void* src, void* dst, long long nbytes, int vec_byte
                       int grid, cudaStream_t st);
 const void* flat_copy_func(int vec_bytes, int unroll);
 
+// Gather / scatter of structs of `width` bytes (at most kMostPackedWidth) at any
+// alignment (packed.cu).  grid 0: one chunk per warp.
+constexpr unsigned kMostPackedWidth = 1u << 20;
+void launch_index_packed(bool gather, const void* src, const int* idx, void* dst, long long bound, long long n,
+                         int width, int grid, cudaStream_t st);
+
+// The same byte by byte, one thread to a row: wider structs.
 void launch_gather_bytes(const void* src, long long src_n, const int* idx, void* dst, long long n,
                          unsigned width, int grid, cudaStream_t st);
 void launch_scatter_bytes(const void* src, const int* idx, void* dst, long long dst_n, long long n,

@@ -1,0 +1,271 @@
+// Gather / scatter of structs of any width at any alignment (packed records:
+// 3, 6, 13 bytes, or 4-byte widths at odd addresses), in 4-byte words.
+//
+// The contiguous side is dealt out by aligned 32-bit words, so a warp reads or
+// writes whole sectors of it; the four bytes of a word come from one row, or
+// where it straddles a row's end from two (or more, below 4 bytes a row).  The
+// random side is read as the aligned words that hold the bytes, joined by a
+// funnel shift.  Bytes that no full word covers (a row's ends on the random
+// side of a scatter, skipped rows, the ends of the arrays) move one by one, and
+// no word is read that is not wholly inside the source array.
+//
+// One thread per row moving bytes was bound by its load / store instructions,
+// each touching 32 rows: 2^22 rows of 13 bytes, gather 153 us (10 % of DRAM's
+// rate) -> 46, scatter 446 -> 113; of 47 bytes 1252 -> 137 and 1604 -> 252.
+// What is left is the instructions of the joins, about 30 a word.
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "flat.h"
+
+namespace trv {
+namespace {
+
+constexpr int kWarps = 8;
+constexpr int kFly = 4;     // words of a lane in flight
+
+__device__ __forceinline__ unsigned ld_word(const unsigned char* p) {
+    unsigned v;
+    asm volatile("ld.global.nc.L2::64B.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
+// The `need` (1 to 4) bytes at p in the low end of a word; what lies above them
+// is undefined.  [lo, hi) is the array that p points into.
+__device__ __forceinline__ unsigned ld_bytes(const unsigned char* p, int need, const unsigned char* lo,
+                                             const unsigned char* hi) {
+    const unsigned off = unsigned(reinterpret_cast<uintptr_t>(p)) & 3u;
+    const unsigned char* a = p - off;
+    const bool two = off + unsigned(need) > 4u;
+    if (a >= lo && a + (two ? 8 : 4) <= hi) {
+        const unsigned w0 = ld_word(a);
+        const unsigned w1 = two ? ld_word(a + 4) : 0u;
+        return __funnelshift_r(w0, w1, off * 8u);
+    }
+    unsigned v = 0;
+    for (int b = 0; b < need; ++b) v |= unsigned(p[b]) << (8 * b);
+    return v;
+}
+
+// The same, skipped where `want` is false, with nothing checked.
+__device__ __forceinline__ void ld_word_if(unsigned& v, const unsigned char* p, bool want) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\t@p ld.global.nc.L2::64B.u32 %0, [%1];\n\t}"
+                 : "+r"(v)
+                 : "l"(p), "r"(int(want)));
+}
+
+// One warp: the destination bytes of kRows rows at a time, as the aligned words
+// inside them and up to 3 bytes at either end.
+template <int kRows>
+__global__ void __launch_bounds__(32 * kWarps)
+gather_packed_kernel(const unsigned char* __restrict__ src, unsigned bound, const int* __restrict__ idx,
+                     unsigned char* __restrict__ dst, long long n, int width) {
+    __shared__ int s_id[kWarps][kRows + 1];
+    const int lane = int(threadIdx.x & 31u), warp = int(threadIdx.x >> 5);
+    const unsigned char* hi = src + (unsigned long long)bound * unsigned(width);
+    // the same for every chunk: kRows rows are a multiple of 4 bytes
+    const int head = int((4u - (reinterpret_cast<uintptr_t>(dst) & 3u)) & 3u);
+    const int bytes = kRows * width, tail = (bytes - head) & 3, words = (bytes - head) / 4;
+    const int step_j = 128 / width, step_r = 128 % width;
+    int* id = s_id[warp];
+    if (lane == 0) id[kRows] = -1;  // read, never used
+    for (long long base = ((long long)blockIdx.x * kWarps + warp) * kRows; base < n;
+         base += (long long)gridDim.x * kWarps * kRows) {
+        __syncwarp();
+        bool inner = true;  // every row valid, and its words inside the array whatever its alignment
+#pragma unroll
+        for (int t = 0; t < kRows; t += 32) {
+            if (kRows < 32 && lane >= kRows) break;
+            const int v = base + t + lane < n ? __ldcs(idx + base + t + lane) : -1;
+            id[t + lane] = unsigned(v) < bound ? v : -1;
+            inner &= v >= 1 && (long long)v + 3 <= (long long)bound;
+        }
+        __syncwarp();
+        inner = __all_sync(0xFFFFFFFFu, inner);
+        unsigned char* out = dst + base * width;
+        if (lane < head + tail) {  // the ends, byte by byte
+            const int o = lane < head ? lane : bytes - tail + lane - head;
+            const int v = id[o / width];
+            if (v >= 0) out[o] = src[(long long)v * width + o % width];
+        }
+        out += head;
+        int j = (head + 4 * lane) / width;
+        int r = head + 4 * lane - j * width;
+        if (inner) {
+            for (int q = lane; q < words; q += 32 * kFly) {
+                unsigned w0[kFly], w1[kFly], w2[kFly], w3[kFly], at0[kFly], at1[kFly], cut[kFly];
+#pragma unroll
+                for (int f = 0; f < kFly; ++f) {
+                    const bool in = q + 32 * f < words;
+                    const int row = in ? j : 0, have = width - r;
+                    const unsigned char* p0 = src + (unsigned long long)unsigned(id[row]) * unsigned(width) + unsigned(r);
+                    const unsigned char* p1 = src + (unsigned long long)unsigned(id[row + 1]) * unsigned(width);
+                    const unsigned o0 = unsigned(reinterpret_cast<uintptr_t>(p0)) & 3u;
+                    const unsigned o1 = unsigned(reinterpret_cast<uintptr_t>(p1)) & 3u;
+                    const bool straddles = have < 4;
+                    w0[f] = w1[f] = w2[f] = w3[f] = 0;
+                    ld_word_if(w0[f], p0 - o0, in);
+                    ld_word_if(w1[f], p0 - o0 + 4, in && int(o0) + (straddles ? have : 4) > 4);
+                    ld_word_if(w2[f], p1 - o1, in && straddles);
+                    ld_word_if(w3[f], p1 - o1 + 4, in && straddles && int(o1) > have);
+                    at0[f] = o0 * 8;
+                    at1[f] = o1 * 8;
+                    cut[f] = straddles ? unsigned(32 - 8 * have) : 0u;
+                    j += step_j;
+                    r += step_r;
+                    if (r >= width) {
+                        r -= width;
+                        ++j;
+                    }
+                }
+#pragma unroll
+                for (int f = 0; f < kFly; ++f) {
+                    // the first row's bytes below the second's
+                    const unsigned v0 = __funnelshift_r(w0[f], w1[f], at0[f]);
+                    const unsigned v1 = __funnelshift_r(w2[f], w3[f], at1[f]);
+                    if (q + 32 * f < words)
+                        __stcs(reinterpret_cast<unsigned*>(out) + q + 32 * f, __funnelshift_r(v0 << cut[f], v1, cut[f]));
+                }
+            }
+            continue;
+        }
+        for (int q = lane; q < words; q += 32) {
+            unsigned val = 0, keep = 0;  // keep: the bytes to write, as a mask
+            const int first = id[j], have = width - r < 4 ? width - r : 4;
+            if (first >= 0) {
+                val = ld_bytes(src + (long long)first * width + r, have, src, hi);
+                keep = 0xFFFFFFFFu >> (8 * (4 - have));
+            }
+            if (have < 4) {
+                const int second = id[j + 1];
+                if (second >= 0) {
+                    const unsigned v = ld_bytes(src + (long long)second * width, 4 - have, src, hi);
+                    val = (val & keep) | (v << (8 * have));
+                    keep |= 0xFFFFFFFFu << (8 * have);
+                }
+            }
+            if (keep == 0xFFFFFFFFu) {
+                __stcs(reinterpret_cast<unsigned*>(out) + q, val);
+            } else if (keep) {
+                for (int b = 0; b < 4; ++b)
+                    if ((keep >> (8 * b)) & 1u) out[4 * q + b] = (unsigned char)(val >> (8 * b));
+            }
+            j += step_j;
+            r += step_r;
+            if (r >= width) {
+                r -= width;
+                ++j;
+            }
+        }
+    }
+}
+
+// One warp: kRows source rows, each as the `slots` aligned words of its
+// destination row; slot k of a row that starts c bytes past a 4-byte boundary
+// holds its bytes 4k - c to 4k - c + 3.
+template <int kRows>
+__global__ void __launch_bounds__(32 * kWarps)
+scatter_packed_kernel(const unsigned char* __restrict__ src, const int* __restrict__ idx,
+                      unsigned char* __restrict__ dst, unsigned bound, long long n, int width) {
+    __shared__ int s_id[kWarps][kRows];
+    const int lane = int(threadIdx.x & 31u), warp = int(threadIdx.x >> 5);
+    const unsigned char* hi = src + n * (long long)width;
+    const int slots = (width + 6) / 4;
+    const int step_j = 32 / slots, step_k = 32 % slots;
+    int* id = s_id[warp];
+    for (long long base = ((long long)blockIdx.x * kWarps + warp) * kRows; base < n;
+         base += (long long)gridDim.x * kWarps * kRows) {
+        __syncwarp();
+#pragma unroll
+        for (int t = 0; t < kRows; t += 32) {
+            if (kRows < 32 && lane >= kRows) break;
+            const int v = base + t + lane < n ? __ldcs(idx + base + t + lane) : -1;
+            id[t + lane] = unsigned(v) < bound ? v : -1;
+        }
+        __syncwarp();
+        const unsigned char* from = src + base * width;
+        const int rows = n - base < kRows ? int(n - base) : kRows;
+        const bool inner = base > 0 && base + rows + 2 <= n;  // words that reach past the rows are inside the array
+        int j = lane / slots, k = lane % slots;
+        while (j < rows) {
+            unsigned w0[kFly], w1[kFly];
+            unsigned at[kFly];
+            unsigned char* out[kFly];
+            int o[kFly];  // the row's byte at the word's start; nothing to write: `width`
+#pragma unroll
+            for (int f = 0; f < kFly; ++f) {
+                const int v = j < rows ? id[j] : -1;
+                unsigned char* d = dst + (unsigned long long)unsigned(v) * unsigned(width);
+                o[f] = v >= 0 ? 4 * k - int(reinterpret_cast<uintptr_t>(d) & 3u) : width;
+                out[f] = d + o[f];
+                const unsigned char* p = from + (long long)(j * width) + o[f];
+                const bool some = o[f] < width;
+                if (inner) {
+                    at[f] = (unsigned(reinterpret_cast<uintptr_t>(p)) & 3u) * 8;
+                    w0[f] = w1[f] = 0;
+                    ld_word_if(w0[f], p - (reinterpret_cast<uintptr_t>(p) & 3u), some);
+                    ld_word_if(w1[f], p - (reinterpret_cast<uintptr_t>(p) & 3u) + 4, some && at[f] != 0);
+                } else {
+                    const int skip = o[f] < 0 ? -o[f] : 0;
+                    const int last = width - o[f] < 4 ? width - o[f] : 4;
+                    at[f] = 0;
+                    if (skip < last) w0[f] = ld_bytes(p + skip, last - skip, src, hi) << (8 * skip);
+                }
+                j += step_j;
+                k += step_k;
+                if (k >= slots) {
+                    k -= slots;
+                    ++j;
+                }
+            }
+#pragma unroll
+            for (int f = 0; f < kFly; ++f) {
+                const unsigned val = inner ? __funnelshift_r(w0[f], w1[f], at[f]) : w0[f];
+                if (o[f] >= 0 && o[f] + 4 <= width) {
+                    *reinterpret_cast<unsigned*>(out[f]) = val;
+                } else {
+#pragma unroll
+                    for (int b = 0; b < 4; ++b)
+                        if (unsigned(o[f] + b) < unsigned(width)) out[f][b] = (unsigned char)(val >> (8 * b));
+                }
+            }
+        }
+    }
+}
+
+unsigned clamp_bound(long long n) { return n > 0x80000000ll ? 0x80000000u : unsigned(n); }
+
+}  // namespace
+
+template <bool GATHER, int ROWS>
+static void launch(const void* src, const int* idx, void* dst, long long bound, long long n, int width, int grid,
+                   cudaStream_t st) {
+    const unsigned char* s = static_cast<const unsigned char*>(src);
+    unsigned char* d = static_cast<unsigned char*>(dst);
+    if (grid <= 0) {
+        const long long need = (n + kWarps * ROWS - 1) / (kWarps * ROWS);
+        grid = need < 0x7FFFFFFFll ? int(need) : 0x7FFFFFFF;
+    }
+    if (GATHER)
+        gather_packed_kernel<ROWS><<<grid, 32 * kWarps, 0, st>>>(s, clamp_bound(bound), idx, d, n, width);
+    else
+        scatter_packed_kernel<ROWS><<<grid, 32 * kWarps, 0, st>>>(s, idx, d, clamp_bound(bound), n, width);
+}
+
+void launch_index_packed(bool gather, const void* src, const int* idx, void* dst, long long bound, long long n,
+                         int width, int grid, cudaStream_t st) {
+    // 128 rows are a whole number of 32-word rounds at any width; where the
+    // rows are few or wide, fewer to a warp keep more warps busy (gathers, us,
+    // at 8 / 32 rows: 2^16 of 217 bytes 15.4 / 40.3, 2^22 of them 553 / 472).
+    if (n < (width > 64 ? 1ll << 19 : 1ll << 15))
+        gather ? launch<true, 8>(src, idx, dst, bound, n, width, grid, st)
+               : launch<false, 8>(src, idx, dst, bound, n, width, grid, st);
+    else if (width > 64 || n < (1ll << 17))
+        gather ? launch<true, 32>(src, idx, dst, bound, n, width, grid, st)
+               : launch<false, 32>(src, idx, dst, bound, n, width, grid, st);
+    else
+        gather ? launch<true, 128>(src, idx, dst, bound, n, width, grid, st)
+               : launch<false, 128>(src, idx, dst, bound, n, width, grid, st);
+}
+
+}  // namespace trv
