@@ -485,3 +485,21 @@ def test_index_ops_packed(cuda, width):
                     expect[perm[ok]] = src_h[:n][ok]
                     assert np.array_equal(check_guards(buf, start, bound * width), expect.reshape(-1)), (n, bound, soff,
                                                                                                          doff)
+
+
+@pytest.mark.parametrize("shift", range(1, 16))
+def test_copy_between_alignments(cuda, shift):
+    """Copies whose two addresses differ modulo 16, on both sides of the length
+    from which they are joined from aligned vectors, at lengths that end
+    anywhere in a vector; bytes around the destination stay."""
+    torch = cuda
+    n = (512 << 10) + 40
+    src_h = np.frombuffer(oracle.random_words(n // 4 + 16, shift).tobytes(), np.uint8)
+    src = to_dev(torch, src_h)
+    for nbytes in [(512 << 10) - 1, 512 << 10, (512 << 10) + shift, n]:
+        for doff in (0, 5, 16 - shift, 15):
+            soff = (doff + shift) % 16
+            for kw in ({}, {"path": "vector", "unroll": 2}, {"path": "vector", "unroll": 8, "grid": 3}):
+                buf, start = guarded(torch, nbytes, offset=doff)
+                tg.copy(buf[start:], src[soff:], nbytes, 1, **kw)
+                assert np.array_equal(check_guards(buf, start, nbytes), src_h[soff:soff + nbytes]), (nbytes, doff, kw)

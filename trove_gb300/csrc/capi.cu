@@ -154,14 +154,30 @@ bool size_ok(uint64_t n, uint32_t width) { return width != 0 && n <= (uint64_t(1
 
 bool struct_width(uint32_t width) { return width % 4 == 0 && width >= 4 && width <= 64; }
 
+// Copies between different alignments are joined from aligned vectors (flat.cu)
+// from this length on: 1 MiB shared 4-byte alignment 1.73 us by words and 1.81
+// joined, odd addresses 2.6 by bytes and 1.8 joined; 64 KiB 1.6 and 1.7.  Short
+// ones take one vector to a thread (1 MiB: 1.8 us at 1, 2.07 at 4; 16 MiB: 7.6
+// and 7.1).
+constexpr uint64_t kShiftCopyBytes = uint64_t(512) << 10;
+constexpr uint64_t kShortShiftBytes = uint64_t(4) << 20;
+
 int copy_flat(void* dst, const void* src, uint64_t nbytes, int unroll, int grid_req, cudaStream_t st) {
     const uintptr_t a = reinterpret_cast<uintptr_t>(src), b = reinterpret_cast<uintptr_t>(dst);
     int vec = 16;
     while (vec > 1 && ((a ^ b) & uintptr_t(vec - 1)) != 0) vec >>= 1;
     long long head = (long long)((vec - (a & uintptr_t(vec - 1))) & uintptr_t(vec - 1));
     if ((uint64_t)head > nbytes) head = (long long)nbytes;
+    const int asked = unroll;
     if (unroll <= 0) unroll = 4;
     if (unroll_slot(unroll) < 0) return TRV_ERR_INVALID_ARGUMENT;
+    if (vec < 16 && nbytes >= kShiftCopyBytes) {
+        const ShiftPlan p = plan_shift_copy(src, dst, (long long)nbytes);
+        const int u = asked > 0 ? std::min(asked, 4) : nbytes < kShortShiftBytes ? 1 : 4;
+        launch_shift_copy(src, dst, (long long)nbytes, p, u,
+                          grid_for(shift_copy_func(), p.body, 256 * u, 256, grid_req), st);
+        return check_launch();
+    }
     const void* func = flat_copy_func(vec, unroll);
     const long long body = ((long long)nbytes - head) / vec;
     const int grid = grid_for(func, body, 256 * unroll, 256, grid_req);

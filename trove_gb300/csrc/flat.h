@@ -33,6 +33,18 @@ void launch_flat_copy(const void* src, void* dst, long long nbytes, int vec_byte
                       int grid, cudaStream_t st);
 const void* flat_copy_func(int vec_bytes, int unroll);
 
+// Copy between addresses that differ modulo 16: `head` leading bytes, then
+// `body` aligned destination vectors (may come out below 1 for short copies),
+// then the rest.  shift: source minus destination address, modulo 16 (not 0).
+struct ShiftPlan {
+    int shift, head;
+    long long body;
+};
+ShiftPlan plan_shift_copy(const void* src, const void* dst, long long nbytes);
+void launch_shift_copy(const void* src, void* dst, long long nbytes, const ShiftPlan& p, int unroll, int grid,
+                       cudaStream_t st);
+const void* shift_copy_func();
+
 // Gather / scatter of structs of `width` bytes (at most kMostPackedWidth) at any
 // alignment (packed.cu).  grid 0: one chunk per warp.
 constexpr unsigned kMostPackedWidth = 1u << 20;
