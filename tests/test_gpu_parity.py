@@ -503,3 +503,47 @@ def test_copy_between_alignments(cuda, shift):
                 buf, start = guarded(torch, nbytes, offset=doff)
                 tg.copy(buf[start:], src[soff:], nbytes, 1, **kw)
                 assert np.array_equal(check_guards(buf, start, nbytes), src_h[soff:soff + nbytes]), (nbytes, doff, kw)
+
+
+@pytest.mark.parametrize("width,offset", [(68, 0), (68, 4), (80, 0), (96, 8), (132, 0), (200, 0), (256, 0), (1028, 0)])
+def test_index_ops_wide_default_route(cuda, width, offset):
+    """Rows wider than 64 bytes as a plain call takes them, at the lengths where
+    the rows to a warp change, at every word size, with skipped rows."""
+    torch = cuda
+    for n in [1, 3, 5, 1 << 13, (1 << 13) + 1, (1 << 15) + 3] + ([(1 << 16) + 5, (1 << 17) + 9] if width < 100 else []):
+        bound = n + 7
+        src_h = oracle.random_structs(bound, width, seed=n)
+        src = torch.zeros(bound * width + 64, dtype=torch.uint8, device="cuda")
+        src[offset:offset + bound * width] = to_dev(torch, src_h)
+        perm = oracle.permutation(bound, n)[:n].copy()
+        perm[n // 2:n // 2 + 1] = -1
+        perm[::11] = bound
+        ok = (perm >= 0) & (perm < bound)
+        idx = torch.from_numpy(perm).cuda()
+        expect = np.full((n, width), SENTINEL, np.uint8)
+        expect[ok] = src_h[perm[ok]]
+        buf, start = guarded(torch, n * width, offset=offset)
+        tg.gather(buf[start:], src[offset:], bound, idx, n, width)
+        assert np.array_equal(check_guards(buf, start, n * width), expect.reshape(-1)), ("gather", n)
+        expect = np.full((bound, width), SENTINEL, np.uint8)
+        expect[perm[ok]] = src_h[:n][ok]
+        buf, start = guarded(torch, bound * width, offset=offset)
+        tg.scatter(buf[start:], bound, src[offset:], idx, n, width)
+        assert np.array_equal(check_guards(buf, start, bound * width), expect.reshape(-1)), ("scatter", n)
+
+
+def test_scatter_wide_rows_in_parts(cuda):
+    """2^21 rows and more wider than 64 bytes go in parts: the sorted and the
+    random form, and 4-byte words."""
+    torch = cuda
+    n, width = (1 << 21) + 3, 68
+    src = torch.randint(0, 255, (n, width), dtype=torch.uint8, device="cuda")
+    for idx in (torch.randperm(n, device="cuda").to(torch.int32), torch.arange(n, device="cuda", dtype=torch.int32)):
+        idx[5] = -1
+        idx[n - 1] = n
+        ok = (idx >= 0) & (idx < n)
+        expect = torch.full((n, width), SENTINEL, dtype=torch.uint8, device="cuda")
+        expect[idx[ok].long()] = src[ok]
+        dst = torch.full((n, width), SENTINEL, dtype=torch.uint8, device="cuda")
+        tg.scatter(dst, n, src, idx, n, width)
+        assert torch.equal(dst, expect)

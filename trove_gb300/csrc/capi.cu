@@ -380,6 +380,14 @@ static int scatter_parts(uint32_t width, uint64_t n, uint64_t dst_n, const void*
     return int(parts);
 }
 
+// Of wide rows only the two sectors at the ends are filled, and the passes pay
+// later: random scatters plain / in parts in us, 2^20 rows of 80 bytes 47 / 53,
+// 2^21 121 / 104; 2^20 of 120 bytes 77 / 87, 2^21 180 / 149; 2^21 of 200 bytes
+// 241 / 224, 2^22 500 / 465; 2^22 of 228 bytes 616 / 600.
+static bool wide_parts_pay(uint32_t width, uint64_t n, uint64_t dst_n, const void* dst) {
+    return width <= 200 && dst_n >= (uint64_t(1) << 21) && scatter_parts(width, n, dst_n, dst) > 1;
+}
+
 // Structs per lane of the row-form kernels when the caller gives none.  A call
 // of at most 2^16 structs does not fill the GPU (2048 warps at one struct per
 // lane): more structs per lane only lengthen each warp (4096 structs of 28
@@ -396,16 +404,17 @@ static int rows_unroll(bool gather, uint32_t width, uint64_t n) {
     return width <= 8 ? 2 : 1;
 }
 
-// L2 fetch hint of a gather's random loads.  A source larger than L2 holds
-// (64 MiB and more) is fetched by 64-byte halves (policy 4): the rest of a
-// 128-byte line would leave L2 before another row of it is asked for.  A
-// source that fits and most of whose rows are read is fetched by whole lines
-// (policy 5), which brings the neighbouring rows in early: 2^20 rows of 64
-// bytes 25.0 us against 28.3 with 64-byte fetches, of 48 bytes 19.1 against
-// 20.0; below 32 bytes the two are within 3 %, and narrow rows keep policy 4.
-constexpr uint64_t kL2SourceBytes = uint64_t(64) << 20;
+// L2 fetch hint of a gather's random loads.  A source larger than L2 is
+// fetched by 64-byte halves (policy 4): the rest of a 128-byte line would leave
+// L2 before another row of it is asked for.  A source that fits (112 MiB of 126)
+// and most of whose rows are read is fetched by whole lines (policy 5), which
+// brings the neighbouring rows in early: in us at 64 / 128-byte fetches, 2^20
+// rows of 64 bytes 28.6 / 25.5, 2^22 of 28 bytes 77.3 / 69.0, 2^23 of 12 bytes
+// 94.7 / 81.9.  8-byte rows and narrower do not care, and between 112 and 256
+// MiB GB300s differ (2^24 of 12 bytes 282 / 257 on one, 220 / 244 on another).
+constexpr uint64_t kL2SourceBytes = uint64_t(112) << 20;
 static int gather_policy(uint32_t width, uint64_t n, uint64_t src_n) {
-    return width >= 32 && src_n * width <= kL2SourceBytes && 2 * n >= src_n ? 5 : 4;
+    return width >= 12 && src_n * width <= kL2SourceBytes && 2 * n >= src_n ? 5 : 4;
 }
 
 // Rows of any width and alignment move in 4-byte words (packed.cu) where that
@@ -445,8 +454,11 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
             c = gather                                    ? trv_launch{TRV_PATH_WARP, 0, 0, 0, 0, gather_policy(width, n, bound)}
                                                           : trv_launch{TRV_PATH_WARP, 0, 0, 0, 0,
                                                                        scatter_parts(width, n, bound, dst) ? 6 : 1};
+        else if (wide_words)
+            c = trv_launch{TRV_PATH_WARP, 0, 0, 0, 0,
+                           gather ? gather_policy(width, n, bound) : wide_parts_pay(width, n, bound, dst) ? 6 : 0};
         else
-            c.path = wide_words ? TRV_PATH_WARP : TRV_PATH_VECTOR;
+            c.path = TRV_PATH_VECTOR;
     }
     if (c.cache_policy < 0 || c.cache_policy > 6 || (gather && c.cache_policy == 6)) return TRV_ERR_INVALID_ARGUMENT;
     const int path = c.path;
@@ -474,10 +486,22 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
         int wb = 16;
         while (wb > 4 && (width % uint32_t(wb) != 0 || !aligned(dst, uintptr_t(wb)) || !aligned(src, uintptr_t(wb))))
             wb >>= 1;
+        const int m = int(width / uint32_t(wb));
+        IndexArgs a{src, dst, idx, (long long)n, (long long)bound, c.cache_policy};
+        if (!gather && c.cache_policy == 6 && n >= 2 && bound >= 1) {
+            const uint64_t parts = std::min<uint64_t>(parts_of(bound * width), 64);
+            if (parts > 1) {
+                launch_scatter_passes(wb, a, m, int(parts), st);
+                return check_launch();
+            }
+            launch_fetch_destination(a, int(width), st);
+        }
+        if (grid_req == 0 && (gather ? c.cache_policy == 4 || c.cache_policy == 5 : c.cache_policy != 2 && c.cache_policy != 3) &&
+            launch_wide_rows(gather, wb, a, m, st))
+            return check_launch();
         const long long warps = (long long)((n + 31) / 32);
         const int grid = grid_for(index_rows_rt_func(gather, wb), warps, 8, 256, grid_req);
-        launch_index_rows_rt(gather, wb, IndexArgs{src, dst, idx, (long long)n, (long long)bound, c.cache_policy},
-                             int(width / uint32_t(wb)), grid, st);
+        launch_index_rows_rt(gather, wb, a, m, grid, st);
         return check_launch();
     }
     if (!struct_width(width)) return TRV_ERR_UNSUPPORTED;

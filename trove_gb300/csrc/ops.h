@@ -64,7 +64,11 @@ struct WidthOps {
 void launch_index_rows_rt(bool gather, int word_bytes, const IndexArgs& a, int m, int grid, cudaStream_t st);
 const void* index_rows_rt_func(bool gather, int word_bytes);
 
-// Scatter onto a large destination (rows_rt.cu), any width that is a multiple
+// The default launches of the same (gathers with cache policy 4 or 5); false
+// where the grid-stride form is the better one.
+bool launch_wide_rows(bool gather, int word_bytes, const IndexArgs& a, int m, cudaStream_t st);
+
+// Scatter onto a large destination (scatter_parts.cu), any width that is a multiple
 // of 4 bytes, n >= 2: in `passes` parts of the destination (one launch), or the
 // fetch of the destination into L2 ahead of a scatter in one pass.
 void launch_scatter_passes(int word_bytes, const IndexArgs& a, int m, int passes, cudaStream_t st);
