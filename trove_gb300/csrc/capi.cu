@@ -404,6 +404,16 @@ static int rows_unroll(bool gather, uint32_t width, uint64_t n) {
     return width <= 8 ? 2 : 1;
 }
 
+// The same for the struct kernels (coalesced_ptr and compiler-generated access),
+// whose loads and stores go through a struct to a lane: 2^23 structs of 4 bytes
+// 48.7 us at 1, 42.3 at 2, 41.1 at 4, 40.7 at 8; contiguous indices of 16 bytes
+// 53.1 / 48.2 / 45.1 at 1 / 2 / 4; of 12 bytes 58.1 / 49.9 / 48.3, but random
+// ones 86.9 / 86.3 / 90.2; from 28 bytes up 1 is as fast or faster.
+static int struct_unroll(uint32_t width, uint64_t n) {
+    if (n <= (uint64_t(1) << 16)) return 1;
+    return width == 4 ? 8 : width == 8 || width == 16 ? 4 : width <= 24 ? 2 : 1;
+}
+
 // L2 fetch hint of a gather's random loads.  A source larger than L2 is
 // fetched by 64-byte halves (policy 4): the rest of a 128-byte line would leave
 // L2 before another row of it is asked for.  A source that fits (112 MiB of 126)
@@ -508,7 +518,7 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
     if (!aligned(dst, 4) || !aligned(src, 4)) return TRV_ERR_MISALIGNED;
     const int u = c.unroll > 0                ? c.unroll
                   : path == TRV_PATH_WARP ? rows_unroll(gather, width, n)
-                                          : default_unroll(width);
+                                          : struct_unroll(width, n);
     const int slot = unroll_slot(u);
     if (slot < 0) return TRV_ERR_INVALID_ARGUMENT;
     const WidthOps* ops = ops_for_words(int(width / 4));

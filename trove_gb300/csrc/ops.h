@@ -24,7 +24,7 @@ struct IndexArgs {
     long long n;
     long long bound;  // src_n for gather, dst_n for scatter
     int policy;       // cache policy of the row-form kernels
-    bool once = false; // row-form kernels: the grid covers every 32*unroll-struct chunk with one warp
+    bool once = false; // the grid covers every 32*unroll-struct chunk with one warp
 };
 
 template <typename Args>

@@ -20,14 +20,14 @@ void launch_copy(const CopyArgs& a, int grid, int block, cudaStream_t st) {
 
 template <int U, int MODE>
 void launch_gather(const IndexArgs& a, int grid, int block, cudaStream_t st) {
-    gather_kernel<S, U, MODE><<<grid, block, 0, st>>>(static_cast<const aos<S>*>(a.src), a.bound, a.idx,
-                                                      static_cast<aos<S>*>(a.dst), a.n);
+    auto* k = a.once ? &gather_kernel<S, U, MODE, false> : &gather_kernel<S, U, MODE, true>;
+    k<<<grid, block, 0, st>>>(static_cast<const aos<S>*>(a.src), a.bound, a.idx, static_cast<aos<S>*>(a.dst), a.n);
 }
 
 template <int U, int MODE>
 void launch_scatter(const IndexArgs& a, int grid, int block, cudaStream_t st) {
-    scatter_kernel<S, U, MODE><<<grid, block, 0, st>>>(static_cast<const aos<S>*>(a.src), a.idx,
-                                                       static_cast<aos<S>*>(a.dst), a.bound, a.n);
+    auto* k = a.once ? &scatter_kernel<S, U, MODE, false> : &scatter_kernel<S, U, MODE, true>;
+    k<<<grid, block, 0, st>>>(static_cast<const aos<S>*>(a.src), a.idx, static_cast<aos<S>*>(a.dst), a.bound, a.n);
 }
 
 // Unroll actually built for table slot k (1, 2, 4, 8): a lane keeps at most
@@ -148,13 +148,13 @@ void fill_copy(CopyKernel (&row)[kUnrolls]) {
 template <int MODE, int k>
 IndexKernel gather_entry() {
     constexpr int U = unroll_for(k);
-    return {&launch_gather<U, MODE>, (const void*)&gather_kernel<S, U, MODE>};
+    return {&launch_gather<U, MODE>, (const void*)&gather_kernel<S, U, MODE, true>};
 }
 
 template <int MODE, int k>
 IndexKernel scatter_entry() {
     constexpr int U = unroll_for(k);
-    return {&launch_scatter<U, MODE>, (const void*)&scatter_kernel<S, U, MODE>};
+    return {&launch_scatter<U, MODE>, (const void*)&scatter_kernel<S, U, MODE, true>};
 }
 
 template <int MODE>
