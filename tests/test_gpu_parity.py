@@ -547,3 +547,23 @@ def test_scatter_wide_rows_in_parts(cuda):
         dst = torch.full((n, width), SENTINEL, dtype=torch.uint8, device="cuda")
         tg.scatter(dst, n, src, idx, n, width)
         assert torch.equal(dst, expect)
+
+
+@pytest.mark.parametrize("modulus", [1, 2, 3, 6, 625, 640, 1 << 31, (1 << 31) + 1, 0xFFFFFFFE, 0xFFFFFFFF])
+def test_copy_exit_moduli(cuda, modulus):
+    """The exit predicate for odd, even, power-of-two and largest moduli, on words
+    around every kind of multiple: the smallest, the largest, the wrap-around."""
+    torch = cuda
+    width, n = 8, 40000
+    words = oracle.random_words(2 * n, modulus & 0xFFFF).astype(np.uint32).copy()
+    edge = np.array([0, 1, modulus - 2, modulus - 1, modulus, 2 * modulus - 1, 0xFFFFFFFF, 0xFFFFFFFE, 1 << 31]) & 0xFFFFFFFF
+    words[0:36:4] = edge.astype(np.uint32)
+    near = (words[2000:4000].astype(np.uint64) // modulus) * modulus + modulus - 1
+    words[2000:4000] = (near & 0xFFFFFFFF).astype(np.uint32)
+    src_h = words.view(np.uint8).reshape(n, width)
+    init = np.full(n * width, SENTINEL, np.uint8)
+    expect, _ = oracle.copy_exit(init, src_h, n, width, modulus)
+    for path in ("warp", "block"):
+        dst = to_dev(torch, init)
+        tg.copy_exit(dst, to_dev(torch, src_h), n, width, modulus, path=path)
+        assert np.array_equal(to_host(dst), expect), (modulus, path)

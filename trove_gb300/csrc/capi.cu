@@ -298,12 +298,26 @@ int32_t trv_copy_ex(void* dst, const void* src, uint64_t n, uint32_t width, cons
     const bool once = one_chunk_per_warp((long long)n, ub, grid_req, &grid);
     const CopyKernel& k = once ? ops->copy[api][slot] : ops->copy_grid[api][slot];
     if (!once) grid = grid_for(k.func, (long long)n, 256 * ub, 256, grid_req);
-    k.launch(CopyArgs{src, dst, (long long)n, 0u}, grid, 256, st);
+    k.launch(CopyArgs{src, dst, (long long)n, {}}, grid, 256, st);
     return check_launch();
 }
 
 int32_t trv_copy(void* dst, const void* src, uint64_t n, uint32_t width, void* stream) {
     return trv_copy_ex(dst, src, n, width, nullptr, stream);
+}
+
+// Structs per lane of the early-exit copy when the caller gives none.  Up to 4
+// MiB the GPU is not full and more to a lane only lengthens each warp (1 MiB of
+// 12 bytes 1.74 us at 1, 1.94 at 2, 2.16 at 4).  Above, narrow structs need
+// several in flight (1 GiB of 4 bytes 770 / 446 / 326 / 305 us at 1 / 2 / 4 / 8;
+// of 8 bytes 442 / 324 / 304 / 306; of 12 bytes 380 / 351 / 309 / 322; of 16 bytes
+// 315 / 303 / 304) and from 24 bytes up one is as good as two or better (24 bytes
+// 298 / 302, 28 bytes 300 / 305).  20 bytes change over: 16 MiB 7.4 / 8.0, 128 MiB
+// 41.8 / 41.5, 1 GiB 315 / 307.
+static int exit_unroll(uint32_t width, uint64_t bytes) {
+    if (bytes <= (uint64_t(4) << 20)) return width == 4 ? 2 : 1;
+    if (width == 20) return bytes >= (uint64_t(128) << 20) ? 2 : 1;
+    return width == 4 ? 8 : width <= 12 ? 4 : width == 16 ? 2 : 1;
 }
 
 int32_t trv_copy_exit_ex(void* dst, const void* src, uint64_t n, uint32_t width, uint32_t modulus,
@@ -323,7 +337,7 @@ int32_t trv_copy_exit_ex(void* dst, const void* src, uint64_t n, uint32_t width,
             u = t.unroll;
             if (grid_req == 0) grid_req = t.grid;
         } else {
-            u = default_unroll(width);
+            u = exit_unroll(width, n * width);
         }
     }
     const int slot = unroll_slot(u);
@@ -333,9 +347,12 @@ int32_t trv_copy_exit_ex(void* dst, const void* src, uint64_t n, uint32_t width,
     const int ub = ops->built_unroll[slot];
     int grid = 0;
     const bool once = one_chunk_per_warp((long long)n, ub, grid_req, &grid);
-    const CopyKernel& k = once ? ops->copy_exit[api][slot] : ops->copy_exit_grid[api][slot];
+    const CopyKernel& k = modulus == 0 ? (once ? ops->copy[api][slot] : ops->copy_grid[api][slot])  // no struct leaves
+                          : once       ? ops->copy_exit[api][slot]
+                                       : ops->copy_exit_grid[api][slot];
     if (!once) grid = grid_for(k.func, (long long)n, 256 * ub, 256, grid_req);
-    k.launch(CopyArgs{src, dst, (long long)n, modulus}, grid, 256, static_cast<cudaStream_t>(stream));
+    k.launch(CopyArgs{src, dst, (long long)n, modulus == 0 ? ExitTest() : ExitTest(modulus)}, grid, 256,
+             static_cast<cudaStream_t>(stream));
     return check_launch();
 }
 
@@ -571,6 +588,21 @@ int32_t trv_scatter(void* dst, uint64_t dst_n, const void* src, const int32_t* i
     return index_op(false, dst, src, dst_n, idx, n, width, nullptr, stream);
 }
 
+// The same for the layout conversions.  To SoA in us at 1 / 2 / 4 / 8: 512 MiB of
+// 4 bytes 366 / 214 / 159 / 153, of 8 bytes 215 / 161 / 154 / 153, of 12 bytes 183 /
+// 179 / 177 / 253 (32 MiB 13.9 / 13.9 / 14.6), of 28 bytes 158 / 162, of 64 bytes 185
+// / 170 (32 MiB 13.2 / 14.1).  From SoA: 512 MiB of 12 bytes 190 / 158 / 156, of 24
+// bytes 159 / 159 / 157, of 28 bytes 156 / 157, of 64 bytes 170 / 168.
+static int layout_unroll(bool to_soa, uint32_t width, uint64_t bytes) {
+    if (bytes <= (uint64_t(4) << 20)) return width == 4 ? 2 : 1;
+    if (width == 4) return 8;
+    if (to_soa) {
+        const bool large = bytes >= (uint64_t(256) << 20);
+        return width == 8 ? 4 : width <= 16 || (large && (width == 32 || width >= 40)) ? 2 : 1;
+    }
+    return width <= 12 ? 4 : width <= 24 ? 2 : 1;
+}
+
 static int32_t layout_op(bool to_soa, void* dst, const void* src, uint64_t n, uint32_t width, const trv_launch* cfg,
                          void* stream) {
     if (!size_ok(n, width)) return TRV_ERR_INVALID_ARGUMENT;
@@ -588,7 +620,7 @@ static int32_t layout_op(bool to_soa, void* dst, const void* src, uint64_t n, ui
             u = t.unroll;
             if (grid_req == 0) grid_req = t.grid;
         } else {
-            u = default_unroll(width);
+            u = layout_unroll(to_soa, width, n * width);
         }
     }
     const int slot = unroll_slot(u);
@@ -600,7 +632,7 @@ static int32_t layout_op(bool to_soa, void* dst, const void* src, uint64_t n, ui
     const CopyKernel& k = once ? (to_soa ? ops->aos_to_soa[slot] : ops->soa_to_aos[slot])
                                : (to_soa ? ops->aos_to_soa_grid[slot] : ops->soa_to_aos_grid[slot]);
     if (!once) grid = grid_for(k.func, (long long)n, 256 * ub, 256, grid_req);
-    k.launch(CopyArgs{src, dst, (long long)n, 0u}, grid, 256, static_cast<cudaStream_t>(stream));
+    k.launch(CopyArgs{src, dst, (long long)n, {}}, grid, 256, static_cast<cudaStream_t>(stream));
     return check_launch();
 }
 

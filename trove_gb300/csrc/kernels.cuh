@@ -20,6 +20,8 @@
 #include <trove/block.h>
 #include <trove/ptr.h>
 
+#include "ops.h"
+
 namespace trv {
 
 template <int S>
@@ -27,9 +29,18 @@ using aos = trove::array<unsigned, S>;
 
 enum Api { API_WARP = 0, API_BLOCK = 1, API_DIRECT = 2 };
 
+// Whether the struct's first word w has w % d == d - 1.  That is w >= d - 1 and d
+// divides w - (d - 1); and d = q * 2^k (q odd) divides x when x times q's inverse
+// modulo 2^32, rotated right by k, is at most (2^32 - 1) / d (Granlund and
+// Montgomery, "Division by Invariant Integers using Multiplication", section 9).
+// Five instructions where the remainder of a run-time d took about twenty of
+// the 84 that 32 structs of 12 bytes cost: 1 GiB of 4 bytes 311 -> 305 us, of 12
+// bytes 321 -> 309, of 20 bytes 316 -> 307, of 24 bytes 301 -> 298.
 template <int S>
-__device__ __forceinline__ bool exits(const aos<S>& v, unsigned modulus) {
-    return modulus != 0u && (v.head % modulus) == modulus - 1u;
+__device__ __forceinline__ bool exits(const aos<S>& v, const ExitTest& t) {
+    const unsigned w = unsigned(v.head);
+    const unsigned x = (w - t.low) * t.inverse;
+    return w >= t.low && __funnelshift_r(x, x, t.rotate) <= t.most;
 }
 
 // Load/store of struct i when the caller's warp is converged and its lanes
@@ -118,9 +129,17 @@ struct WarpGrid {
 // to 32+ registers and below full occupancy (2048 threads per SM), which is
 // where a one-chunk kernel gets its loads in flight.  LOOP = true serves
 // caller-chosen and persistent grids.
+// Resident blocks that the early-exit copy is built for, by the words of a lane:
+// up to 12 words fit 32 registers and 24 words 40 without spills, but ptxas takes
+// 38-48 where it may (1 GiB of 12 bytes, 4 structs to a lane, 326 us at 40
+// registers and 309 at 32; 24 bytes, 2 to a lane, 319 and 302).  One struct of 11
+// words and more to a lane is left alone: its 48 warps fill the memory system
+// (44 bytes 301.8 us, 303.6 at 64 warps).
+constexpr int exit_blocks(int words, int unroll) { return words <= (unroll > 1 ? 12 : 10) ? 8 : unroll > 1 && words <= 24 ? 6 : 1; }
+
 template <int S, int U, int API, bool EXIT>
 __device__ __forceinline__ void copy_chunk(const aos<S>* __restrict__ src, aos<S>* __restrict__ dst, long long n,
-                                           unsigned modulus, long long base, int lane) {
+                                           const ExitTest& test, long long base, int lane) {
     constexpr int CH = 32 * U;
     if (base + CH <= n) {
         aos<S> v[U];
@@ -128,7 +147,7 @@ __device__ __forceinline__ void copy_chunk(const aos<S>* __restrict__ src, aos<S
         for (int u = 0; u < U; ++u) v[u] = load_conv<S, API>(src, base + u * 32 + lane);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            if (!EXIT || !exits(v[u], modulus)) {
+            if (!EXIT || !exits(v[u], test)) {
                 if constexpr (EXIT)
                     store_any<S, API>(dst, base + u * 32 + lane, v[u]);
                 else
@@ -141,23 +160,23 @@ __device__ __forceinline__ void copy_chunk(const aos<S>* __restrict__ src, aos<S
             const long long i = base + u * 32 + lane;
             if (i < n) {
                 const aos<S> v = src[i];
-                if (!EXIT || !exits(v, modulus)) dst[i] = v;
+                if (!EXIT || !exits(v, test)) dst[i] = v;
             }
         }
     }
 }
 
 template <int S, int U, int API, bool EXIT, bool LOOP>
-__global__ void __launch_bounds__(256) copy_kernel(const aos<S>* __restrict__ src, aos<S>* __restrict__ dst,
-                                                   long long n, unsigned modulus) {
+__global__ void __launch_bounds__(256, EXIT && !LOOP ? exit_blocks(S * U, U) : 1) copy_kernel(const aos<S>* __restrict__ src, aos<S>* __restrict__ dst,
+                                                   long long n, ExitTest test) {
     const WarpGrid g;
     constexpr int CH = 32 * U;
     if constexpr (LOOP) {
         for (long long base = g.warp * CH; base < n; base += g.warps * CH)
-            copy_chunk<S, U, API, EXIT>(src, dst, n, modulus, base, g.lane);
+            copy_chunk<S, U, API, EXIT>(src, dst, n, test, base, g.lane);
     } else {
         const long long base = g.warp * CH;
-        if (base < n) copy_chunk<S, U, API, EXIT>(src, dst, n, modulus, base, g.lane);
+        if (base < n) copy_chunk<S, U, API, EXIT>(src, dst, n, test, base, g.lane);
     }
 }
 

@@ -10,11 +10,24 @@ namespace trv {
 // Unroll factors offered (structs per lane per pass); index = log2(unroll).
 constexpr int kUnrolls = 4;  // 1, 2, 4, 8
 
+// The early-exit test w % d == d - 1 without a division (kernels.cuh, exits).
+struct ExitTest {
+    unsigned low = 0, inverse = 1, rotate = 0, most = 0;
+    ExitTest() = default;
+    explicit ExitTest(unsigned d) : low(d - 1), most(0xFFFFFFFFu / d) {  // d > 0
+        while (d % 2 == 0) {
+            d /= 2;
+            ++rotate;
+        }
+        for (int k = 0; k < 5; ++k) inverse *= 2u - d * inverse;  // Newton: 5 steps give 32 bits and more
+    }
+};
+
 struct CopyArgs {
     const void* src;
     void* dst;
     long long n;
-    unsigned modulus;
+    ExitTest test;
 };
 
 struct IndexArgs {

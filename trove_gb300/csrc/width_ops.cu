@@ -15,7 +15,7 @@ constexpr int S = TRV_WIDTH;
 template <int U, int API, bool EXIT, bool LOOP>
 void launch_copy(const CopyArgs& a, int grid, int block, cudaStream_t st) {
     copy_kernel<S, U, API, EXIT, LOOP><<<grid, block, 0, st>>>(static_cast<const aos<S>*>(a.src),
-                                                               static_cast<aos<S>*>(a.dst), a.n, a.modulus);
+                                                               static_cast<aos<S>*>(a.dst), a.n, a.test);
 }
 
 template <int U, int MODE>
