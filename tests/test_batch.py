@@ -352,3 +352,42 @@ def test_autotune_on_gpu(cuda, tmp_path):
     tg.autotune_save(tmp_path / "cache.json")
     assert json.loads((tmp_path / "cache.json").read_text())
     tg.autotune_clear()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("width", [4, 8, 12, 20, 24, 28, 36, 52, 60])
+def test_staged_rows_of_narrow_words(cuda, width):
+    """The staged movers of 4- and 8-byte words: task lengths around a piece and
+    a tile, pieces with and without skipped rows (written by one bulk copy or
+    word by word), destinations that bulk copies cannot write, both builds."""
+    torch = cuda
+    per = min(11008 // width // 32 * 32, 480)
+    lengths = [1, 31, per - 1, per, per + 1, 3 * per + 5, 7 * per, 20011]
+    for blocks in (2, 4):
+        for skip in (0, 1, 997):
+            for offset in (0, 8):
+                tasks, checks = [], []
+                for k, n in enumerate(lengths):
+                    src_h = oracle.random_structs(n, width, seed=width + n)
+                    sbuf = torch.zeros(n * width + 16, dtype=torch.uint8, device="cuda")
+                    sbuf[offset:offset + n * width] = torch.from_numpy(src_h.reshape(-1).copy()).cuda()
+                    uni, perm = oracle.uniform_indices(n, n, k).copy(), oracle.permutation(n, k).copy()
+                    if skip:
+                        uni[skip - 1::skip * 7] = -1
+                        perm[skip - 1::skip * 7] = n + 3
+                    for op, idx_h in ((tg.OP_GATHER, uni), (tg.OP_SCATTER, perm)):
+                        dst = torch.full((n * width + 32,), SENTINEL, dtype=torch.uint8, device="cuda")
+                        idx = torch.from_numpy(idx_h).cuda()
+                        tasks.append(dict(op=op, width=width, n=n, src=sbuf[offset:], dst=dst[offset:], idx=idx, bound=n))
+                        expect = np.full((n, width), SENTINEL, np.uint8)
+                        ok = (idx_h >= 0) & (idx_h < n)
+                        if op == tg.OP_GATHER:
+                            expect[ok] = src_h[idx_h[ok]]
+                        else:
+                            expect[idx_h[ok]] = src_h[ok]
+                        checks.append((dst, expect, sbuf))
+                tg.Batch(tasks, blocks_per_sm=blocks, tile_bytes=[0, 4096][skip == 1]).launch()
+                for dst, expect, _ in checks:
+                    h = dst.cpu().numpy()
+                    assert np.array_equal(h[offset:offset + expect.size], expect.reshape(-1)), (blocks, skip, offset, expect.shape)
+                    assert (h[:offset] == SENTINEL).all() and (h[offset + expect.size:] == SENTINEL).all()

@@ -36,26 +36,36 @@ constexpr int kBulkChunk = 8 << 10;
 
 // Launch shapes of the persistent kernel: block size, resident blocks per SM
 // it is built for (hence the register budget), the staged gather / scatter
-// piece with its index slots, and the copy ring's stages.  Staged movers
-// cycle through two pieces per block; four per block measured slower (18.5
-// vs 14.9 ms for the 4096-array batch's gathers at 2 blocks per SM): more
-// resident blocks is what pays (12.1 ms at 4), as block barriers then
-// overlap.  128-thread blocks, 8 per SM, with 8 KiB pieces measured no
-// better (23.8 vs 22.9 ms for the whole batch).  The copy ring reuses the
-// piece buffers.  Either shape holds 160 KiB of shared memory per SM.
+// pieces with their index slots, and the copy ring's stages, which reuse the
+// pieces' memory.  128-thread blocks, 8 per SM, with 8 KiB pieces measured no
+// better than 256-thread ones (23.8 vs 22.9 ms for a 4096-array batch).
+//
+// The pieces' size is a balance of the two halves of an SM's 256 KiB.  Rows that
+// are copied by 4 or 8 bytes pass through L1, a 128-byte line for each row in
+// flight, so the more shared memory the blocks take, the fewer rows are in
+// flight; rows copied by 16 bytes go around L1 and are in flight in the pieces
+// alone.  2^24 rows of 12 / 20 / 64 bytes from sources of 2^19, us: 12 KiB pieces
+// with 1024 indices (212 KiB an SM, 28 KiB of L1) 264 / 328 / 348; these (163 and
+// 92) 150 / 180 / 333; 8 KiB with 416 (127 and 124) 147 / 176 / 369; 4 KiB with
+// 256 (100 and 156, but twice the barriers) 185 / 215 / 519.
+constexpr int kPieces = 3;      // staged pieces in shared memory (words of 4 and 8 bytes)
+constexpr int kIndexSlots = 4;  // index arrays of as many pieces
+
 template <int BLOCK, int MINB, int PIECE, int RING>
 struct Shape {
     static constexpr int block = BLOCK;
     static constexpr int warps = BLOCK / 32;
     static constexpr int minb = MINB;
-    static constexpr int piece = PIECE;           // bytes of one staged piece
-    static constexpr int idx_slots = PIECE / 16;  // indices of one staged piece
-    static constexpr int ring = RING;             // copy stages of kBulkChunk bytes
-    static constexpr int dyn_smem = 2 * (PIECE + idx_slots * int(sizeof(int)));
-    static_assert(RING * kBulkChunk <= 2 * PIECE, "the copy ring fits the piece buffers");
+    static constexpr int piece = PIECE;     // bytes of one staged piece
+    static constexpr int idx_slots = 480;   // indices of one staged piece
+    static constexpr int wide_piece = kPieces * PIECE / 2;  // the same of the two pieces of 16-byte words
+    static constexpr int wide_slots = kIndexSlots * idx_slots / 2;
+    static constexpr int ring = RING;       // copy stages of kBulkChunk bytes
+    static constexpr int dyn_smem = kPieces * PIECE + kIndexSlots * idx_slots * int(sizeof(int));
+    static_assert(RING * kBulkChunk <= kPieces * PIECE, "the copy ring fits the piece buffers");
 };
-using Shape2 = Shape<256, 2, 16 << 10, 4>;  // 128 registers per thread
-using Shape4 = Shape<256, 4, 16 << 10, 4>;  // 64 registers
+using Shape2 = Shape<256, 2, 11008, 4>;  // 128 registers per thread
+using Shape4 = Shape<256, 4, 11008, 4>;  // 64 registers
 
 // ---- per-tile movers (all warps of the CTA cooperate on one tile) --------
 
@@ -207,20 +217,26 @@ __device__ __forceinline__ void tile_index_rows(const V* src, V* dst, const int*
 }
 
 // Gather / scatter of the structs [first, first + cnt) of the contiguous side
-// staged through shared memory with cp.async.  Gather: the warps issue
-// asynchronous word copies from the random source rows straight into a
-// shared-memory buffer (no registers hold the data in flight, so far more of
-// it can be), then write the buffer out to the contiguous destination with
-// coalesced stores.  Scatter: the contiguous source piece is copied in the
-// same way, then each word is stored to its random destination row from
-// shared memory (stores need no registers held in flight either).  Two
-// buffers of S::piece bytes alternate, so the next piece's copies are in
-// flight while the current one is written.  Word q of a piece (words of
-// sizeof(V)) belongs to struct q / m; the piece's indices are staged in
-// shared memory first (one coalesced read), invalid ones marked -1.  PF is
-// the L2 prefetch size the random row copies ask for on a miss: 0 the
-// context's fetch granularity, 64 or 128 bytes (GB300s differ in their
-// default, and the best size depends on the struct width).
+// staged through shared memory.  Gather: the warps issue asynchronous word
+// copies from the random source rows straight into a shared-memory piece (no
+// registers hold the data in flight, so far more of it can be), and one bulk
+// copy writes the piece to the contiguous destination.  Scatter: the
+// contiguous source piece is copied in, and each word is stored to its random
+// destination row from shared memory.  PF is the L2 prefetch size the random
+// row copies ask for on a miss: 0 the context's fetch granularity, 64 or 128
+// bytes (GB300s differ in their default, and the best size depends on the
+// struct width).
+//
+// Words of 4 and 8 bytes (tile_index_staged): three pieces of S::piece bytes
+// rotate, two filling while one is written, with one barrier a piece.  A thread
+// copies word r of rows j, j + step, ...: r and its source column are fixed for
+// the whole tile, so a word costs its index from shared memory, an address and
+// the copy; a gather's indices are copied in two pieces ahead of their rows.
+// (Dividing for each word, reading each piece's indices when its turn came and
+// writing the piece out word by word: 2^24 rows of 20 bytes 221 us, 180 since;
+// of 28 bytes 274 and 223; of 12 bytes 169 and 150.)
+// Words of 16 bytes (tile_index_wide): two pieces of half the memory each, and
+// the threads write them out; their words are few enough.
 template <int PF>
 __device__ __forceinline__ void cp_async_word(void* smem, const void* gmem, int bytes) {
     const unsigned s = smem_addr(smem);
@@ -279,20 +295,161 @@ __device__ __forceinline__ void cp_async_range(V* smem, const V* gmem, int bytes
 }
 
 template <class S, typename V, bool GATHER, int PF>
-__device__ void tile_index_staged(const V* src, V* dst, const int* idx, long long bound, long long first,
-                                  long long cnt, int m, unsigned char* stage, int* s_idx) {
-    constexpr int D = 2;
+__device__ void tile_index_staged(const V* src, V* dst, const int* idx, long long bound64, long long first, int cnt,
+                                  int m, unsigned char* stage, int* s_idx, int* s_bad) {
     const int tid = opaque_tid();
+    const unsigned bound = bound64 > 0x80000000ll ? 0x80000000u : unsigned(bound64);
     // structs per piece: a multiple of 32 that fits the buffer and the index slots
     int per = (S::piece / int(sizeof(V))) / m / 32 * 32;
     if (per > S::idx_slots) per = S::idx_slots;
+    const int pieces = (cnt + per - 1) / per;
+    // this thread's word of a row, its first row, and the rows that the block's
+    // threads cover together (the last few threads have no row where m does not
+    // divide the block)
+    const int step = S::block / m;
+    const int j0 = tid < step * m ? tid / m : S::idx_slots;
+    const int r = tid < step * m ? tid - tid / m * m : 0;
+    const unsigned row_bytes = unsigned(m) * unsigned(sizeof(V));
+    idx += first;
+    if (GATHER)
+        dst += first * m;
+    else
+        src += first * m;
+    const V* column = src + (GATHER ? r : 0);
+    V* out_column = dst + (GATHER ? 0 : r);
+    auto rows_of = [&](int p) { return cnt - p * per < per ? cnt - p * per : per; };
+    auto piece_at = [&](int p) { return reinterpret_cast<V*>(stage + (p % kPieces) * S::piece); };
+    auto index_at = [&](int p) { return s_idx + (p % kIndexSlots) * S::idx_slots; };
+    auto issue_indices = [&](int p) {
+        if (p < pieces) cp_async_range<S>(index_at(p), idx + p * per, rows_of(p) * 4, tid);
+    };
+    auto issue = [&](int p) {  // piece p, one group (an empty one past the end)
+        if (p < pieces) {
+            const int rows = rows_of(p);
+            if (GATHER) {
+                const int* ix = index_at(p);
+                V* buf = piece_at(p) + tid;
+                bool bad = false;
+                int j = j0;
+                for (; j + 3 * step < rows; j += 4 * step, buf += 4 * step * m) {
+                    int v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) v[u] = ix[j + u * step];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        if (unsigned(v[u]) < bound)
+                            cp_async_word<PF>(buf + u * step * m,
+                                              reinterpret_cast<const char*>(column) + (unsigned long long)unsigned(v[u]) * row_bytes,
+                                              int(sizeof(V)));
+                        else
+                            bad = true;
+                    }
+                }
+                for (; j < rows; j += step, buf += step * m) {
+                    const int v = ix[j];
+                    if (unsigned(v) < bound)
+                        cp_async_word<PF>(buf, reinterpret_cast<const char*>(column) + (unsigned long long)unsigned(v) * row_bytes,
+                                          int(sizeof(V)));
+                    else
+                        bad = true;
+                }
+                if (bad) s_bad[p % kIndexSlots] = 1;
+                issue_indices(p + 2);
+            } else {
+                cp_async_range<S>(index_at(p), idx + p * per, rows * 4, tid);
+                cp_async_range<S>(piece_at(p), src + (long long)p * per * m, rows * int(row_bytes), tid);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // Word by word: every scatter, and a gather's piece with rows to leave
+    // untouched or a destination that bulk copies cannot write.
+    auto drain = [&](int p) {
+        const int rows = rows_of(p);
+        const int* ix = index_at(p);
+        const V* buf = piece_at(p) + tid;
+        V* out = out_column + (GATHER ? (long long)p * per * m + tid : 0);
+        int j = j0;
+        for (; j + 3 * step < rows; j += 4 * step, buf += 4 * step * m, out += GATHER ? 4 * step * m : 0) {
+            int v[4];
+            V w[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                v[u] = ix[j + u * step];
+                w[u] = buf[u * step * m];
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (unsigned(v[u]) >= bound) continue;
+                if (GATHER)
+                    __stcs(out + u * step * m, w[u]);
+                else
+                    *reinterpret_cast<V*>(reinterpret_cast<char*>(out) + (unsigned long long)unsigned(v[u]) * row_bytes) = w[u];
+            }
+        }
+        for (; j < rows; j += step, buf += step * m, out += GATHER ? step * m : 0) {
+            const int v = ix[j];
+            if (unsigned(v) >= bound) continue;
+            if (GATHER)
+                __stcs(out, *buf);
+            else
+                *reinterpret_cast<V*>(reinterpret_cast<char*>(out) + (unsigned long long)unsigned(v) * row_bytes) = *buf;
+        }
+    };
+    const bool bulk = GATHER && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0;
+    if (GATHER) {
+        if (tid < kIndexSlots) s_bad[tid] = 0;
+        issue_indices(0);
+        issue_indices(1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        cp_async_wait_pending(0);
+        __syncthreads();  // the first two pieces' indices
+    }
+    issue(0);
+    issue(1);
+    for (int p = 0; p < pieces; ++p) {
+        cp_async_wait_pending(1);  // piece p, and the indices of piece p + 2
+        if (GATHER) {
+            fence_proxy_async_shared();  // the piece is read by a bulk copy
+            if (tid == 0) bulk_wait_read_0();  // piece p - 1 has been read: piece p + 2 takes its place
+        }
+        __syncthreads();
+        if (GATHER) {
+            const unsigned bytes = unsigned(rows_of(p)) * row_bytes;
+            if (bulk && (bytes & 15u) == 0 && s_bad[p % kIndexSlots] == 0) {
+                if (tid == 0) bulk_store(dst + (long long)p * per * m, piece_at(p), bytes);
+            } else {
+                drain(p);
+                __syncthreads();  // before the indices of piece p + 4 and the rows of piece p + 3 take its place
+            }
+            if (tid == 0) s_bad[(p + 3) % kIndexSlots] = 0;
+            issue(p + 2);
+        } else {
+            issue(p + 2);
+            drain(p);
+        }
+    }
+    cp_async_wait_pending(0);
+    if (GATHER && tid == 0) bulk_wait_read_0();  // the pieces are free for the next tile
+}
+
+// The same for 16-byte words.  Word q of a piece belongs to struct q / m; the
+// piece's indices are staged first (one coalesced read), invalid ones marked -1.
+template <class S, typename V, bool GATHER, int PF>
+__device__ void tile_index_wide(const V* src, V* dst, const int* idx, long long bound, long long first,
+                                  long long cnt, int m, unsigned char* stage, int* s_idx) {
+    constexpr int D = 2, kPiece = S::wide_piece, kSlots = S::wide_slots;
+    const int tid = opaque_tid();
+    // structs per piece: a multiple of 32 that fits the buffer and the index slots
+    int per = (kPiece / int(sizeof(V))) / m / 32 * 32;
+    if (per > kSlots) per = kSlots;
     // q / m for q < 2^12 and m <= 16 as a multiply and shift (exact there)
     const unsigned inv_m = (65536u + unsigned(m) - 1) / unsigned(m);
     const long long pieces = (cnt + per - 1) / per;
     auto issue = [&](long long p) {
         const int b = int(p % D);
-        V* buf = reinterpret_cast<V*>(stage + b * S::piece);
-        int* ix = s_idx + b * S::idx_slots;
+        V* buf = reinterpret_cast<V*>(stage + b * kPiece);
+        int* ix = s_idx + b * kSlots;
         const long long base = first + p * per;
         const int n_here = int(cnt - p * per < per ? cnt - p * per : per);
         const int words = n_here * m;
@@ -315,8 +472,8 @@ __device__ void tile_index_staged(const V* src, V* dst, const int* idx, long lon
     };
     auto drain = [&](long long p) {
         const int b = int(p % D);
-        const V* buf = reinterpret_cast<const V*>(stage + b * S::piece);
-        const int* ix = s_idx + b * S::idx_slots;
+        const V* buf = reinterpret_cast<const V*>(stage + b * kPiece);
+        const int* ix = s_idx + b * kSlots;
         const long long base = first + p * per;
         const int n_here = int(cnt - p * per < per ? cnt - p * per : per);
         const int words = n_here * m;
@@ -359,18 +516,18 @@ __device__ __forceinline__ void tile_index(const BatchTask& t, long long first, 
 }
 
 template <class S, bool GATHER, int PF>
-__device__ __forceinline__ void tile_staged_pf(const BatchTask& t, long long first, long long cnt, int m,
-                                               unsigned char* stage, int* s_idx) {
+__device__ __forceinline__ void tile_staged_pf(const BatchTask& t, long long first, int cnt, int m,
+                                               unsigned char* stage, int* s_idx, int* s_bad) {
     if (t.word_log2 == 4)
-        tile_index_staged<S, uint4, GATHER, PF>(reinterpret_cast<const uint4*>(t.src), reinterpret_cast<uint4*>(t.dst),
-                                                t.idx, t.bound, first, cnt, m, stage, s_idx);
+        tile_index_wide<S, uint4, GATHER, PF>(reinterpret_cast<const uint4*>(t.src), reinterpret_cast<uint4*>(t.dst),
+                                              t.idx, t.bound, first, cnt, m, stage, s_idx);
     else if (t.word_log2 == 3)
         tile_index_staged<S, uint2, GATHER, PF>(reinterpret_cast<const uint2*>(t.src), reinterpret_cast<uint2*>(t.dst),
-                                                t.idx, t.bound, first, cnt, m, stage, s_idx);
+                                                t.idx, t.bound, first, cnt, m, stage, s_idx, s_bad);
     else
         tile_index_staged<S, unsigned, GATHER, PF>(reinterpret_cast<const unsigned*>(t.src),
                                                    reinterpret_cast<unsigned*>(t.dst), t.idx, t.bound, first, cnt, m,
-                                                   stage, s_idx);
+                                                   stage, s_idx, s_bad);
 }
 
 // index_mode 2: staged with the context's fetch size; 3 / 4 (gathers): with
@@ -378,17 +535,17 @@ __device__ __forceinline__ void tile_staged_pf(const BatchTask& t, long long fir
 // register-held movers, index_mode 0 / 1 (register rows, plain or with the
 // 64-byte hint) are staged the same way: plain, or with the 64-byte hint.
 template <class S>
-__device__ __forceinline__ void tile_staged(const BatchTask& t, long long first, long long cnt, unsigned char* stage,
-                                            int* s_idx) {
+__device__ __forceinline__ void tile_staged(const BatchTask& t, long long first, int cnt, unsigned char* stage,
+                                            int* s_idx, int* s_bad) {
     const int m = t.words * 4 >> t.word_log2;
     if (t.op != TRV_OP_GATHER)
-        tile_staged_pf<S, false, 0>(t, first, cnt, m, stage, s_idx);
+        tile_staged_pf<S, false, 0>(t, first, cnt, m, stage, s_idx, s_bad);
     else if (t.index_mode == 3 || t.index_mode == 1)
-        tile_staged_pf<S, true, 64>(t, first, cnt, m, stage, s_idx);
+        tile_staged_pf<S, true, 64>(t, first, cnt, m, stage, s_idx, s_bad);
     else if (t.index_mode == 4)
-        tile_staged_pf<S, true, 128>(t, first, cnt, m, stage, s_idx);
+        tile_staged_pf<S, true, 128>(t, first, cnt, m, stage, s_idx, s_bad);
     else
-        tile_staged_pf<S, true, 0>(t, first, cnt, m, stage, s_idx);
+        tile_staged_pf<S, true, 0>(t, first, cnt, m, stage, s_idx, s_bad);
 }
 
 // Task of tile number `tile`: the last k with prefix[k] <= tile (tasks without
@@ -420,7 +577,8 @@ batch_kernel(const BatchTask* __restrict__ tasks, int ntasks, const long long* _
     __shared__ int s_lo;
     __shared__ __align__(8) unsigned long long s_bar[S::ring];
     extern __shared__ __align__(128) unsigned char s_stage[];  // S::dyn_smem bytes
-    int* s_idx = reinterpret_cast<int*>(s_stage + 2 * S::piece);
+    __shared__ int s_bad[kIndexSlots];
+    int* s_idx = reinterpret_cast<int*>(s_stage + kPieces * S::piece);
     unsigned long long seq = 0;  // thread 0: bulk loads issued so far
     if (threadIdx.x == 0) {
         for (int k = 0; k < S::ring; ++k) mbar_init(&s_bar[k], 1);
@@ -476,7 +634,7 @@ batch_kernel(const BatchTask* __restrict__ tasks, int ntasks, const long long* _
             // the 128-register build: rows staged through shared memory, or
             // held in registers (index_mode 0 / 1)
             if (t.index_mode >= 2)
-                tile_staged<S>(t, first, cnt, s_stage, s_idx);
+                tile_staged<S>(t, first, int(cnt), s_stage, s_idx, s_bad);
             else if (t.op == TRV_OP_GATHER)
                 tile_index<S, true>(t, first, cnt);
             else
@@ -487,7 +645,7 @@ batch_kernel(const BatchTask* __restrict__ tasks, int ntasks, const long long* _
             // as well made it spill (456 bytes a thread) in every path, and
             // without them the 4096-array batch runs 21.32 instead of 22.22 ms
             // (its gathers 10.90 instead of 11.73 ms).
-            tile_staged<S>(t, first, cnt, s_stage, s_idx);
+            tile_staged<S>(t, first, int(cnt), s_stage, s_idx, s_bad);
         }
     }
 }
