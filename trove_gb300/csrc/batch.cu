@@ -155,7 +155,6 @@ __device__ bool tile_copy_bulk(const unsigned char* s, unsigned char* d, long lo
             mbar_wait(&bar[k % S::ring], unsigned((k / S::ring) & 1));
         }
     }
-    bulk_wait_read_0();  // stages free for the next tile
     seq += (unsigned long long)issued;
     for (long long b = body; b < nbytes; ++b) d[b] = s[b];
     return ok;
@@ -430,7 +429,6 @@ __device__ void tile_index_staged(const V* src, V* dst, const int* idx, long lon
         }
     }
     cp_async_wait_pending(0);
-    if (GATHER && tid == 0) bulk_wait_read_0();  // the pieces are free for the next tile
 }
 
 // The same for 16-byte words.  Word q of a piece belongs to struct q / m; the
@@ -607,7 +605,10 @@ batch_kernel(const BatchTask* __restrict__ tasks, int ntasks, const long long* _
                     s_end = __ldg(tile_prefix + lo + 1);
                 }
             }
-            if (lane == 0) s_tile = tile;
+            if (lane == 0) {
+                s_tile = tile;
+                bulk_wait_read_0();  // the last tile's bulk copies have read the pieces: the next one may fill them
+            }
         }
         __syncthreads();
         const long long tile = s_tile;
