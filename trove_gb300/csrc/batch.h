@@ -41,6 +41,10 @@ struct TaskPlan {
 long long plan_task(int op, uint32_t width, uint64_t n, uint64_t bound, const void* src, void* dst,
                     const int32_t* idx, const TaskPlan& p, BatchTask* d);
 
+// Tile size of a task of a batch that moves `bytes` bytes of structs in all on
+// `blocks` resident blocks, where nothing else chooses it.
+int fit_tile_bytes(int op, double bytes, int blocks);
+
 // Option checks shared by trv_batch_create and trv_batch_run_static.
 int check_batch_options(const trv_batch_options* opt);
 

@@ -69,11 +69,24 @@ int validate(const trv_task& t) {
     return TRV_OK;
 }
 
-// Size rule when no tuned tile exists: big enough to amortise the queue
+// The largest tile when no tuned one exists: big enough to amortise the queue
 // step, small enough to balance the tail across 152 SMs.
 int default_tile_bytes(int op) { return op == TRV_OP_COPY ? (128 << 10) : (64 << 10); }
 
 }  // namespace
+
+// A block takes about 25 us for a 64 KiB tile of gathered rows, so a batch that
+// comes to a few tiles a block is as long as its last ones: four tiles to each
+// resident block where the batch is that small, down to 8 KiB, below which the
+// queue step is felt.  Batches in us at the largest tiles / 2 / 4 / 8 to a block:
+// 87 arrays of 2-64 K structs 48.9 / 36.9 / 33.1 / 38.9, 343 of 0.5-64 K 68.4 /
+// 69.0 / 62.3 / 56.2, 16 of 4-32 K 26.6 / 12.3 / 12.3 / 12.3; 225 of 256-1024
+// 10.6 / 9.6 / 9.2 / 9.3 at 8 KiB and 10.3-10.4 at 4 KiB.
+int fit_tile_bytes(int op, double bytes, int blocks) {
+    const int most = default_tile_bytes(op), least = 8 << 10;
+    const double want = bytes / (4.0 * blocks);
+    return want >= most ? most : want <= least ? least : int(want) / 1024 * 1024;
+}
 
 long long plan_task(int op, uint32_t width, uint64_t n, uint64_t bound, const void* src, void* dst,
                     const int32_t* idx, const TaskPlan& p, BatchTask* d) {
@@ -118,6 +131,8 @@ int plan_batch(const trv_task* tasks, uint64_t count, const trv_batch_options* o
     // bytes of gather / scatter tasks whose tuned entry prefers 2 / 4 blocks per
     // SM (their movers set the register budget; copy tiles barely use one)
     uint64_t vote2 = 0, vote4 = 0, total = 0;
+    double all = 0;  // bytes of structs, unchecked as yet
+    for (uint64_t k = 0; k < count; ++k) all += double(tasks[k].n) * tasks[k].width;
     prefix[0] = 0;
     for (uint64_t k = 0; k < count; ++k) {
         const trv_task& t = tasks[k];
@@ -128,7 +143,7 @@ int plan_batch(const trv_task* tasks, uint64_t count, const trv_batch_options* o
         TaskPlan p;
         p.tile_bytes = (opt && opt->tile_bytes > 0) ? opt->tile_bytes
                        : (tuned && c.tile_bytes > 0) ? c.tile_bytes
-                                                     : default_tile_bytes(t.op);
+                                                     : fit_tile_bytes(t.op, all, 4 * device_info().sm_count);
         // Gather and scatter rows are staged through shared memory with
         // cp.async unless chosen otherwise: on the 4096-array workload (4
         // blocks per SM) its gathers took 12.1 ms that way against 20.5 ms

@@ -295,13 +295,16 @@ struct trv_server {
             }
             const Tables h(s.h_tables, take), d(s.d_tables, take);
             long long tiles[2] = {0, 0};
+            double bytes[2] = {0, 0};
+            for (size_t k = 0; k < take; ++k) bytes[k < ns ? 0 : 1] += double(s.todo[k].first.n) * s.todo[k].first.width;
             for (size_t k = 0; k < take; ++k) {
                 const trv_request& r = s.todo[k].first;
+                const int grp = k < ns ? 0 : 1;
                 TuneChoice c;
                 const bool tuned = tune_lookup(TuneKey{SCOPE_BATCH, r.op, int(r.width), len_bucket(r.n)}, &c);
                 const int tb = cfg.tile_bytes > 0 ? cfg.tile_bytes
                                : (tuned && c.tile_bytes > 0) ? c.tile_bytes
-                                                             : (r.op == TRV_OP_COPY ? (128 << 10) : (64 << 10));
+                                                             : fit_tile_bytes(r.op, bytes[grp], grp ? grid_large : grid);
                 TaskPlan p;
                 p.tile_bytes = tb;
                 p.gather_policy = 7;  // rows staged through shared memory, 128-byte L2 fetches
@@ -309,7 +312,6 @@ struct trv_server {
                 p.copy_bulk = 1;
                 const long long nt = plan_task(r.op, r.width, r.n, r.src_n, r.src, arena.base() + s.todo[k].second,
                                                r.idx, p, &h.tasks[k]);
-                const int grp = k < ns ? 0 : 1;
                 h.prefix[k + size_t(grp)] = tiles[grp];
                 tiles[grp] += nt;
             }
