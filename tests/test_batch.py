@@ -391,3 +391,37 @@ def test_staged_rows_of_narrow_words(cuda, width):
                     h = dst.cpu().numpy()
                     assert np.array_equal(h[offset:offset + expect.size], expect.reshape(-1)), (blocks, skip, offset, expect.shape)
                     assert (h[:offset] == SENTINEL).all() and (h[offset + expect.size:] == SENTINEL).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("width", [8, 12, 36, 60, 64])
+def test_scatter_destinations_fetched_in_batches(cuda, width):
+    """Batches of more than 200 MB fetch a scatter's destination ahead of its rows:
+    destinations around the sizes where that begins (256 KiB) and the tile it is
+    done by (1 MiB), random and sorted indices, rows that stay untouched."""
+    torch = cuda
+    filler = (104 << 20) // 64
+    fsrc = torch.randint(0, 255, (filler * 64,), dtype=torch.uint8, device="cuda")
+    fdst = [torch.zeros_like(fsrc) for _ in range(2)]
+    tasks = [dict(op=tg.OP_COPY, width=64, n=filler, src=fsrc, dst=d) for d in fdst]
+    checks = []
+    for size in ((256 << 10) - width, (256 << 10) + width, 1 << 20, (1 << 20) + width, 5 << 20):
+        bound = size // width
+        n = bound - 3
+        src = torch.randint(0, 255, (n, width), dtype=torch.uint8, device="cuda")
+        for idx in (torch.randperm(bound, device="cuda")[:n].to(torch.int32), torch.arange(n, device="cuda", dtype=torch.int32)):
+            idx[7] = -1
+            idx[n - 2] = bound
+            dst = torch.full((bound + 2, width), SENTINEL, dtype=torch.uint8, device="cuda")
+            expect = dst.clone()
+            ok = (idx >= 0) & (idx < bound)
+            expect[1 + idx[ok].long()] = src[ok]
+            tasks.append(dict(op=tg.OP_SCATTER, width=width, n=n, src=src, dst=dst[1:], idx=idx, bound=bound))
+            checks.append((dst, expect))
+    for blocks in (0, 2):
+        for dst, _ in checks:
+            dst.fill_(SENTINEL)
+        tg.Batch(tasks, blocks_per_sm=blocks).launch()
+        for dst, expect in checks:
+            assert torch.equal(dst, expect)
+        assert all(torch.equal(d, fsrc) for d in fdst)

@@ -19,6 +19,7 @@
 
 #include "autotune.h"
 #include "batch.h"
+#include "fetch.cuh"
 #include "kernels.cuh"
 #include "runtime.h"
 #include "tma.cuh"
@@ -617,7 +618,17 @@ batch_kernel(const BatchTask* __restrict__ tasks, int ntasks, const long long* _
         __syncthreads();  // read before warp 0 writes the next tile's
         if (tile >= total) break;
         const BatchTask& t = tasks[lo];
-        const long long first = (tile - begin) * t.tile_structs;
+        if (tile - begin < t.fetch_tiles) {
+            const int row_bytes = 4 * t.words;
+            if (!IndexSample(t.idx, t.n, opaque_tid() & 31).local(row_bytes)) {
+                const unsigned long long p = reinterpret_cast<unsigned long long>(t.dst);
+                const unsigned long long part = p + (unsigned long long)(tile - begin) * kFetchTileBytes;
+                const unsigned long long end = p + (unsigned long long)t.bound * unsigned(row_bytes);
+                fetch_part(part, part + kFetchTileBytes < end ? part + kFetchTileBytes : end, 0, 1);
+            }
+            continue;
+        }
+        const long long first = (tile - begin - t.fetch_tiles) * t.tile_structs;
         const long long cnt = t.n - first < t.tile_structs ? t.n - first : t.tile_structs;
         const long long w = 4ll * t.words;
         if (t.op == TRV_OP_COPY) {

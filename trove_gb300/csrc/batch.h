@@ -20,13 +20,17 @@ struct alignas(16) BatchTask {
     int op;           // TRV_OP_*
     int words;        // struct width / 4
     int tile_structs; // structs per tile, a multiple of 32
-    int word_log2;    // gather / scatter: log2 of the word moved per lane (2, 3 or 4)
-    int index_mode;   // gather / scatter: 0 = rows held in registers, 1 = the same with the 64-byte
+    short word_log2;  // gather / scatter: log2 of the word moved per lane (2, 3 or 4)
+    short index_mode; // gather / scatter: 0 = rows held in registers, 1 = the same with the 64-byte
                       // L2 prefetch-size hint on random loads (gather), 2 = rows staged through
                       // shared memory with cp.async, 3 / 4 = staged with the 64 / 128-byte hint
                       // (gather)
     int copy_bulk;    // copy: 1 = TMA bulk tiles where 16-byte aligned, 0 = flat vector tiles
+    int fetch_tiles;  // scatter: the task's first tiles fetch its destination into L2, kFetchTileBytes each
 };
+static_assert(sizeof(BatchTask) == 64, "a task is two 32-byte sectors");
+
+constexpr long long kFetchTileBytes = 1 << 20;  // 256 threads, 4 KiB each
 
 // Per-task choices that are not in the task itself.
 struct TaskPlan {
@@ -35,6 +39,7 @@ struct TaskPlan {
                               // memory, 6 / 7 staged with the 64 / 128-byte hint
     int scatter_policy;       // 1 plain, 5 staged through shared memory
     int copy_bulk;            // copy tiles through the TMA bulk engine where aligned
+    bool fetch_scatters = false;  // scatter destinations are fetched into L2 ahead of their rows
 };
 
 // Fills one task-table entry from a validated task; returns its tile count.

@@ -88,6 +88,25 @@ int fit_tile_bytes(int op, double bytes, int blocks) {
     return want >= most ? most : want <= least ? least : int(want) / 1024 * 1024;
 }
 
+// Tiles that fetch a scatter task's destination ahead of its rows: where rows
+// leave sectors partly written, each such write that misses L2 is filled from
+// DRAM at the rate of random accesses (scatter_parts.cu), and in a batch larger
+// than L2 the destination is seldom there when its turn comes.  2^24 scattered
+// rows in arrays of 2^19, plain / fetched in us: 8 bytes 185 / 121, 12 bytes 242 /
+// 146, 20 bytes 335 / 203, 36 bytes 463 / 302; arrays of 72 and 80 MiB 531 / 430
+// and 410 / 334, but of 144 MiB, which L2 does not hold, 628 / 641.  A batch of
+// little more than L2 only pays for the tiles (343 arrays, 124 MB of structs, 62.6
+// / 64.3 us; 60 arrays, 300 MB, 161.3 / 157.0).
+constexpr uint64_t kFetchLeast = uint64_t(256) << 10, kFetchMost = uint64_t(100) << 20;
+constexpr double kFetchBatchBytes = 200e6;  // bytes of structs in the batch
+
+static int fetch_tiles(uint32_t width, uint64_t n, uint64_t bound, const void* dst) {
+    const uint64_t bytes = bound * width;
+    if (width < 8 || (width % 32 == 0 && (reinterpret_cast<uintptr_t>(dst) & 31u) == 0)) return 0;
+    if (n < 2 || 2 * n < bound || bytes < kFetchLeast || bytes > kFetchMost) return 0;
+    return int((bytes + kFetchTileBytes - 1) / kFetchTileBytes);
+}
+
 long long plan_task(int op, uint32_t width, uint64_t n, uint64_t bound, const void* src, void* dst,
                     const int32_t* idx, const TaskPlan& p, BatchTask* d) {
     long long tile = (long long)p.tile_bytes / width;
@@ -111,7 +130,8 @@ long long plan_task(int op, uint32_t width, uint64_t n, uint64_t bound, const vo
                     : op == TRV_OP_SCATTER ? (p.scatter_policy == 5 ? 2 : 0)
                                            : 0;
     d->copy_bulk = p.copy_bulk;
-    return ((long long)n + tile - 1) / tile;
+    d->fetch_tiles = op == TRV_OP_SCATTER && n > 0 && p.fetch_scatters ? fetch_tiles(width, n, bound, dst) : 0;
+    return ((long long)n + tile - 1) / tile + d->fetch_tiles;
 }
 
 int check_batch_options(const trv_batch_options* opt) {
@@ -159,6 +179,7 @@ int plan_batch(const trv_task* tasks, uint64_t count, const trv_batch_options* o
                                                         : 5;
         const int cp = (opt && opt->copy_path) ? opt->copy_path : (tuned && c.path) ? c.path : TRV_PATH_AUTO;
         p.copy_bulk = cp == TRV_PATH_VECTOR ? 0 : 1;
+        p.fetch_scatters = all > kFetchBatchBytes;
         prefix[k + 1] = prefix[k] + plan_task(t.op, t.width, t.n, t.bound, t.src, t.dst, t.idx, p, &out[k]);
         const uint64_t tb = 2 * t.n * t.width + (t.op == TRV_OP_COPY ? 0 : 4 * t.n);
         total += tb;

@@ -11,6 +11,7 @@
 //  - a destination larger than L2 is written in parts that fit, one pass each.
 #include <cuda_runtime.h>
 
+#include "fetch.cuh"
 #include "ops.h"
 
 namespace trv {
@@ -43,35 +44,6 @@ __device__ __forceinline__ unsigned ld_once(const unsigned* p, unsigned long lon
 }
 __device__ __forceinline__ int ld_once(const int* p, unsigned long long pol) {
     return int(ld_once(reinterpret_cast<const unsigned*>(p), pol));
-}
-
-// Whether indices mostly step from one row to the next (sorted, runs): then
-// the writes of neighbouring rows meet in L2 by themselves, and neither remedy
-// is needed.  Every warp takes the same 32 pairs of the index array, so every
-// warp of a launch comes to the same answer.
-struct IndexSample {
-    int a, b;
-    __device__ __forceinline__ IndexSample(const int* __restrict__ idx, long long n, int lane) {
-        const long long p = (long long)lane * (n - 1) >> 5;  // n >= 2
-        a = __ldg(idx + p);
-        b = __ldg(idx + p + 1);
-    }
-    __device__ __forceinline__ bool local(int row_bytes) const {
-        const long long d = (long long)b - a;
-        const bool near = (d < 0 ? -d : d) * row_bytes <= 256;
-        return __popc(__ballot_sync(0xFFFFFFFFu, near)) >= 20;
-    }
-};
-
-// Fetches [p0, p1) into L2: block c of `blocks`, 4 KiB an instruction.
-__device__ __forceinline__ void fetch_part(unsigned long long p0, unsigned long long p1, unsigned c, unsigned blocks) {
-    p0 = (p0 + 15) & ~15ull;
-    p1 &= ~15ull;
-    const unsigned long long step = (unsigned long long)blocks * blockDim.x * 4096;
-    for (unsigned long long p = p0 + ((unsigned long long)c * blockDim.x + threadIdx.x) * 4096; p < p1; p += step) {
-        const unsigned bytes = p1 - p < 4096 ? unsigned(p1 - p) : 4096u;
-        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-    }
 }
 
 // Ahead of a one-pass scatter: the whole destination.
