@@ -92,21 +92,29 @@ scatter_passes_kernel(const V* __restrict__ src, const int* __restrict__ idx, V*
     const int lane = int(threadIdx.x & 31u), warp = int(threadIdx.x >> 5);
     const unsigned long long row = (unsigned long long)m * sizeof(V);
     const IndexSample sample(idx, n, lane);
-    const unsigned pass = blockIdx.x / (plan.fetch + plan.body);
-    unsigned c = blockIdx.x - pass * (plan.fetch + plan.body);
-    unsigned lo = pass * plan.rows_per_pass;
-    unsigned rows = plan.bound - lo < plan.rows_per_pass ? plan.bound - lo : plan.rows_per_pass;
-    const bool local = sample.local(int(row));
-    if (local) {  // one pass over everything
-        if (pass != 0) return;
-        rows = plan.bound;
+    unsigned lo = 0, rows = plan.bound, c;
+    if (sample.local(int(row))) {  // one pass over everything
+        // The blocks to spare take about 1 ns each to leave.  Rows of 8- and
+        // 16-byte words are bound by DRAM: every passes-th block works, and the
+        // others leave meanwhile (2^24 sorted rows of 24 / 40 / 48 bytes 143 / 229
+        // / 261 us, 148 / 239 / 278 where they leave at the end).  Rows of 4-byte
+        // words are bound by instructions, and the first blocks work (2^24 of 36
+        // bytes 264 us against 278).
+        const unsigned step = sizeof(V) > 4 ? plan.passes : 1u;
+        c = blockIdx.x / step;
+        if (c * step != blockIdx.x || c >= plan.body) return;
+    } else {
+        const unsigned pass = blockIdx.x / (plan.fetch + plan.body);
+        c = blockIdx.x - pass * (plan.fetch + plan.body);
+        lo = pass * plan.rows_per_pass;
+        rows = plan.bound - lo < plan.rows_per_pass ? plan.bound - lo : plan.rows_per_pass;
+        if (c < plan.fetch) {
+            const unsigned long long p = reinterpret_cast<unsigned long long>(dst) + lo * row;
+            fetch_part(p, p + rows * row, c, plan.fetch);
+            return;
+        }
+        c -= plan.fetch;
     }
-    if (c < plan.fetch) {
-        const unsigned long long p = reinterpret_cast<unsigned long long>(dst) + lo * row;
-        if (!local) fetch_part(p, p + rows * row, c, plan.fetch);
-        return;
-    }
-    c -= plan.fetch;
     const unsigned long long pol = l2_evict_first_policy();
     const int step_j = 32 / m, step_r = 32 % m;
     int* to = s_to[warp];
@@ -163,7 +171,7 @@ constexpr int kFetchBlocks = 64;
 // enough to leave quickly where the indices are local, enough that two passes
 // overlap only briefly.  2^24 / 3 * 2^24 random rows of 24 bytes: 458 / 2073 us
 // at 608 (one resident wave), 406 / 1840 at 2048, 395 / 1793 at 4096; 2^24
-// sorted rows of 48 bytes: 264 / 277 / 331 us.
+// sorted rows of 48 bytes, the others leaving at the end: 264 / 277 / 331 us.
 constexpr int kBodyBlocks = 2048;
 
 template <typename V, int G>
