@@ -142,8 +142,9 @@ int32_t trv_copy_exit_ex(void* dst, const void* src, uint64_t n, uint32_t width,
 
 /* dst[i] = src[idx[i]] for i < n; idx[i] outside [0, src_n) is skipped.
  * Widths 4..64 in steps of 4 have per-width kernels; wider multiples of 4
- * use the row-form kernel with a run-time word count; other widths a
- * byte-wise kernel.
+ * use the row-form kernel with a run-time word count; other widths and
+ * addresses that are not 4-byte aligned move as aligned words, or byte by
+ * byte where rows are narrow and few.
  * Replaces the coalesced_ptr gather kernel (reference trove/ptr.h:76-90,
  * tests/benchmark.cu:90-99). */
 int32_t trv_gather(void* dst, const void* src, uint64_t src_n, const int32_t* idx, uint64_t n,

@@ -1,6 +1,6 @@
 // Width-agnostic kernels: the flat vector copy (TRV_PATH_VECTOR), the TMA
-// bulk copy (TRV_PATH_BULK), byte-wise gather/scatter for widths the struct
-// kernels do not cover, and the seeded input generator.
+// bulk copy (TRV_PATH_BULK), byte-wise gather/scatter of what neither the struct
+// kernels nor packed.cu take, and the seeded input generator.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -205,7 +205,7 @@ void launch_shift_copy(const void* src, void* dst, long long nbytes, const Shift
     }
 }
 
-// ---- byte-wise gather / scatter for widths outside 4..64 step 4 ----------
+// ---- byte-wise gather / scatter: rows too narrow or few for packed.cu ----
 __global__ void gather_bytes_kernel(const unsigned char* __restrict__ s, long long src_n,
                                     const int* __restrict__ idx, unsigned char* __restrict__ d, long long n,
                                     unsigned width) {
