@@ -70,15 +70,20 @@ int validate(const trv_task& t) {
 }
 
 // The largest tile when no tuned one exists: big enough to amortise the queue
-// step, small enough to balance the tail across 152 SMs.
-int default_tile_bytes(int op) { return op == TRV_OP_COPY ? (128 << 10) : (64 << 10); }
+// step and the filling of the pieces, small enough that the tiles in flight, and
+// with them the sources and destinations in use, stay in L2, and that the last
+// ones balance across 152 SMs.  512 arrays of 1 K-4 M structs (14.9 GB) in us at
+// 24 / 32 / 48 / 64 / 128 KiB: copies 1013 / 1015 / 1020 / 1026 / 1032, gathers
+// 1479 / 1390 / 1356 / 1370 / 1508, scatters 510 / 513 / 523 / 538 / 672; all of
+// them 2844 with 128, 64 and 64 KiB and 2803 with these.
+int default_tile_bytes(int op) { return op == TRV_OP_SCATTER ? (24 << 10) : (48 << 10); }
 
 }  // namespace
 
 // A block takes about 25 us for a 64 KiB tile of gathered rows, so a batch that
 // comes to a few tiles a block is as long as its last ones: four tiles to each
 // resident block where the batch is that small, down to 8 KiB, below which the
-// queue step is felt.  Batches in us at the largest tiles / 2 / 4 / 8 to a block:
+// queue step is felt.  Batches in us at 64 KiB (copies 128) / 2 / 4 / 8 to a block:
 // 87 arrays of 2-64 K structs 48.9 / 36.9 / 33.1 / 38.9, 343 of 0.5-64 K 68.4 /
 // 69.0 / 62.3 / 56.2, 16 of 4-32 K 26.6 / 12.3 / 12.3 / 12.3; 225 of 256-1024
 // 10.6 / 9.6 / 9.2 / 9.3 at 8 KiB and 10.3-10.4 at 4 KiB.
