@@ -505,6 +505,20 @@ def test_copy_between_alignments(cuda, shift):
                 assert np.array_equal(check_guards(buf, start, nbytes), src_h[soff:soff + nbytes]), (nbytes, doff, kw)
 
 
+@pytest.mark.parametrize("offset", [0, 3, 15])
+def test_copy_equal_alignment_short(cuda, offset):
+    """Copies whose addresses agree modulo 16, around the length up to which
+    a thread takes one vector; bytes around the destination stay."""
+    torch = cuda
+    n = (1 << 20) + 40
+    src_h = np.frombuffer(oracle.random_words(n // 4 + 16, offset).tobytes(), np.uint8)
+    src = to_dev(torch, src_h)
+    for nbytes in (16 - offset, 17, 4096 - offset, 4097, (1 << 20) - 1, 1 << 20, (1 << 20) + 1, n):
+        buf, start = guarded(torch, nbytes, offset=offset)
+        tg.copy(buf[start:], src[offset:], nbytes, 1)
+        assert np.array_equal(check_guards(buf, start, nbytes), src_h[offset:offset + nbytes]), nbytes
+
+
 @pytest.mark.parametrize("width,offset", [(68, 0), (68, 4), (80, 0), (96, 8), (132, 0), (200, 0), (256, 0), (1028, 0)])
 def test_index_ops_wide_default_route(cuda, width, offset):
     """Rows wider than 64 bytes as a plain call takes them, at the lengths where
