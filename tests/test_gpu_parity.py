@@ -563,17 +563,19 @@ def test_scatter_wide_rows_in_parts(cuda):
         assert torch.equal(dst, expect)
 
 
+@pytest.mark.parametrize("width", [8, 44])
 @pytest.mark.parametrize("modulus", [1, 2, 3, 6, 625, 640, 1 << 31, (1 << 31) + 1, 0xFFFFFFFE, 0xFFFFFFFF])
-def test_copy_exit_moduli(cuda, modulus):
+def test_copy_exit_moduli(cuda, modulus, width):
     """The exit predicate for odd, even, power-of-two and largest moduli, on words
     around every kind of multiple: the smallest, the largest, the wrap-around."""
     torch = cuda
-    width, n = 8, 40000
-    words = oracle.random_words(2 * n, modulus & 0xFFFF).astype(np.uint32).copy()
+    n = 40000
+    words = oracle.random_words(width // 4 * n, modulus & 0xFFFF).astype(np.uint32).copy()
+    first = words[::width // 4]
     edge = np.array([0, 1, modulus - 2, modulus - 1, modulus, 2 * modulus - 1, 0xFFFFFFFF, 0xFFFFFFFE, 1 << 31]) & 0xFFFFFFFF
-    words[0:36:4] = edge.astype(np.uint32)
-    near = (words[2000:4000].astype(np.uint64) // modulus) * modulus + modulus - 1
-    words[2000:4000] = (near & 0xFFFFFFFF).astype(np.uint32)
+    first[0:18:2] = edge.astype(np.uint32)
+    near = (first[2000:4000].astype(np.uint64) // modulus) * modulus + modulus - 1
+    first[2000:4000] = (near & 0xFFFFFFFF).astype(np.uint32)
     src_h = words.view(np.uint8).reshape(n, width)
     init = np.full(n * width, SENTINEL, np.uint8)
     expect, _ = oracle.copy_exit(init, src_h, n, width, modulus)

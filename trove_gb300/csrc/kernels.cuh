@@ -35,10 +35,14 @@ enum Api { API_WARP = 0, API_BLOCK = 1, API_DIRECT = 2 };
 // Montgomery, "Division by Invariant Integers using Multiplication", section 9).
 // Five instructions where the remainder of a run-time d took about twenty of
 // the 84 that 32 structs of 12 bytes cost: 1 GiB of 4 bytes 311 -> 305 us, of 12
-// bytes 321 -> 309, of 20 bytes 316 -> 307, of 24 bytes 301 -> 298.
+// bytes 321 -> 309, of 20 bytes 316 -> 307, of 24 bytes 301 -> 298.  Structs of an
+// odd number of words from 36 bytes up are bound by DRAM either way and keep the
+// remainder (36 bytes 301.2 us, 302.0 by multiplication; 44 bytes 300.7 and 301.6;
+// 60 bytes 300.9 and 301.4), even ones gain from 32 bytes on (305.0 -> 303.1).
 template <int S>
 __device__ __forceinline__ bool exits(const aos<S>& v, const ExitTest& t) {
     const unsigned w = unsigned(v.head);
+    if (S >= 9 && S % 2 == 1) return w % (t.low + 1u) == t.low;
     const unsigned x = (w - t.low) * t.inverse;
     return w >= t.low && __funnelshift_r(x, x, t.rotate) <= t.most;
 }
