@@ -487,6 +487,35 @@ def test_index_ops_packed(cuda, width):
                                                                                                          doff)
 
 
+@pytest.mark.parametrize("width,n", [(7, 65537), (7, 524291), (7, 1 << 20), (13, 32767), (13, 32768), (13, 131073),
+                                     (13, 786439), (13, 3145729), (29, 49153), (29, 1048577), (47, 131071), (47, 131072), (47, 524291),
+                                     (47, 2097153), (111, 393217), (111, 1048579), (217, 393216), (217, 393215)])
+def test_index_ops_packed_rows_to_a_warp(cuda, width, n):
+    """Packed rows at the lengths where the rows to a warp change: every chunk
+    size with a remainder, skipped rows, arrays at odd addresses."""
+    torch = cuda
+    raw = torch.zeros(n * width + 64, dtype=torch.uint8, device="cuda")
+    tg.fill_random_u32(raw, raw.numel() // 4, seed=width)
+    src = raw[3:3 + n * width]
+    perm = torch.empty(n, dtype=torch.int32, device="cuda")
+    tg.fill_permutation(perm, n, 5)
+    perm[::7] = -1
+    ok = perm >= 0
+    rows = src.view(n, width)
+    for scatter in (False, True):
+        buf = torch.full((n * width + 32,), SENTINEL, dtype=torch.uint8, device="cuda")
+        dst = buf[17:17 + n * width]
+        expect = torch.full((n, width), SENTINEL, dtype=torch.uint8, device="cuda")
+        if scatter:
+            tg.scatter(dst, n, src, perm, n, width)
+            expect[perm[ok].long()] = rows[ok]
+        else:
+            tg.gather(dst, src, n, perm, n, width)
+            expect[ok] = rows[perm[ok].long()]
+        assert torch.equal(dst.view(n, width), expect), scatter
+        assert bool((buf[:17] == SENTINEL).all()) and bool((buf[17 + n * width:] == SENTINEL).all()), scatter
+
+
 @pytest.mark.parametrize("shift", range(1, 16))
 def test_copy_between_alignments(cuda, shift):
     """Copies whose two addresses differ modulo 16, on both sides of the length

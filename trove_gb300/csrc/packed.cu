@@ -237,35 +237,55 @@ unsigned clamp_bound(long long n) { return n > 0x80000000ll ? 0x80000000u : unsi
 
 }  // namespace
 
-template <bool GATHER, int ROWS>
-static void launch(const void* src, const int* idx, void* dst, long long bound, long long n, int width, int grid,
-                   cudaStream_t st) {
+template <int ROWS>
+static void launch(bool gather, const void* src, const int* idx, void* dst, long long bound, long long n, int width,
+                   int grid, cudaStream_t st) {
     const unsigned char* s = static_cast<const unsigned char*>(src);
     unsigned char* d = static_cast<unsigned char*>(dst);
     if (grid <= 0) {
         const long long need = (n + kWarps * ROWS - 1) / (kWarps * ROWS);
         grid = need < 0x7FFFFFFFll ? int(need) : 0x7FFFFFFF;
     }
-    if (GATHER)
+    if (gather)
         gather_packed_kernel<ROWS><<<grid, 32 * kWarps, 0, st>>>(s, clamp_bound(bound), idx, d, n, width);
     else
         scatter_packed_kernel<ROWS><<<grid, 32 * kWarps, 0, st>>>(s, idx, d, clamp_bound(bound), n, width);
 }
 
+// Rows to a warp, 8 to 128.  More rows to a warp waste less on its start and its
+// last round of 32 words; fewer keep more warps busy where the rows are few, and
+// the wider the rows, the fewer make up a warp's work.  Random gathers in us at 8 /
+// 16 / 32 / 64 / 128: 2^16 rows of 13 bytes 4.5 / 3.7 / 4.1 / 5.6 / 8.9, 2^20 of them
+// 47.6 / 25.5 / 16.1 / 14.5 / 16.7, 2^22 185 / 96 / 57 / 47 / 45; 2^17 of 29 bytes 7.3
+// / 5.0 / 6.5 / 9.6 / 16.0, 2^20 48.8 / 29.5 / 25.6 / 25.6 / 30.4; 2^18 of 47 bytes
+// 14.9 / 12.3 / 12.8 / 18.1 / 31.0, 2^20 54.0 / 42.3 / 34.0 / 37.4 / 47.4; 2^20 of 217
+// bytes 142 / 127 / 133 / 156 / 202.  Scatters lie the same way (2^17 of 29 bytes 8.6
+// / 6.6 / 6.9 / 8.6 / 12.9; 2^20 of 47 bytes 75.5 / 63.4 / 59.9 / 61.1 / 66.9); sorted
+// ones of many rows want the most (2^20 of 7 bytes 51 / 27 / 14.6 / 13.6 / 11.8).
+static int rows_to_a_warp(int width, long long n) {
+    constexpr long long K = 1 << 10, M = 1 << 20, never = 1ll << 62;
+    constexpr long long from[6][4] = {  // the least n for 16, 32, 64 and 128 rows
+        {32 * K, 64 * K, 512 * K, 1 * M},   // up to 8 bytes
+        {32 * K, 128 * K, 768 * K, 3 * M},  // up to 16
+        {48 * K, 256 * K, 1 * M, 8 * M},    // up to 32
+        {128 * K, 512 * K, 2 * M, 6 * M},   // up to 64
+        {384 * K, 1 * M, never, never},     // up to 128
+        {384 * K, 2 * M, never, never}};
+    const long long* at = from[width <= 8 ? 0 : width <= 16 ? 1 : width <= 32 ? 2 : width <= 64 ? 3 : width <= 128 ? 4 : 5];
+    int rows = 8;
+    for (int k = 0; k < 4 && n >= at[k]; ++k) rows *= 2;
+    return rows;
+}
+
 void launch_index_packed(bool gather, const void* src, const int* idx, void* dst, long long bound, long long n,
                          int width, int grid, cudaStream_t st) {
-    // 128 rows are a whole number of 32-word rounds at any width; where the
-    // rows are few or wide, fewer to a warp keep more warps busy (gathers, us,
-    // at 8 / 32 rows: 2^16 of 217 bytes 15.4 / 40.3, 2^22 of them 553 / 472).
-    if (n < (width > 64 ? 1ll << 19 : 1ll << 15))
-        gather ? launch<true, 8>(src, idx, dst, bound, n, width, grid, st)
-               : launch<false, 8>(src, idx, dst, bound, n, width, grid, st);
-    else if (width > 64 || n < (1ll << 17))
-        gather ? launch<true, 32>(src, idx, dst, bound, n, width, grid, st)
-               : launch<false, 32>(src, idx, dst, bound, n, width, grid, st);
-    else
-        gather ? launch<true, 128>(src, idx, dst, bound, n, width, grid, st)
-               : launch<false, 128>(src, idx, dst, bound, n, width, grid, st);
+    switch (rows_to_a_warp(width, n)) {
+        case 8: return launch<8>(gather, src, idx, dst, bound, n, width, grid, st);
+        case 16: return launch<16>(gather, src, idx, dst, bound, n, width, grid, st);
+        case 32: return launch<32>(gather, src, idx, dst, bound, n, width, grid, st);
+        case 64: return launch<64>(gather, src, idx, dst, bound, n, width, grid, st);
+        default: return launch<128>(gather, src, idx, dst, bound, n, width, grid, st);
+    }
 }
 
 }  // namespace trv
