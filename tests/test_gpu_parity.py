@@ -592,6 +592,25 @@ def test_scatter_wide_rows_in_parts(cuda):
         assert torch.equal(dst, expect)
 
 
+@pytest.mark.parametrize("width", [(34 << 20) + 4, (8 << 20) + 4, 8 << 20])
+def test_scatter_rows_of_many_mebibytes_with_parts_asked_for(cuda, width):
+    """Rows so wide that the last ones of 512 lie beyond 4 GiB of 4-byte words' worth
+    of offset, and rows around the widest that go in parts: the row named by the one
+    valid index arrives, the others stay."""
+    torch = cuda
+    n, bound = 512, (64 << 20) // width + 2
+    src = torch.empty(n * width, dtype=torch.uint8, device="cuda")
+    row = torch.randint(0, 255, (width,), dtype=torch.uint8, device="cuda")
+    for at in (510, 3):
+        src[at * width:(at + 1) * width] = row
+        idx = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+        idx[at] = bound - 1
+        dst = torch.full((bound * width,), SENTINEL, dtype=torch.uint8, device="cuda")
+        tg.scatter(dst, bound, src, idx, n, width, path="warp", policy=6)
+        assert torch.equal(dst[(bound - 1) * width:], row)
+        assert bool((dst[:(bound - 1) * width] == SENTINEL).all())
+
+
 @pytest.mark.parametrize("width", [8, 44])
 @pytest.mark.parametrize("modulus", [1, 2, 3, 6, 625, 640, 1 << 31, (1 << 31) + 1, 0xFFFFFFFE, 0xFFFFFFFF])
 def test_copy_exit_moduli(cuda, modulus, width):

@@ -15,6 +15,7 @@
 #include "bulk.h"
 #include "flat.h"
 #include "ops.h"
+#include "rules.h"
 #include "runtime.h"
 #include "trove_gb300.h"
 
@@ -522,11 +523,11 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
         IndexArgs a{src, dst, idx, (long long)n, (long long)bound, c.cache_policy};
         if (!gather && c.cache_policy == 6 && n >= 2 && bound >= 1) {
             const uint64_t parts = std::min<uint64_t>(parts_of(bound * width), 64);
-            if (parts > 1) {
+            if (parts > 1 && uint32_t(m) <= kMostPassWords) {
                 launch_scatter_passes(wb, a, m, int(parts), st);
                 return check_launch();
             }
-            launch_fetch_destination(a, int(width), st);
+            if (parts == 1) launch_fetch_destination(a, int(width), st);
         }
         if (grid_req == 0 && (gather ? c.cache_policy == 4 || c.cache_policy == 5 : c.cache_policy != 2 && c.cache_policy != 3) &&
             launch_wide_rows(gather, wb, a, m, st))

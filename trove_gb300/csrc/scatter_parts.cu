@@ -13,6 +13,7 @@
 
 #include "fetch.cuh"
 #include "ops.h"
+#include "rules.h"
 
 namespace trv {
 namespace {
@@ -60,7 +61,8 @@ fetch_destination_kernel(const unsigned char* dst, long long bytes, const int* _
 // starts as the one before it drains; between two passes come the blocks that
 // fetch the next part.
 //
-// A warp reads the indices of a slab of kSlab structs (all loads in flight at
+// Rows have at most kMostPassWords words, which keeps the offsets in a slab below
+// 2^30.  A warp reads the indices of a slab of kSlab structs (all loads in flight at
 // once), compacts the ones of its pass into a list in shared memory, and moves
 // the listed structs with every lane busy: word q = l + 32k of the list's
 // words is word q % m of struct list[q / m].  A pass so reads the index array
@@ -71,8 +73,6 @@ fetch_destination_kernel(const unsigned char* dst, long long bytes, const int* _
 // in 233 us (one pass of the row-form kernel 544 us, three passes of it over
 // 64 MiB parts 380 us); of 24 bytes 406 us (one pass 717), of 48 bytes 682 us
 // (1147), of 60 bytes 916 us (1358).
-constexpr int kSlabRounds = 16;
-constexpr int kSlab = 32 * kSlabRounds;
 constexpr int kPassWarps = 8;
 
 struct PassPlan {
