@@ -85,11 +85,11 @@ typedef struct trv_launch {
                               3 as 1, random side kept in L2 (evict-last); 4 as 1, random-side
                               loads with a 64-byte L2 prefetch-size hint; 5 as 1, random-side
                               loads with a 128-byte L2 prefetch-size hint (gathers); 6 (scatters)
-                              as 1, onto a destination fetched into L2 first, in one pass or,
-                              above 64 MiB, in passes over 56 MiB parts of it, so that
-                              partial-sector writes meet and merge in L2 (the default for
-                              structs that do not fill whole 32-byte sectors onto
-                              destinations of 22 MiB to about 1.3 GiB) */
+                              the default: as 1, but onto destinations of 22 MiB to about
+                              1.3 GiB structs that do not fill whole 32-byte sectors go after
+                              the destination has been fetched into L2, in one pass or, above
+                              64 MiB, in passes over 56 MiB parts of it, so that partial-sector
+                              writes meet and merge in L2 */
 } trv_launch;
 
 const char* trv_status_string(int32_t status);

@@ -13,6 +13,10 @@ SHIM = """
 extern "C" {
 int slab() { return trv::kSlab; }
 unsigned most_pass_words() { return trv::kMostPassWords; }
+unsigned widest_in_parts() { return trv::kWidestInParts; }
+int parts(unsigned width, unsigned long long n, unsigned long long dst_n, int sectors) {
+    return trv::scatter_parts(width, n, dst_n, sectors, width > 64 && width % 4 == 0);
+}
 }
 """
 
@@ -25,6 +29,7 @@ def rules(tmp_path_factory):
                     str(d / "rules.so")], check=True)
     lib = ctypes.CDLL(str(d / "rules.so"))
     lib.most_pass_words.restype = ctypes.c_uint32
+    lib.parts.argtypes = [ctypes.c_uint32, ctypes.c_uint64, ctypes.c_uint64, ctypes.c_int]
     return lib
 
 
@@ -34,4 +39,20 @@ def test_rows_in_parts_keep_32_bit_offsets(rules):
     most = rules.most_pass_words()
     in_flight = 32 * 8  # words that a round of a warp covers
     assert rules.slab() * most + 2 * in_flight <= 2**31 - 1
-    assert most * 16 >= 200  # every width that goes in parts by default, in words of any size
+    assert rules.widest_in_parts() <= 4 * most
+
+
+def test_parts_follow_the_destination_not_the_entry(rules):
+    """What policy 6 comes to, whoever asked for it: nothing special on short
+    destinations, on ones that are mostly not written, on more parts than pay."""
+    for width in (4, 8, 12, 24, 48, 64):
+        assert rules.parts(width, 1 << 14, 1 << 14, 1) == 0  # fits L2
+        assert rules.parts(width, 1, 1, 1) == 0
+    assert rules.parts(12, 1 << 24, 1 << 24, 1) == 4
+    assert rules.parts(12, 1 << 24, 1 << 30, 1) == 0  # 64 parts of a destination that is mostly left alone
+    assert rules.parts(24, 5 << 24, 5 << 24, 1) == 0  # 35 parts
+    for width in (80, 256):
+        assert rules.parts(width, 1 << 17, 1 << 17, 1) == 0  # the fetch alone does not pay for wide rows
+    assert rules.parts(204, 1 << 22, 1 << 22, 1) == 0
+    assert rules.parts((34 << 20) + 4, 512, 3, 1) == 0
+    assert rules.parts(13, 1 << 21, 1 << 21, 0) == 1  # packed rows: one pass after the fetch

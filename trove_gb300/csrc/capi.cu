@@ -368,49 +368,6 @@ int32_t trv_copy_exit(void* dst, const void* src, uint64_t n, uint32_t width, ui
     return trv_copy_exit_ex(dst, src, n, width, modulus, &cfg, stream);
 }
 
-// In how many parts a scatter writes its destination (scatter_parts.cu): 0, as
-// one plain pass; 1, one pass after the destination has been fetched into L2;
-// more, a pass for each part.  Measured on GB300 with random permutations:
-//  - rows that fill whole 32-byte sectors need no fill: one plain pass;
-//  - up to about 22 MiB of destination L2 absorbs the partial sectors (2^20 rows
-//    of 20 bytes, 20 MiB: 15.1 us, 18.4 with the fetch; of 24 bytes, 24 MiB:
-//    23.1 against 18.8), and 4-byte rows gain nothing from the fetch alone (2^24:
-//    103 against 104 us);
-//  - up to 64 MiB one pass is still best (2^24 rows of 4 bytes, 64 MiB: 104 us,
-//    114 in two; 3 * 2^20 of 20 bytes, 60 MiB: 49.4 and 55.0);
-//  - parts of 48, 56 and 64 MiB: 2^24 rows of 24 bytes 406 / 409 / 429 us, of 60
-//    bytes 931 / 916 / 927, 5 * 2^24 of 16 bytes 2921 / 2820 / 2848;
-//  - a pass costs about 1 ns per index whatever it writes, so many parts lose
-//    again: 5 * 2^24 rows of 20 bytes in 29 parts 3548 us against 3812 plain, of
-//    24 bytes in 35 parts 4053 against 3853;
-//  - a destination most of whose rows are not written would be fetched for
-//    nothing.
-constexpr uint64_t kPlainScatterBytes = uint64_t(22) << 20;
-constexpr uint64_t kOnePassBytes = uint64_t(64) << 20;
-constexpr uint64_t kPartBytes = uint64_t(56) << 20;
-constexpr uint64_t kMostParts = 24;
-
-static uint64_t parts_of(uint64_t bytes) {
-    return bytes <= kOnePassBytes ? 1 : (bytes + kPartBytes - 1) / kPartBytes;
-}
-
-static int scatter_parts(uint32_t width, uint64_t n, uint64_t dst_n, const void* dst) {
-    const uint64_t bytes = dst_n * width;
-    if (bytes <= kPlainScatterBytes || 2 * n < dst_n) return 0;
-    if (width % 32 == 0 && aligned(dst, 32)) return 0;
-    const uint64_t parts = parts_of(bytes);
-    if (parts > kMostParts || (parts == 1 && width < 8)) return 0;
-    return int(parts);
-}
-
-// Of wide rows only the two sectors at the ends are filled, and the passes pay
-// later: random scatters plain / in parts in us, 2^20 rows of 80 bytes 47 / 53,
-// 2^21 121 / 104; 2^20 of 120 bytes 77 / 87, 2^21 180 / 149; 2^21 of 200 bytes
-// 241 / 224, 2^22 500 / 465; 2^22 of 228 bytes 616 / 600.
-static bool wide_parts_pay(uint32_t width, uint64_t n, uint64_t dst_n, const void* dst) {
-    return width <= 200 && dst_n >= (uint64_t(1) << 21) && scatter_parts(width, n, dst_n, dst) > 1;
-}
-
 // Structs per lane of the row-form kernels when the caller gives none.  A call
 // of at most 2^16 structs does not fill the GPU (2048 warps at one struct per
 // lane): more structs per lane only lengthen each warp (4096 structs of 28
@@ -485,23 +442,25 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
             c = trv_launch{t.path, t.unroll, 0, t.grid, 0, t.cache_policy};
         else if (structs)
             c = gather                                    ? trv_launch{TRV_PATH_WARP, 0, 0, 0, 0, gather_policy(width, n, bound)}
-                                                          : trv_launch{TRV_PATH_WARP, 0, 0, 0, 0,
-                                                                       scatter_parts(width, n, bound, dst) ? 6 : 1};
+                                                          : trv_launch{TRV_PATH_WARP, 0, 0, 0, 0, 6};
         else if (wide_words)
-            c = trv_launch{TRV_PATH_WARP, 0, 0, 0, 0,
-                           gather ? gather_policy(width, n, bound) : wide_parts_pay(width, n, bound, dst) ? 6 : 0};
+            c = trv_launch{TRV_PATH_WARP, 0, 0, 0, 0, gather ? gather_policy(width, n, bound) : 6};
         else
             c.path = TRV_PATH_VECTOR;
     }
     if (c.cache_policy < 0 || c.cache_policy > 6 || (gather && c.cache_policy == 6)) return TRV_ERR_INVALID_ARGUMENT;
     const int path = c.path;
     const int grid_req = c.grid_blocks;
+    // Policy 6 asks for parts where they pay on the destination at hand: a tuned
+    // entry does not know the destination's length.
+    const int parts = gather ? 0 : scatter_parts(width, n, bound, aligned(dst, 32), path == TRV_PATH_WARP && width > 64);
+    if (c.cache_policy == 6 && parts == 0) c.cache_policy = 1;
     if (path == TRV_PATH_VECTOR) {  // any width, any alignment
         const long long blocks = (long long)((n + 255) / 256);
         const int cap = device_info().sm_count * 8;
         const int g = grid_req > 0 ? grid_req : (blocks < cap ? int(blocks) : cap);
         if (width <= kMostPackedWidth && packed_words_pay(gather, width, n)) {
-            if (!gather && n >= 2 && c.path == TRV_PATH_VECTOR && scatter_parts(width, n, bound, dst) == 1)
+            if (parts == 1)
                 launch_fetch_destination(IndexArgs{src, dst, idx, (long long)n, (long long)bound, 1}, int(width), st);
             launch_index_packed(gather, src, idx, dst, (long long)bound, (long long)n, int(width),
                                 grid_req > 0 ? grid_req : grid_req < 0 ? cap : 0, st);
@@ -521,13 +480,9 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
             wb >>= 1;
         const int m = int(width / uint32_t(wb));
         IndexArgs a{src, dst, idx, (long long)n, (long long)bound, c.cache_policy};
-        if (!gather && c.cache_policy == 6 && n >= 2 && bound >= 1) {
-            const uint64_t parts = std::min<uint64_t>(parts_of(bound * width), 64);
-            if (parts > 1 && uint32_t(m) <= kMostPassWords) {
-                launch_scatter_passes(wb, a, m, int(parts), st);
-                return check_launch();
-            }
-            if (parts == 1) launch_fetch_destination(a, int(width), st);
+        if (c.cache_policy == 6) {
+            launch_scatter_passes(wb, a, m, parts, st);
+            return check_launch();
         }
         if (grid_req == 0 && (gather ? c.cache_policy == 4 || c.cache_policy == 5 : c.cache_policy != 2 && c.cache_policy != 3) &&
             launch_wide_rows(gather, wb, a, m, st))
@@ -558,12 +513,11 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
     int grid = 0;
     const bool once = one_chunk_per_warp((long long)n, ops->built_unroll[slot], grid_req, &grid);
     if (!once) grid = grid_for(k.func, (long long)n, 256 * ops->built_unroll[slot], 256, grid_req);
-    if (!gather && path == TRV_PATH_WARP && c.cache_policy == 6 && n >= 2 && bound >= 1) {  // in parts
+    if (path == TRV_PATH_WARP && c.cache_policy == 6) {
         const IndexArgs a{src, dst, idx, (long long)n, (long long)bound, 1, once};
-        const uint64_t parts = std::min<uint64_t>(parts_of(bound * width), 64);
         if (parts > 1) {
             const int wb = kp == &ops->scatter_rows[0][slot] ? ops->rows_word_bytes : 4;
-            launch_scatter_passes(wb, a, int(width) / wb, int(parts), st);
+            launch_scatter_passes(wb, a, int(width) / wb, parts, st);
         } else {
             launch_fetch_destination(a, int(width), st);
             k.launch(a, grid, 256, st);

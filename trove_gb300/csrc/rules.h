@@ -9,13 +9,50 @@ namespace trv {
 
 // ---- scatters in parts (scatter_parts.cu) ----------------------------------
 
-// Rows that a warp of the parts kernel takes at a time, and the widest rows, in
-// words moved, for which its offsets inside such a slab stay below 2^30 and so
-// within 32 bits.  Wider rows are scattered in one pass of the row kernels, whose
-// row offsets have 64 bits; with 8 MiB and more to a row there are no partial
-// sectors worth saving.
+// In how many parts a scatter writes its destination: 0, as one plain pass; 1,
+// one pass after the destination has been fetched into L2; more, a pass for each
+// part.  This is policy 6, asked for, tuned or by default.  `sectors`: the
+// destination is 32-byte aligned.  Measured on GB300 with random permutations:
+//  - rows that fill whole 32-byte sectors need no fill: one plain pass;
+//  - up to about 22 MiB of destination L2 absorbs the partial sectors (2^20 rows
+//    of 20 bytes, 20 MiB: 15.1 us, 18.4 with the fetch; of 24 bytes, 24 MiB:
+//    23.1 against 18.8), and 4-byte rows gain nothing from the fetch alone (2^24:
+//    103 against 104 us);
+//  - up to 64 MiB one pass is still best (2^24 rows of 4 bytes, 64 MiB: 104 us,
+//    114 in two; 3 * 2^20 of 20 bytes, 60 MiB: 49.4 and 55.0);
+//  - parts of 48, 56 and 64 MiB: 2^24 rows of 24 bytes 406 / 409 / 429 us, of 60
+//    bytes 931 / 916 / 927, 5 * 2^24 of 16 bytes 2921 / 2820 / 2848;
+//  - a pass costs about 1 ns per index whatever it writes, so many parts lose
+//    again: 5 * 2^24 rows of 20 bytes in 29 parts 3548 us against 3812 plain, of
+//    24 bytes in 35 parts 4053 against 3853;
+//  - a destination most of whose rows are not written would be fetched for
+//    nothing;
+//  - of rows wider than 64 bytes only the two sectors at the ends are filled, and
+//    the passes pay later: plain / in parts in us, 2^20 rows of 80 bytes 47 / 53,
+//    2^21 121 / 104; 2^20 of 120 bytes 77 / 87, 2^21 180 / 149; 2^21 of 200 bytes
+//    241 / 224, 2^22 500 / 465; 2^22 of 228 bytes 616 / 600.  The fetch alone they
+//    never take (`wide`: the row kernels' rows above 64 bytes, not packed ones).
+constexpr uint64_t kPlainScatterBytes = uint64_t(22) << 20;
+constexpr uint64_t kOnePassBytes = uint64_t(64) << 20;
+constexpr uint64_t kPartBytes = uint64_t(56) << 20;
+constexpr uint64_t kMostParts = 24;
+constexpr uint32_t kWidestInParts = 200;
+
+inline int scatter_parts(uint32_t width, uint64_t n, uint64_t dst_n, bool sectors, bool wide) {
+    const uint64_t bytes = dst_n * width;
+    if (n < 2 || bytes <= kPlainScatterBytes || 2 * n < dst_n) return 0;
+    if (width % 32 == 0 && sectors) return 0;
+    if (wide && (width > kWidestInParts || dst_n < (uint64_t(1) << 21))) return 0;
+    const uint64_t parts = bytes <= kOnePassBytes ? 1 : (bytes + kPartBytes - 1) / kPartBytes;
+    if (parts > kMostParts || (parts == 1 && (width < 8 || wide))) return 0;
+    return int(parts);
+}
+
+// Rows that a warp of the parts kernel takes at a time: its offsets inside such a
+// slab have 32 bits.
 constexpr int kSlabRounds = 16;
 constexpr int kSlab = 32 * kSlabRounds;
 constexpr uint32_t kMostPassWords = (1u << 30) / kSlab;
+static_assert(kWidestInParts / 4 <= kMostPassWords, "a slab of the widest rows that go in parts");
 
 }  // namespace trv

@@ -61,8 +61,7 @@ fetch_destination_kernel(const unsigned char* dst, long long bytes, const int* _
 // starts as the one before it drains; between two passes come the blocks that
 // fetch the next part.
 //
-// Rows have at most kMostPassWords words, which keeps the offsets in a slab below
-// 2^30.  A warp reads the indices of a slab of kSlab structs (all loads in flight at
+// A warp reads the indices of a slab of kSlab structs (all loads in flight at
 // once), compacts the ones of its pass into a list in shared memory, and moves
 // the listed structs with every lane busy: word q = l + 32k of the list's
 // words is word q % m of struct list[q / m].  A pass so reads the index array
