@@ -89,7 +89,10 @@ typedef struct trv_launch {
                               1.3 GiB structs that do not fill whole 32-byte sectors go after
                               the destination has been fetched into L2, in one pass or, above
                               64 MiB, in passes over 56 MiB parts of it, so that partial-sector
-                              writes meet and merge in L2 */
+                              writes meet and merge in L2.  With a grid given, the parts are
+                              launched one by one on that grid with `unroll` structs to a lane
+                              and nothing is fetched (rows above 64 bytes: one pass); otherwise
+                              the parts have a grid and a layout of their own */
 } trv_launch;
 
 const char* trv_status_string(int32_t status);

@@ -2,6 +2,8 @@
 the C ABI.  Sizes are small enough for the oracle to finish in seconds; the
 full-size workloads are checked through size-independent properties in
 test_gpu_fullsize.py."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -34,6 +36,32 @@ def check_guards(buf, start, nbytes):
     assert (h[:start] == SENTINEL).all(), "write before the destination"
     assert (h[start + nbytes:] == SENTINEL).all(), "write past the destination"
     return h[start:start + nbytes]
+
+
+class KernelNodeParams(ctypes.Structure):  # CUDA_KERNEL_NODE_PARAMS_v2
+    _fields_ = [("func", ctypes.c_void_p), ("grid", ctypes.c_uint * 3), ("block", ctypes.c_uint * 3),
+                ("shared", ctypes.c_uint), ("params", ctypes.c_void_p), ("extra", ctypes.c_void_p),
+                ("kern", ctypes.c_void_p), ("ctx", ctypes.c_void_p)]
+
+
+def launched_grids(torch, run):
+    """Blocks of each kernel that run() launches, read from a captured graph."""
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g):
+        run()
+    cu, graph = ctypes.CDLL("libcuda.so.1"), ctypes.c_void_p(g.raw_cuda_graph())
+    count = ctypes.c_size_t(0)
+    assert cu.cuGraphGetNodes(graph, None, ctypes.byref(count)) == 0
+    nodes = (ctypes.c_void_p * count.value)()
+    assert cu.cuGraphGetNodes(graph, nodes, ctypes.byref(count)) == 0
+    grids = []
+    for node in nodes:
+        kind, p = ctypes.c_int(-1), KernelNodeParams()
+        assert cu.cuGraphNodeGetType(ctypes.c_void_p(node), ctypes.byref(kind)) == 0
+        if kind.value == 0:  # a kernel
+            assert cu.cuGraphKernelNodeGetParams_v2(ctypes.c_void_p(node), ctypes.byref(p)) == 0
+            grids.append(p.grid[0])
+    return grids
 
 
 @pytest.mark.parametrize("width", WIDTHS)
@@ -424,6 +452,34 @@ def test_scatter_in_parts(cuda, width, offset):
                 buf, start = guarded(torch, bound * width, offset=offset)
                 tg.scatter(buf[start:], bound, src[offset:], idx, n, width, **kw)
                 assert np.array_equal(check_guards(buf, start, bound * width), expect.reshape(-1)), (bound, kw)
+
+
+@pytest.mark.parametrize("width", [12, 36, 48, 68])
+@pytest.mark.parametrize("grid,unroll", [(1, 0), (37, 2), (-1, 1)])
+def test_scatter_in_parts_on_a_requested_grid(cuda, width, grid, unroll):
+    """Policy 6 onto a little more than 128 MiB: what is launched is that grid, and
+    the rows arrive as on the default one."""
+    torch = cuda
+    bound = (128 << 20) // width + 1
+    n = (1 << 16) + 3 if grid == 1 else bound - 2
+    if grid == 1:
+        bound = 2 * n  # a few blocks: small enough to stay quick, one pass
+    src = torch.randint(0, 255, (n, width), dtype=torch.uint8, device="cuda")
+    idx = torch.randperm(bound, device="cuda")[:n].to(torch.int32)
+    idx[5], idx[n - 1] = -1, bound
+    ok = (idx >= 0) & (idx < bound)
+    expect = torch.full((bound, width), SENTINEL, dtype=torch.uint8, device="cuda")
+    expect[idx[ok].long()] = src[ok]
+    dst = torch.full((bound, width), SENTINEL, dtype=torch.uint8, device="cuda")
+
+    def run():
+        tg.scatter(dst, bound, src, idx, n, width, path="warp", policy=6, grid=grid,
+                   unroll=unroll if width <= 64 else 0)
+
+    run()
+    assert torch.equal(dst, expect)
+    grids = launched_grids(torch, run)
+    assert len(set(grids)) == 1 and (grid < 0 or grids[0] == grid), grids
 
 
 @pytest.mark.parametrize("n", [1, 2, 33, 4097])

@@ -480,7 +480,7 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
             wb >>= 1;
         const int m = int(width / uint32_t(wb));
         IndexArgs a{src, dst, idx, (long long)n, (long long)bound, c.cache_policy};
-        if (c.cache_policy == 6) {
+        if (c.cache_policy == 6 && grid_req == 0) {
             launch_scatter_passes(wb, a, m, parts, st);
             return check_launch();
         }
@@ -513,8 +513,17 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
     int grid = 0;
     const bool once = one_chunk_per_warp((long long)n, ops->built_unroll[slot], grid_req, &grid);
     if (!once) grid = grid_for(k.func, (long long)n, 256 * ops->built_unroll[slot], 256, grid_req);
+    if (path == TRV_PATH_WARP && c.cache_policy == 6 && grid_req != 0) {
+        // a requested grid is each part's, and the requested structs per lane too
+        for (int p = 0; p < parts; ++p) {
+            IndexArgs a{src, dst, idx, (long long)n, (long long)bound * (p + 1) / parts, 1};
+            a.lo = (long long)bound * p / parts;
+            k.launch(a, grid, 256, st);
+        }
+        return check_launch();
+    }
     if (path == TRV_PATH_WARP && c.cache_policy == 6) {
-        const IndexArgs a{src, dst, idx, (long long)n, (long long)bound, 1, once};
+        const IndexArgs a{src, dst, idx, (long long)n, (long long)bound, 1, 0, once};
         if (parts > 1) {
             const int wb = kp == &ops->scatter_rows[0][slot] ? ops->rows_word_bytes : 4;
             launch_scatter_passes(wb, a, int(width) / wb, parts, st);
@@ -524,7 +533,7 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
         }
         return check_launch();
     }
-    k.launch(IndexArgs{src, dst, idx, (long long)n, (long long)bound, c.cache_policy, once}, grid, 256, st);
+    k.launch(IndexArgs{src, dst, idx, (long long)n, (long long)bound, c.cache_policy, 0, once}, grid, 256, st);
     return check_launch();
 }
 

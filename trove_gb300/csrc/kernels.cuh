@@ -568,7 +568,8 @@ scatter_rows_once_kernel(const V* __restrict__ src, const int* __restrict__ idx,
 }
 
 // The grid-stride form with the policy given at run time: caller-chosen and
-// persistent grids, and cache policies 2 and 3.
+// persistent grids, and cache policies 2 and 3.  A scatter writes the rows
+// [lo, dst_n) of its destination.
 template <int S, typename V, int U>
 __global__ void __launch_bounds__(256)
 gather_rows_kernel(const V* __restrict__ src, long long src_n, const int* __restrict__ idx, V* __restrict__ dst,
@@ -608,8 +609,8 @@ gather_rows_kernel(const V* __restrict__ src, long long src_n, const int* __rest
 
 template <int S, typename V, int U>
 __global__ void __launch_bounds__(256)
-scatter_rows_kernel(const V* __restrict__ src, const int* __restrict__ idx, V* __restrict__ dst, long long dst_n,
-                    long long n, int policy) {
+scatter_rows_kernel(const V* __restrict__ src, const int* __restrict__ idx, V* __restrict__ dst, long long lo,
+                    long long dst_n, long long n, int policy) {
     constexpr int m = S * 4 / int(sizeof(V));
     const WarpGrid g;
     constexpr int CH = 32 * U;
@@ -620,7 +621,7 @@ scatter_rows_kernel(const V* __restrict__ src, const int* __restrict__ idx, V* _
         for (int u = 0; u < U; ++u) {
             const long long i = base + u * 32 + g.lane;
             const int v = i < n ? ld_index(idx + i, policy) : -1;
-            id[u] = (v >= 0 && (long long)v < dst_n) ? v : -1;
+            id[u] = ((long long)v >= lo && (long long)v < dst_n) ? v : -1;
         }
         V val[U][m];
         int to[U][m];

@@ -37,6 +37,7 @@ struct IndexArgs {
     long long n;
     long long bound;  // src_n for gather, dst_n for scatter
     int policy;       // cache policy of the row-form kernels
+    long long lo = 0; // grid-stride row-form scatter: only destinations in [lo, bound) are written
     bool once = false; // the grid covers every 32*unroll-struct chunk with one warp
 };
 

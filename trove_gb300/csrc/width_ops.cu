@@ -100,7 +100,7 @@ void launch_scatter_rows(const IndexArgs& a, int grid, int block, cudaStream_t s
         if (a.policy != 2 && a.policy != 3) return launch_scatter_once<V, U, 1>(a, grid, block, st);
     }
     scatter_rows_kernel<S, V, U><<<grid, block, 0, st>>>(static_cast<const V*>(a.src), a.idx,
-                                                         static_cast<V*>(a.dst), a.bound, a.n, a.policy);
+                                                         static_cast<V*>(a.dst), a.lo, a.bound, a.n, a.policy);
 }
 
 template <typename V, int k>
