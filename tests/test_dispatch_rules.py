@@ -4,6 +4,7 @@ import ctypes
 import subprocess
 from pathlib import Path
 
+import numpy as np
 import pytest
 
 CSRC = Path(__file__).resolve().parent.parent / "trove_gb300" / "csrc"
@@ -16,6 +17,16 @@ unsigned most_pass_words() { return trv::kMostPassWords; }
 unsigned widest_in_parts() { return trv::kWidestInParts; }
 int parts(unsigned width, unsigned long long n, unsigned long long dst_n, int sectors) {
     return trv::scatter_parts(width, n, dst_n, sectors, width > 64 && width % 4 == 0);
+}
+// whether the sample of idx says that the rows lie in order
+int local(const int* idx, long long n, int row_bytes) {
+    int near = 0;
+    for (int lane = 0; lane < trv::kSamples; ++lane) {
+        const long long p = trv::sample_position(lane, n);
+        if (p < 0 || p + 1 >= n) return -1;
+        near += trv::sample_near(idx[p], idx[p + 1], row_bytes);
+    }
+    return near >= trv::kNearPairs;
 }
 }
 """
@@ -30,6 +41,7 @@ def rules(tmp_path_factory):
     lib = ctypes.CDLL(str(d / "rules.so"))
     lib.most_pass_words.restype = ctypes.c_uint32
     lib.parts.argtypes = [ctypes.c_uint32, ctypes.c_uint64, ctypes.c_uint64, ctypes.c_int]
+    lib.local.argtypes = [ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int]
     return lib
 
 
@@ -56,3 +68,25 @@ def test_parts_follow_the_destination_not_the_entry(rules):
     assert rules.parts(204, 1 << 22, 1 << 22, 1) == 0
     assert rules.parts((34 << 20) + 4, 512, 3, 1) == 0
     assert rules.parts(13, 1 << 21, 1 << 21, 0) == 1  # packed rows: one pass after the fetch
+
+
+@pytest.mark.parametrize("n", [2, 3, 31, 225, 226, 4097, 1 << 16, (1 << 16) + 32, 1 << 20, (1 << 20) - 1])
+def test_sampled_order_of_indices(rules, n):
+    """Rows in order, backwards, with gaps and in shuffled runs of 8 to 4096 are
+    told from random ones, whatever power of two the array's length is."""
+    rng = np.random.default_rng(n)
+
+    def local(idx, row_bytes):
+        idx = np.ascontiguousarray(idx, np.int32)
+        return rules.local(idx.ctypes.data, len(idx), row_bytes)
+
+    order = np.arange(n)
+    for row_bytes in (12, 48, 200):
+        assert local(order, row_bytes) == local(order[::-1], row_bytes) == 1
+        assert local(np.sort(rng.permutation(4 * n)[:n]), row_bytes) == 1
+        for run in (8, 32, 128, 4096):
+            if n >= 32 * run and n % run == 0:
+                runs = rng.permutation(n // run)[:, None] * run + np.arange(run)
+                assert local(runs.reshape(-1), row_bytes) == 1, run
+        if n >= 1 << 16:
+            assert local(rng.permutation(n), row_bytes) == 0

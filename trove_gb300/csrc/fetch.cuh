@@ -5,6 +5,8 @@
 
 #include <cuda_runtime.h>
 
+#include "rules.h"
+
 namespace trv {
 
 // Whether indices mostly step from one row to the next (sorted, runs): then
@@ -14,14 +16,12 @@ namespace trv {
 struct IndexSample {
     int a, b;
     __device__ __forceinline__ IndexSample(const int* __restrict__ idx, long long n, int lane) {
-        const long long p = (long long)lane * (n - 1) >> 5;  // n >= 2
+        const long long p = sample_position(lane, n);  // n >= 2
         a = __ldg(idx + p);
         b = __ldg(idx + p + 1);
     }
     __device__ __forceinline__ bool local(int row_bytes) const {
-        const long long d = (long long)b - a;
-        const bool near = (d < 0 ? -d : d) * row_bytes <= 256;
-        return __popc(__ballot_sync(0xFFFFFFFFu, near)) >= 20;
+        return __popc(__ballot_sync(0xFFFFFFFFu, sample_near(a, b, row_bytes))) >= kNearPairs;
     }
 };
 

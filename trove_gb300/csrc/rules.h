@@ -5,6 +5,12 @@
 
 #include <cstdint>
 
+#ifdef __CUDACC__
+#define TRV_HOST_DEVICE __host__ __device__
+#else
+#define TRV_HOST_DEVICE
+#endif
+
 namespace trv {
 
 // ---- scatters in parts (scatter_parts.cu) ----------------------------------
@@ -46,6 +52,26 @@ inline int scatter_parts(uint32_t width, uint64_t n, uint64_t dst_n, bool sector
     const uint64_t parts = bytes <= kOnePassBytes ? 1 : (bytes + kPartBytes - 1) / kPartBytes;
     if (parts > kMostParts || (parts == 1 && (width < 8 || wide))) return 0;
     return int(parts);
+}
+
+// The sample that tells scatters onto large destinations how their indices lie
+// (fetch.cuh): lane k of a warp takes the indices at this position of n >= 2 and
+// at the next one.  32 positions spread over the array, each seven further off a
+// multiple of the array's 32nd than the one before: without that, in an array of a
+// power of two all pairs lay across the same place of every run of 32 (2^24 rows of
+// 48 bytes in shuffled runs of 32 were taken for random, 513 us against 268 plain).
+constexpr int kSamples = 32;
+TRV_HOST_DEVICE inline long long sample_position(int lane, long long n) {
+    const long long p = (long long)lane * (n - 1) / kSamples, back = 7ll * lane;
+    return p >= back ? p - back : p;
+}
+
+// Rows so near each other that their writes meet in L2 by themselves, and how
+// many of the pairs have to be near.
+constexpr int kNearBytes = 4096, kNearPairs = 20;
+TRV_HOST_DEVICE inline bool sample_near(int a, int b, int row_bytes) {
+    const long long d = (long long)b - a;
+    return (d < 0 ? -d : d) * row_bytes <= kNearBytes;
 }
 
 // Rows that a warp of the parts kernel takes at a time: its offsets inside such a
