@@ -454,7 +454,7 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
     // Policy 6 asks for parts where they pay on the destination at hand: a tuned
     // entry does not know the destination's length.
     const int parts = gather ? 0 : scatter_parts(width, n, bound, aligned(dst, 32), path == TRV_PATH_WARP && width > 64);
-    if (c.cache_policy == 6 && parts == 0) c.cache_policy = 1;
+    if (c.cache_policy == 6 && parts == 0) c.cache_policy = width > 64 ? 0 : 1;
     if (path == TRV_PATH_VECTOR) {  // any width, any alignment
         const long long blocks = (long long)((n + 255) / 256);
         const int cap = device_info().sm_count * 8;
