@@ -26,7 +26,7 @@ int local(const int* idx, long long n, int row_bytes) {
         if (p < 0 || p + 1 >= n) return -1;
         near += trv::sample_near(idx[p], idx[p + 1], row_bytes);
     }
-    return near >= trv::kNearPairs;
+    return near >= trv::near_pairs(row_bytes);
 }
 }
 """

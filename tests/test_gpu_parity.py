@@ -454,6 +454,38 @@ def test_scatter_in_parts(cuda, width, offset):
                 assert np.array_equal(check_guards(buf, start, bound * width), expect.reshape(-1)), (bound, kw)
 
 
+@pytest.mark.parametrize("mib", [41, 65, 130])
+@pytest.mark.parametrize("width", [8, 12, 24, 36, 48, 72, 13])
+def test_scatter_orders_of_indices(cuda, width, mib):
+    """Destinations that are fetched first and ones in two or more parts, with rows
+    in order, in shuffled runs, at random, at random within a tenth of the destination
+    (one part, or less than L2 holds) and few valid ones: whichever form the sample of
+    the indices picks, every valid row arrives and nothing else changes."""
+    torch = cuda
+    bound = (mib << 20) // width
+    n = bound - 3
+    src = torch.randint(0, 255, (n, width), dtype=torch.uint8, device="cuda")
+    order = torch.arange(n, device="cuda")
+    runs = (torch.randperm(n // 32, device="cuda")[:, None] * 32 + torch.arange(32, device="cuda")).reshape(-1)
+    tenth = bound // 10
+    inside = torch.full((n,), -1, device="cuda", dtype=torch.int64)
+    inside[torch.randperm(n, device="cuda")[:tenth]] = torch.randperm(tenth, device="cuda") + bound // 2
+    wide = torch.full((n,), -1, device="cuda", dtype=torch.int64)
+    wide[::3] = (torch.randperm(bound // 2, device="cuda") + bound // 4)[:(n + 2) // 3]
+    few = torch.full((n,), bound, device="cuda", dtype=torch.int64)
+    few[7] = bound - 1
+    for name, idx in (("order", order), ("runs", torch.cat([runs, order[runs.numel():]])),
+                      ("random", torch.randperm(bound, device="cuda")[:n]), ("inside", inside), ("wide", wide),
+                      ("few", few)):
+        idx = idx.to(torch.int32)
+        ok = (idx >= 0) & (idx < bound)
+        expect = torch.full((bound, width), SENTINEL, dtype=torch.uint8, device="cuda")
+        expect[idx[ok].long()] = src[ok]
+        dst = torch.full((bound, width), SENTINEL, dtype=torch.uint8, device="cuda")
+        tg.scatter(dst, bound, src, idx, n, width)
+        assert torch.equal(dst, expect), name
+
+
 @pytest.mark.parametrize("width", [12, 36, 48, 68])
 @pytest.mark.parametrize("grid,unroll", [(1, 0), (37, 2), (-1, 1)])
 def test_scatter_in_parts_on_a_requested_grid(cuda, width, grid, unroll):

@@ -21,7 +21,15 @@ struct IndexSample {
         b = __ldg(idx + p + 1);
     }
     __device__ __forceinline__ bool local(int row_bytes) const {
-        return __popc(__ballot_sync(0xFFFFFFFFu, sample_near(a, b, row_bytes))) >= kNearPairs;
+        return __popc(__ballot_sync(0xFFFFFFFFu, sample_near(a, b, row_bytes))) >= near_pairs(row_bytes);
+    }
+    // The rows [first, first + rows) that the sampled indices below `bound` lie in.
+    __device__ __forceinline__ void span(unsigned bound, unsigned& first, unsigned& rows) const {
+        const bool va = unsigned(a) < bound, vb = unsigned(b) < bound;
+        const unsigned lo = __reduce_min_sync(0xFFFFFFFFu, min(va ? unsigned(a) : bound, vb ? unsigned(b) : bound));
+        const unsigned hi = __reduce_max_sync(0xFFFFFFFFu, max(va ? unsigned(a) + 1 : 0u, vb ? unsigned(b) + 1 : 0u));
+        first = lo;
+        rows = hi > lo ? hi - lo : 0u;
     }
 };
 

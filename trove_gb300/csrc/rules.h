@@ -67,8 +67,10 @@ TRV_HOST_DEVICE inline long long sample_position(int lane, long long n) {
 }
 
 // Rows so near each other that their writes meet in L2 by themselves, and how
-// many of the pairs have to be near.
-constexpr int kNearBytes = 4096, kNearPairs = 20;
+// many of the pairs have to be near: of wide rows fewer, since parts give them less
+// (2^21 rows of 120 bytes of which half lie in order 126 us plain, 143 in parts).
+constexpr int kNearBytes = 4096;
+TRV_HOST_DEVICE inline int near_pairs(int row_bytes) { return row_bytes > 64 ? 12 : 20; }
 TRV_HOST_DEVICE inline bool sample_near(int a, int b, int row_bytes) {
     const long long d = (long long)b - a;
     return (d < 0 ? -d : d) * row_bytes <= kNearBytes;

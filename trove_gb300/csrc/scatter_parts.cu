@@ -47,13 +47,17 @@ __device__ __forceinline__ int ld_once(const int* p, unsigned long long pol) {
     return int(ld_once(reinterpret_cast<const unsigned*>(p), pol));
 }
 
-// Ahead of a one-pass scatter: the whole destination.
+// Ahead of a one-pass scatter: what the sampled indices span of the destination.
 __global__ void __launch_bounds__(256)
-fetch_destination_kernel(const unsigned char* dst, long long bytes, const int* __restrict__ idx, long long n,
+fetch_destination_kernel(const unsigned char* dst, unsigned bound, const int* __restrict__ idx, long long n,
                          int row_bytes) {
-    if (IndexSample(idx, n, int(threadIdx.x & 31u)).local(row_bytes)) return;
-    const unsigned long long p = reinterpret_cast<unsigned long long>(dst);
-    fetch_part(p, p + (unsigned long long)bytes, blockIdx.x, gridDim.x);
+    const IndexSample sample(idx, n, int(threadIdx.x & 31u));
+    if (sample.local(row_bytes)) return;
+    unsigned first, rows;
+    sample.span(bound, first, rows);
+    if (rows * (unsigned long long)unsigned(row_bytes) <= kPlainScatterBytes) return;
+    const unsigned long long p = reinterpret_cast<unsigned long long>(dst) + first * (unsigned long long)unsigned(row_bytes);
+    fetch_part(p, p + rows * (unsigned long long)unsigned(row_bytes), blockIdx.x, gridDim.x);
 }
 
 // Scatter in passes: pass p moves the rows whose index lies in the p-th part
@@ -82,6 +86,64 @@ struct PassPlan {
     unsigned fetch;          // blocks that fetch a part
 };
 
+// Every row in one pass, where the sample says that the parts have nothing to
+// give.  The rows are read in their own order, whatever their indices.  A launch
+// with its most blocks to a part works in slabs with as many blocks as one part
+// has; the others take about 1 ns each to leave, so for rows of 8- and 16-byte
+// words, which are bound by DRAM, every passes-th block works and the others leave
+// meanwhile (2^24 sorted rows of 24 / 40 / 48 bytes 143 / 229 / 261 us, 148 / 239 /
+// 278 where they leave at the end; of 36 bytes, bound by instructions, 278 and 264
+// where the first blocks work).  On fewer rows, slabs would come to hardly more
+// than a wave of blocks, and all blocks take kOrderRows rows to a warp (200 MiB of
+// sorted rows of 80 bytes 83 us in slabs, 68 so, 66 plain).
+constexpr int kOrderRows = 128;
+constexpr int kBodyBlocks = 2048;  // blocks that move a part's structs, at most (launch_passes)
+
+template <typename V, int G>
+__device__ __forceinline__ void scatter_in_order(const V* __restrict__ src, const int* __restrict__ idx,
+                                                 V* __restrict__ dst, long long n, int m, const PassPlan& plan, int* to,
+                                                 unsigned long long pol, int lane, int warp) {
+    const bool slabs = plan.body == kBodyBlocks;
+    const unsigned each = slabs && sizeof(V) > 4 ? plan.passes : 1u;
+    const unsigned c = blockIdx.x / each, blocks = slabs ? plan.body : gridDim.x;
+    if (c * each != blockIdx.x || c >= blocks) return;
+    const int rows = slabs ? kSlab : kOrderRows;
+    const int step_j = 32 / m, step_r = 32 % m;
+    for (long long base = ((long long)c * kPassWarps + warp) * rows; base < n;
+         base += (long long)blocks * kPassWarps * rows) {
+        const int rem = n - base < rows ? int(n - base) : rows;
+        __syncwarp();  // the previous rows' list has been read
+        for (int t0 = lane; t0 < rem; t0 += 128) {
+            int v[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) v[t] = t0 + 32 * t < rem ? ld_once(idx + base + t0 + 32 * t, pol) : -1;
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+                if (t0 + 32 * t < rem) to[t0 + 32 * t] = unsigned(v[t]) < plan.bound ? v[t] : -1;
+        }
+        __syncwarp();
+        const V* from = src + base * m;
+        const int words = rem * m;
+        int j = lane / m, r = lane % m;
+        for (int q = lane; q < words; q += 32 * G) {
+            V val[G];
+#pragma unroll
+            for (int g = 0; g < G; ++g)
+                if (q + 32 * g < words) val[g] = ld_once(from + q + 32 * g, pol);
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                if (q + 32 * g < words && to[j] >= 0) dst[(long long)to[j] * m + r] = val[g];
+                j += step_j;
+                r += step_r;
+                if (r >= m) {
+                    r -= m;
+                    ++j;
+                }
+            }
+        }
+    }
+}
+
 template <typename V, int G>
 __global__ void __launch_bounds__(32 * kPassWarps)
 scatter_passes_kernel(const V* __restrict__ src, const int* __restrict__ idx, V* __restrict__ dst, long long n, int m,
@@ -91,32 +153,39 @@ scatter_passes_kernel(const V* __restrict__ src, const int* __restrict__ idx, V*
     const int lane = int(threadIdx.x & 31u), warp = int(threadIdx.x >> 5);
     const unsigned long long row = (unsigned long long)m * sizeof(V);
     const IndexSample sample(idx, n, lane);
-    unsigned lo = 0, rows = plan.bound, c;
-    if (sample.local(int(row))) {  // one pass over everything
-        // The blocks to spare take about 1 ns each to leave.  Rows of 8- and
-        // 16-byte words are bound by DRAM: every passes-th block works, and the
-        // others leave meanwhile (2^24 sorted rows of 24 / 40 / 48 bytes 143 / 229
-        // / 261 us, 148 / 239 / 278 where they leave at the end).  Rows of 4-byte
-        // words are bound by instructions, and the first blocks work (2^24 of 36
-        // bytes 264 us against 278).
-        const unsigned step = sizeof(V) > 4 ? plan.passes : 1u;
-        c = blockIdx.x / step;
-        if (c * step != blockIdx.x || c >= plan.body) return;
-    } else {
-        const unsigned pass = blockIdx.x / (plan.fetch + plan.body);
-        c = blockIdx.x - pass * (plan.fetch + plan.body);
-        lo = pass * plan.rows_per_pass;
-        rows = plan.bound - lo < plan.rows_per_pass ? plan.bound - lo : plan.rows_per_pass;
-        if (c < plan.fetch) {
-            const unsigned long long p = reinterpret_cast<unsigned long long>(dst) + lo * row;
-            fetch_part(p, p + rows * row, c, plan.fetch);
-            return;
-        }
-        c -= plan.fetch;
-    }
+    unsigned first, spanned;
+    sample.span(plan.bound, first, spanned);
+    int* to = s_to[warp];
     const unsigned long long pol = l2_evict_first_policy();
     const int step_j = 32 / m, step_r = 32 % m;
-    int* to = s_to[warp];
+    if (sample.local(int(row)) || spanned * row <= kPlainScatterBytes) {
+        scatter_in_order<V, G>(src, idx, dst, n, m, plan, to, pol, lane, warp);
+        return;
+    }
+    const unsigned pass = blockIdx.x / (plan.fetch + plan.body);
+    unsigned c = blockIdx.x - pass * (plan.fetch + plan.body);
+    unsigned passes = plan.passes, step = plan.rows_per_pass;
+    if (spanned < plan.bound / 4 * 3) {
+        // All of the sample within three quarters of the destination (of 64 rows at
+        // random, one time in a million): as many parts as those rows need, the
+        // outer ones with what lies outside.
+        passes = (spanned + plan.rows_per_pass - 1) / plan.rows_per_pass;
+        if (pass >= passes) return;
+        step = (spanned + passes - 1) / passes;
+    } else {
+        first = 0;
+    }
+    unsigned lo = first + pass * step;
+    unsigned end = plan.bound - lo < step ? plan.bound : lo + step;
+    if (c < plan.fetch) {
+        const unsigned long long p = reinterpret_cast<unsigned long long>(dst);
+        fetch_part(p + lo * row, p + end * row, c, plan.fetch);
+        return;
+    }
+    if (pass == 0) lo = 0;
+    if (pass == passes - 1) end = plan.bound;
+    const unsigned rows = end - lo;
+    c -= plan.fetch;
     unsigned short* at = s_at[warp];
     for (long long base = ((long long)c * kPassWarps + warp) * kSlab; base < n;
          base += (long long)plan.body * kPassWarps * kSlab) {
@@ -166,12 +235,10 @@ scatter_passes_kernel(const V* __restrict__ src, const int* __restrict__ idx, V*
 }
 
 constexpr int kFetchBlocks = 64;
-// Blocks that move a pass's structs, at most (more slabs run in a loop): few
-// enough to leave quickly where the indices are local, enough that two passes
-// overlap only briefly.  2^24 / 3 * 2^24 random rows of 24 bytes: 458 / 2073 us
-// at 608 (one resident wave), 406 / 1840 at 2048, 395 / 1793 at 4096; 2^24
+// kBodyBlocks: few enough to leave quickly where the indices are local, enough that
+// two passes overlap only briefly.  2^24 / 3 * 2^24 random rows of 24 bytes: 458 /
+// 2073 us at 608 (one resident wave), 406 / 1840 at 2048, 395 / 1793 at 4096; 2^24
 // sorted rows of 48 bytes, the others leaving at the end: 264 / 277 / 331 us.
-constexpr int kBodyBlocks = 2048;
 
 template <typename V, int G>
 void launch_passes(const IndexArgs& a, int m, int passes, cudaStream_t st) {
@@ -189,8 +256,8 @@ void launch_passes(const IndexArgs& a, int m, int passes, cudaStream_t st) {
 }  // namespace
 
 void launch_fetch_destination(const IndexArgs& a, int row_bytes, cudaStream_t st) {
-    fetch_destination_kernel<<<kFetchBlocks, 256, 0, st>>>(static_cast<const unsigned char*>(a.dst),
-                                                           a.bound * row_bytes, a.idx, a.n, row_bytes);
+    fetch_destination_kernel<<<kFetchBlocks, 256, 0, st>>>(static_cast<const unsigned char*>(a.dst), unsigned(a.bound > 0x80000000ll ? 0x80000000ll : a.bound),
+                                                           a.idx, a.n, row_bytes);
 }
 
 void launch_scatter_passes(int word_bytes, const IndexArgs& a, int m, int passes, cudaStream_t st) {
