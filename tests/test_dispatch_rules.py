@@ -60,14 +60,17 @@ def test_parts_follow_the_destination_not_the_entry(rules):
     for width in (4, 8, 12, 24, 48, 64):
         assert rules.parts(width, 1 << 14, 1 << 14, 1) == 0  # fits L2
         assert rules.parts(width, 1, 1, 1) == 0
+        assert rules.parts(width, (34 << 20) // width, (34 << 20) // width, 1) == 0
     assert rules.parts(12, 1 << 24, 1 << 24, 1) == 4
     assert rules.parts(12, 1 << 24, 1 << 30, 1) == 0  # 64 parts of a destination that is mostly left alone
     assert rules.parts(24, 5 << 24, 5 << 24, 1) == 0  # 35 parts
     for width in (80, 256):
         assert rules.parts(width, 1 << 17, 1 << 17, 1) == 0  # the fetch alone does not pay for wide rows
-    assert rules.parts(204, 1 << 22, 1 << 22, 1) == 0
+    assert rules.parts(80, 1 << 20, 1 << 21, 1) == 0  # half of the rows written: too few to a pass
+    assert rules.parts(200, 1 << 22, 1 << 22, 1) == 0
     assert rules.parts((34 << 20) + 4, 512, 3, 1) == 0
-    assert rules.parts(13, 1 << 21, 1 << 21, 0) == 1  # packed rows: one pass after the fetch
+    for width in (12, 13, 24, 48):  # one pass after the fetch
+        assert rules.parts(width, (41 << 20) // width, (41 << 20) // width, 0) == 1
 
 
 @pytest.mark.parametrize("n", [2, 3, 31, 225, 226, 4097, 1 << 16, (1 << 16) + 32, 1 << 20, (1 << 20) - 1])

@@ -20,10 +20,13 @@ namespace trv {
 // part.  This is policy 6, asked for, tuned or by default.  `sectors`: the
 // destination is 32-byte aligned.  Measured on GB300 with random permutations:
 //  - rows that fill whole 32-byte sectors need no fill: one plain pass;
-//  - up to about 22 MiB of destination L2 absorbs the partial sectors (2^20 rows
-//    of 20 bytes, 20 MiB: 15.1 us, 18.4 with the fetch; of 24 bytes, 24 MiB:
-//    23.1 against 18.8), and 4-byte rows gain nothing from the fetch alone (2^24:
-//    103 against 104 us);
+//  - up to 40 MiB of destination L2 absorbs the partial sectors of a destination
+//    that it may still hold from its last use: plain / with the fetch in us, three
+//    destinations in turn and one that is not in L2, of 24 bytes 24 MiB 12 / 18 and
+//    29 / 25, 32 MiB 16 / 24 and 39 / 29, 40 MiB 26 / 29 and 47 / 33, 48 MiB 48 / 32
+//    and 57 / 43; of 8 bytes 32 MiB 25 / 32, 40 MiB 39 / 41, 48 MiB 69 / 46; of 48
+//    bytes 32 MiB 15 / 22, 40 MiB 24 / 25, 48 MiB 32 / 28.  The fetch costs rows in
+//    order 2 us.  4-byte rows gain nothing from it (2^24: 103 against 104 us);
 //  - up to 64 MiB one pass is still best (2^24 rows of 4 bytes, 64 MiB: 104 us,
 //    114 in two; 3 * 2^20 of 20 bytes, 60 MiB: 49.4 and 55.0);
 //  - parts of 48, 56 and 64 MiB: 2^24 rows of 24 bytes 406 / 409 / 429 us, of 60
@@ -35,20 +38,21 @@ namespace trv {
 //    nothing;
 //  - of rows wider than 64 bytes only the two sectors at the ends are filled, and
 //    the passes pay later: plain / in parts in us, 2^20 rows of 80 bytes 47 / 53,
-//    2^21 121 / 104; 2^20 of 120 bytes 77 / 87, 2^21 180 / 149; 2^21 of 200 bytes
-//    241 / 224, 2^22 500 / 465; 2^22 of 228 bytes 616 / 600.  The fetch alone they
-//    never take (`wide`: the row kernels' rows above 64 bytes, not packed ones).
-constexpr uint64_t kPlainScatterBytes = uint64_t(22) << 20;
+//    2^21 121 / 104; 2^20 of 120 bytes 77 / 87, 2^21 180 / 149; 400 MiB of 132 bytes
+//    337 / 276, of 200 bytes 241 / 225 and, where half of them lie in order, 185 /
+//    225: wider than 136 bytes they stay plain.  The fetch alone they never take
+//    (`wide`: the row kernels' rows above 64 bytes, not packed ones).
+constexpr uint64_t kPlainScatterBytes = uint64_t(40) << 20;
 constexpr uint64_t kOnePassBytes = uint64_t(64) << 20;
 constexpr uint64_t kPartBytes = uint64_t(56) << 20;
 constexpr uint64_t kMostParts = 24;
-constexpr uint32_t kWidestInParts = 200;
+constexpr uint32_t kWidestInParts = 136;
 
 inline int scatter_parts(uint32_t width, uint64_t n, uint64_t dst_n, bool sectors, bool wide) {
     const uint64_t bytes = dst_n * width;
     if (n < 2 || bytes <= kPlainScatterBytes || 2 * n < dst_n) return 0;
     if (width % 32 == 0 && sectors) return 0;
-    if (wide && (width > kWidestInParts || dst_n < (uint64_t(1) << 21))) return 0;
+    if (wide && (width > kWidestInParts || n < (uint64_t(1) << 21))) return 0;
     const uint64_t parts = bytes <= kOnePassBytes ? 1 : (bytes + kPartBytes - 1) / kPartBytes;
     if (parts > kMostParts || (parts == 1 && (width < 8 || wide))) return 0;
     return int(parts);
