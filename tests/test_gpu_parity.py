@@ -454,6 +454,43 @@ def test_scatter_in_parts(cuda, width, offset):
                 assert np.array_equal(check_guards(buf, start, bound * width), expect.reshape(-1)), (bound, kw)
 
 
+@pytest.mark.parametrize("where", ["dst", "src", "idx"])
+@pytest.mark.parametrize("width", [12, 80])
+def test_scatter_with_host_memory_is_one_plain_pass(cuda, width, where):
+    torch = cuda
+    n = (1 << 21) + 3 if width == 80 else (65 << 20) // width
+    src = torch.randint(0, 255, (n, width), dtype=torch.uint8)
+    idx = torch.randperm(n).to(torch.int32)
+    expect = torch.empty_like(src)
+    expect[idx.long()] = src
+    side = {"src": src, "idx": idx, "dst": torch.zeros_like(src)}
+    side = {k: t.pin_memory() if k == where else t.cuda() for k, t in side.items()}
+
+    def run():
+        tg.scatter(side["dst"], n, side["src"], side["idx"], n, width)
+
+    run()
+    torch.cuda.synchronize()
+    assert torch.equal(side["dst"].cpu(), expect)
+    on_gpu = {k: t.cuda() for k, t in side.items()}
+    assert len(launched_grids(torch, run)) == 1
+    rows = launched_grids(torch, run)[0]
+    passes = launched_grids(torch, lambda: tg.scatter(on_gpu["dst"], n, on_gpu["src"], on_gpu["idx"], n, width))
+    assert passes != [rows]
+
+
+@pytest.mark.parametrize("src_at,dst_at", [(4, 0), (8, 4), (1, 0)])
+def test_copy_to_host_memory_between_alignments(cuda, src_at, dst_at):
+    torch = cuda
+    nbytes = (1 << 20) + 5
+    src = torch.randint(0, 255, (nbytes + 64,), dtype=torch.uint8, device="cuda")
+    dst = torch.zeros(nbytes + 64, dtype=torch.uint8).pin_memory()
+    tg.copy(dst.data_ptr() + dst_at, src.data_ptr() + src_at, nbytes, 1)
+    torch.cuda.synchronize()
+    assert torch.equal(dst[dst_at:dst_at + nbytes], src[src_at:src_at + nbytes].cpu())
+    assert not dst[:dst_at].any() and not dst[dst_at + nbytes:].any()
+
+
 @pytest.mark.parametrize("mib", [41, 65, 130])
 @pytest.mark.parametrize("width", [8, 12, 24, 36, 48, 72, 13])
 def test_scatter_orders_of_indices(cuda, width, mib):

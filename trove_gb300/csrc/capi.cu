@@ -151,6 +151,18 @@ namespace {
 
 bool aligned(const void* p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
 
+// Whether p lies in this GPU's own memory: what is read or written again and again,
+// or counts on L2, is not worth it over the link to host memory or another GPU.
+// (The question takes about 0.1 us; only calls of tens of microseconds ask it.)
+bool on_this_gpu(const void* p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == device_info().device;
+}
+
 bool size_ok(uint64_t n, uint32_t width) { return width != 0 && n <= (uint64_t(1) << 62) / width; }
 
 bool struct_width(uint32_t width) { return width % 4 == 0 && width >= 4 && width <= 64; }
@@ -159,7 +171,9 @@ bool struct_width(uint32_t width) { return width % 4 == 0 && width >= 4 && width
 // from this length on: 1 MiB shared 4-byte alignment 1.73 us by words and 1.81
 // joined, odd addresses 2.6 by bytes and 1.8 joined; 64 KiB 1.6 and 1.7.  Short
 // ones take one vector to a thread (1 MiB: 1.8 us at 1, 2.07 at 4; 16 MiB: 7.6
-// and 7.1).
+// and 7.1).  Host memory is written faster by words than by joined vectors (144 MB
+// that share 4-byte alignment 391 us by words, 440 joined), but not by bytes (524
+// and 438).
 constexpr uint64_t kShiftCopyBytes = uint64_t(512) << 10;
 constexpr uint64_t kShortShiftBytes = uint64_t(4) << 20;
 
@@ -177,7 +191,7 @@ int copy_flat(void* dst, const void* src, uint64_t nbytes, int unroll, int grid_
     const int asked = unroll;
     if (unroll <= 0) unroll = vec == 16 && nbytes <= kShortFlatBytes ? 1 : 4;
     if (unroll_slot(unroll) < 0) return TRV_ERR_INVALID_ARGUMENT;
-    if (vec < 16 && nbytes >= kShiftCopyBytes) {
+    if (vec < 16 && nbytes >= kShiftCopyBytes && (vec < 4 || on_this_gpu(dst))) {
         const ShiftPlan p = plan_shift_copy(src, dst, (long long)nbytes);
         const int u = asked > 0 ? std::min(asked, 4) : nbytes < kShortShiftBytes ? 1 : 4;
         launch_shift_copy(src, dst, (long long)nbytes, p, u,
@@ -453,7 +467,10 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
     const int grid_req = c.grid_blocks;
     // Policy 6 asks for parts where they pay on the destination at hand: a tuned
     // entry does not know the destination's length.
-    const int parts = gather ? 0 : scatter_parts(width, n, bound, aligned(dst, 32), path == TRV_PATH_WARP && width > 64);
+    // Each part reads the indices and much of the source again, which host memory is
+    // too far away for (3 * 2^20 rows of 24 bytes from there 361 us, 652 in parts).
+    int parts = gather ? 0 : scatter_parts(width, n, bound, aligned(dst, 32), path == TRV_PATH_WARP && width > 64);
+    if (parts && !(on_this_gpu(dst) && on_this_gpu(src) && on_this_gpu(idx))) parts = 0;
     if (c.cache_policy == 6 && parts == 0) c.cache_policy = width > 64 ? 0 : 1;
     if (path == TRV_PATH_VECTOR) {  // any width, any alignment
         const long long blocks = (long long)((n + 255) / 256);
