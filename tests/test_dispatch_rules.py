@@ -16,8 +16,11 @@ int slab() { return trv::kSlab; }
 unsigned most_pass_words() { return trv::kMostPassWords; }
 unsigned widest_in_parts() { return trv::kWidestInParts; }
 int parts(unsigned width, unsigned long long n, unsigned long long dst_n, int sectors) {
-    return trv::scatter_parts(width, n, dst_n, sectors, width > 64 && width % 4 == 0);
+    return trv::scatter_parts(width, n, dst_n, sectors,
+                              width % 4 ? trv::kPackedRows : width > 64 ? trv::kWideRows : trv::kStructRows);
 }
+int packed(int gather, unsigned width, unsigned long long n) { return trv::packed_form(gather, width, n); }
+unsigned least_packed() { return trv::kLeastPackedWidth; }
 // whether the sample of idx says that the rows lie in order
 int local(const int* idx, long long n, int row_bytes) {
     int near = 0;
@@ -41,6 +44,7 @@ def rules(tmp_path_factory):
     lib = ctypes.CDLL(str(d / "rules.so"))
     lib.most_pass_words.restype = ctypes.c_uint32
     lib.parts.argtypes = [ctypes.c_uint32, ctypes.c_uint64, ctypes.c_uint64, ctypes.c_int]
+    lib.packed.argtypes = [ctypes.c_int, ctypes.c_uint32, ctypes.c_uint64]
     lib.local.argtypes = [ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int]
     return lib
 
@@ -93,3 +97,16 @@ def test_sampled_order_of_indices(rules, n):
                 assert local(runs.reshape(-1), row_bytes) == 1, run
         if n >= 1 << 16:
             assert local(rng.permutation(n), row_bytes) == 0
+
+
+def test_packed_words_only_where_they_are_right(rules):
+    """A word has bytes of two rows at most and reads at most eight bytes past a row."""
+    assert 2 * rules.least_packed() >= 8 and rules.least_packed() + 1 > 4
+    for gather in (0, 1):
+        for n in (1, 1 << 16, 1 << 20, 1 << 28):
+            for width in (1, 2, 3, (1 << 20) + 1, 2**32 - 1):
+                assert rules.packed(gather, width, n) == 0
+    # long scatters of narrow rows: a thread per row where a sample finds them in order
+    for width, n, scatter, gather in [(6, 1 << 12, 0, 0), (6, 1 << 18, 1, 0), (8, 1 << 20, 2, 1), (10, 1 << 20, 1, 1),
+                                      (11, 1 << 16, 1, 0), (13, 16, 1, 1)]:
+        assert (rules.packed(0, width, n), rules.packed(1, width, n)) == (scatter, gather), width

@@ -612,6 +612,50 @@ def test_index_ops_packed(cuda, width):
                                                                                                          doff)
 
 
+@pytest.mark.parametrize("width", [6, 7, 8, 9, 10, 11, 13, 30, 33, 47])
+def test_index_ops_packed_orders_of_indices(cuda, width):
+    """Rows in order, backwards, in shuffled runs, with most of them skipped, and all
+    of these in one array: rows that go by bytes, by words, and by what the sample of
+    the indices says."""
+    torch = cuda
+    for n in (100, 70003, (1 << 20) + 7):
+        src = torch.randint(0, 255, (n * width + 8,), dtype=torch.uint8, device="cuda")
+        rows = src[1:1 + n * width].view(n, width)
+        order = torch.arange(n, device="cuda")
+        few = torch.full((n,), -1, device="cuda", dtype=torch.int64)
+        few[::11] = torch.randperm(n, device="cuda")[:few[::11].numel()]
+        mixed = torch.randperm(n, device="cuda")
+        mixed[n // 3:n // 2] = few[n // 3:n // 2]
+        free = torch.ones(n, dtype=torch.bool, device="cuda")  # rows that mixed's first third does not name
+        free[mixed[:n // 3]] = False
+        mixed[n // 2:] = torch.where(free[order[n // 2:]], order[n // 2:], torch.full_like(order[n // 2:], n))
+        for name, idx in (("order", order), ("back", order.flip(0)), ("few", few),
+                          ("runs", torch.cat([(torch.randperm(n // 32, device="cuda")[:, None] * 32 + torch.arange(
+                              32, device="cuda")).reshape(-1), order[n // 32 * 32:]])), ("mixed", mixed)):
+            ok = (idx >= 0) & (idx < n)
+            i32 = idx.to(torch.int32)
+            expect = torch.full((n, width), SENTINEL, dtype=torch.uint8, device="cuda")
+            expect[ok] = rows[idx[ok]]
+            dst = torch.full((n * width + 8,), SENTINEL, dtype=torch.uint8, device="cuda")
+            tg.gather(dst[3:], rows, n, i32, n, width)
+            assert torch.equal(dst[3:3 + n * width].view(n, width), expect), ("gather", n, name)
+            assert bool((dst[:3] == SENTINEL).all()) and bool((dst[3 + n * width:] == SENTINEL).all())
+            if name == "mixed":  # no row twice: few's part may repeat one of the others
+                seen = torch.zeros(n + 1, dtype=torch.bool, device="cuda")
+                seen[torch.cat([idx[:n // 3], idx[n // 2:]])] = True
+                mid = idx[n // 3:n // 2]
+                idx = idx.clone()
+                idx[n // 3:n // 2] = torch.where((mid >= 0) & ~seen[mid.clamp(min=0)], mid, torch.full_like(mid, -1))
+                ok = (idx >= 0) & (idx < n)
+                i32 = idx.to(torch.int32)
+            expect = torch.full((n, width), SENTINEL, dtype=torch.uint8, device="cuda")
+            expect[idx[ok]] = rows[ok]
+            dst = torch.full((n * width + 8,), SENTINEL, dtype=torch.uint8, device="cuda")
+            tg.scatter(dst[2:], n, rows, i32, n, width)
+            assert torch.equal(dst[2:2 + n * width].view(n, width), expect), ("scatter", n, name)
+            assert bool((dst[:2] == SENTINEL).all()) and bool((dst[2 + n * width:] == SENTINEL).all())
+
+
 @pytest.mark.parametrize("width,n", [(7, 65537), (7, 524291), (7, 1 << 20), (13, 32767), (13, 32768), (13, 131073),
                                      (13, 786439), (13, 3145729), (29, 49153), (29, 1048577), (47, 131071), (47, 131072), (47, 524291),
                                      (47, 2097153), (111, 393217), (111, 1048579), (217, 393216), (217, 393215)])

@@ -421,19 +421,6 @@ static int gather_policy(uint32_t width, uint64_t n, uint64_t src_n) {
     return width >= 12 && src_n * width <= kL2SourceBytes && 2 * n >= src_n ? 5 : 4;
 }
 
-// Rows of any width and alignment move in 4-byte words (packed.cu) where that
-// beats a thread per row moving bytes.  Random rows, bytes / words in us: gathers
-// of 29 bytes 6.5 / 2.8 for 2^12, of 13 bytes 4.8 / 3.9 for 2^16, of 6 bytes 5.1
-// / 5.6 for 2^18 and 16.4 / 9.5 for 2^20.  Scatters of 13 bytes 4.9 / 2.4 for
-// 2^12, of 6 bytes 3.1 / 2.9 for 2^12 and 5.7 / 4.0 for 2^16.  Sorted indices
-// favour the bytes for longer (2^20 of 6 bytes: gather 7.5 / 8.0, scatter 7.5 /
-// 11.4; of 13 bytes 29.7 / 18.9 and 29.9 / 20.5), and below 6 bytes most words
-// straddle rows.
-static bool packed_words_pay(bool gather, uint32_t width, uint64_t n) {
-    if (gather) return width >= 13 || (width >= 6 && n >= (1u << 19));
-    return width >= 13 || (width >= 6 && n >= (1u << 16));
-}
-
 // Without a tuned entry, struct gathers and scatters take the row-form path,
 // streaming the index and contiguous side; scatters onto large destinations
 // run in parts (policy 6).
@@ -469,24 +456,28 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
     // entry does not know the destination's length.
     // Each part reads the indices and much of the source again, which host memory is
     // too far away for (3 * 2^20 rows of 24 bytes from there 361 us, 652 in parts).
-    int parts = gather ? 0 : scatter_parts(width, n, bound, aligned(dst, 32), path == TRV_PATH_WARP && width > 64);
+    const RowKind kind = path == TRV_PATH_VECTOR ? kPackedRows : width > 64 ? kWideRows : kStructRows;
+    int parts = gather ? 0 : scatter_parts(width, n, bound, aligned(dst, 32), kind);
     if (parts && !(on_this_gpu(dst) && on_this_gpu(src) && on_this_gpu(idx))) parts = 0;
     if (c.cache_policy == 6 && parts == 0) c.cache_policy = width > 64 ? 0 : 1;
     if (path == TRV_PATH_VECTOR) {  // any width, any alignment
         const long long blocks = (long long)((n + 255) / 256);
         const int cap = device_info().sm_count * 8;
         const int g = grid_req > 0 ? grid_req : (blocks < cap ? int(blocks) : cap);
-        if (width <= kMostPackedWidth && packed_words_pay(gather, width, n)) {
+        const PackedForm form = packed_form(gather, width, n);
+        const bool sampled = form == kBySample;
+        if (form != kByBytes) {
             if (parts == 1)
                 launch_fetch_destination(IndexArgs{src, dst, idx, (long long)n, (long long)bound, 1}, int(width), st);
             launch_index_packed(gather, src, idx, dst, (long long)bound, (long long)n, int(width),
-                                grid_req > 0 ? grid_req : grid_req < 0 ? cap : 0, st);
-            return check_launch();
+                                grid_req > 0 ? grid_req : grid_req < 0 ? cap : 0, sampled, st);
         }
-        if (gather)
-            launch_gather_bytes(src, (long long)bound, idx, dst, (long long)n, width, g, st);
-        else
-            launch_scatter_bytes(src, idx, dst, (long long)bound, (long long)n, width, g, st);
+        if (form != kByWords) {
+            if (gather)
+                launch_gather_bytes(src, (long long)bound, idx, dst, (long long)n, width, g, st);
+            else
+                launch_scatter_bytes(src, idx, dst, (long long)bound, (long long)n, width, g, sampled, st);
+        }
         return check_launch();
     }
     if (path != TRV_PATH_COALESCED && path != TRV_PATH_DIRECT && path != TRV_PATH_WARP) return TRV_ERR_UNSUPPORTED;

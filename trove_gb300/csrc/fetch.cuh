@@ -23,6 +23,12 @@ struct IndexSample {
     __device__ __forceinline__ bool local(int row_bytes) const {
         return __popc(__ballot_sync(0xFFFFFFFFu, sample_near(a, b, row_bytes))) >= near_pairs(row_bytes);
     }
+    // Whether neighbouring lanes' rows mostly lie in the same sectors, or hardly any
+    // are valid: then a thread per row does best for narrow rows.
+    __device__ __forceinline__ bool rows_adjoin(int row_bytes) const {
+        const long long d = (long long)b - a;
+        return __popc(__ballot_sync(0xFFFFFFFFu, (d < 0 ? -d : d) * row_bytes <= 64)) >= 20;
+    }
     // The rows [first, first + rows) that the sampled indices below `bound` lie in.
     __device__ __forceinline__ void span(unsigned bound, unsigned& first, unsigned& rows) const {
         const bool va = unsigned(a) < bound, vb = unsigned(b) < bound;

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fetch.cuh"
 #include "flat.h"
 
 namespace trv {
@@ -205,7 +206,7 @@ void launch_shift_copy(const void* src, void* dst, long long nbytes, const Shift
     }
 }
 
-// ---- byte-wise gather / scatter: rows too narrow or few for packed.cu ----
+// ---- byte-wise gather / scatter: rows too narrow or few for packed.cu -------
 __global__ void gather_bytes_kernel(const unsigned char* __restrict__ s, long long src_n,
                                     const int* __restrict__ idx, unsigned char* __restrict__ d, long long n,
                                     unsigned width) {
@@ -221,7 +222,8 @@ __global__ void gather_bytes_kernel(const unsigned char* __restrict__ s, long lo
 
 __global__ void scatter_bytes_kernel(const unsigned char* __restrict__ s, const int* __restrict__ idx,
                                      unsigned char* __restrict__ d, long long dst_n, long long n,
-                                     unsigned width) {
+                                     unsigned width, bool sampled) {
+    if (sampled && !IndexSample(idx, n, int(threadIdx.x & 31u)).rows_adjoin(int(width))) return;
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         const int j = idx[i];
@@ -239,9 +241,9 @@ void launch_gather_bytes(const void* src, long long src_n, const int* idx, void*
 }
 
 void launch_scatter_bytes(const void* src, const int* idx, void* dst, long long dst_n, long long n,
-                          unsigned width, int grid, cudaStream_t st) {
+                          unsigned width, int grid, bool sampled, cudaStream_t st) {
     scatter_bytes_kernel<<<grid, 256, 0, st>>>(static_cast<const unsigned char*>(src), idx,
-                                               static_cast<unsigned char*>(dst), dst_n, n, width);
+                                               static_cast<unsigned char*>(dst), dst_n, n, width, sampled);
 }
 
 }  // namespace trv

@@ -45,16 +45,17 @@ void launch_shift_copy(const void* src, void* dst, long long nbytes, const Shift
                        cudaStream_t st);
 const void* shift_copy_func();
 
-// Gather / scatter of structs of `width` bytes (at most kMostPackedWidth) at any
-// alignment (packed.cu).  grid 0: one chunk per warp.
-constexpr unsigned kMostPackedWidth = 1u << 20;
+// Gather / scatter of structs of `width` bytes (kLeastPackedWidth to
+// kMostPackedWidth, rules.h) at any alignment (packed.cu).  grid 0: one chunk per
+// warp.  sampled: a scatter of n >= 2 that leaves where its rows lie in order.
 void launch_index_packed(bool gather, const void* src, const int* idx, void* dst, long long bound, long long n,
-                         int width, int grid, cudaStream_t st);
+                         int width, int grid, bool sampled, cudaStream_t st);
 
-// The same byte by byte, one thread to a row: wider structs.
+// The same byte by byte, one thread to a row, any width.  sampled: leaves where the
+// other does not.
 void launch_gather_bytes(const void* src, long long src_n, const int* idx, void* dst, long long n,
                          unsigned width, int grid, cudaStream_t st);
 void launch_scatter_bytes(const void* src, const int* idx, void* dst, long long dst_n, long long n,
-                          unsigned width, int grid, cudaStream_t st);
+                          unsigned width, int grid, bool sampled, cudaStream_t st);
 
 }  // namespace trv

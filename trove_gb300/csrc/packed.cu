@@ -1,9 +1,10 @@
-// Gather / scatter of structs of any width at any alignment (packed records:
-// 3, 6, 13 bytes, or 4-byte widths at odd addresses), in 4-byte words.
+// Gather / scatter of structs of any width from kLeastPackedWidth bytes up at any
+// alignment (packed records: 6, 13 bytes, or 4-byte widths at odd addresses), in
+// 4-byte words.
 //
 // The contiguous side is dealt out by aligned 32-bit words, so a warp reads or
 // writes whole sectors of it; the four bytes of a word come from one row, or
-// where it straddles a row's end from two (or more, below 4 bytes a row).  The
+// where it straddles a row's end from two.  The
 // random side is read as the aligned words that hold the bytes, joined by a
 // funnel shift.  Bytes that no full word covers (a row's ends on the random
 // side of a scatter, skipped rows, the ends of the arrays) move one by one, and
@@ -16,6 +17,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fetch.cuh"
 #include "flat.h"
 
 namespace trv {
@@ -166,9 +168,10 @@ gather_packed_kernel(const unsigned char* __restrict__ src, unsigned bound, cons
 template <int kRows>
 __global__ void __launch_bounds__(32 * kWarps)
 scatter_packed_kernel(const unsigned char* __restrict__ src, const int* __restrict__ idx,
-                      unsigned char* __restrict__ dst, unsigned bound, long long n, int width) {
+                      unsigned char* __restrict__ dst, unsigned bound, long long n, int width, bool sampled) {
     __shared__ int s_id[kWarps][kRows];
     const int lane = int(threadIdx.x & 31u), warp = int(threadIdx.x >> 5);
+    if (sampled && IndexSample(idx, n, lane).rows_adjoin(width)) return;
     const unsigned char* hi = src + n * (long long)width;
     const int slots = (width + 6) / 4;
     const int step_j = 32 / slots, step_k = 32 % slots;
@@ -239,7 +242,7 @@ unsigned clamp_bound(long long n) { return n > 0x80000000ll ? 0x80000000u : unsi
 
 template <int ROWS>
 static void launch(bool gather, const void* src, const int* idx, void* dst, long long bound, long long n, int width,
-                   int grid, cudaStream_t st) {
+                   int grid, bool sampled, cudaStream_t st) {
     const unsigned char* s = static_cast<const unsigned char*>(src);
     unsigned char* d = static_cast<unsigned char*>(dst);
     if (grid <= 0) {
@@ -249,7 +252,7 @@ static void launch(bool gather, const void* src, const int* idx, void* dst, long
     if (gather)
         gather_packed_kernel<ROWS><<<grid, 32 * kWarps, 0, st>>>(s, clamp_bound(bound), idx, d, n, width);
     else
-        scatter_packed_kernel<ROWS><<<grid, 32 * kWarps, 0, st>>>(s, idx, d, clamp_bound(bound), n, width);
+        scatter_packed_kernel<ROWS><<<grid, 32 * kWarps, 0, st>>>(s, idx, d, clamp_bound(bound), n, width, sampled);
 }
 
 // Rows to a warp, 8 to 128.  More rows to a warp waste less on its start and its
@@ -278,13 +281,13 @@ static int rows_to_a_warp(int width, long long n) {
 }
 
 void launch_index_packed(bool gather, const void* src, const int* idx, void* dst, long long bound, long long n,
-                         int width, int grid, cudaStream_t st) {
+                         int width, int grid, bool sampled, cudaStream_t st) {
     switch (rows_to_a_warp(width, n)) {
-        case 8: return launch<8>(gather, src, idx, dst, bound, n, width, grid, st);
-        case 16: return launch<16>(gather, src, idx, dst, bound, n, width, grid, st);
-        case 32: return launch<32>(gather, src, idx, dst, bound, n, width, grid, st);
-        case 64: return launch<64>(gather, src, idx, dst, bound, n, width, grid, st);
-        default: return launch<128>(gather, src, idx, dst, bound, n, width, grid, st);
+        case 8: return launch<8>(gather, src, idx, dst, bound, n, width, grid, sampled, st);
+        case 16: return launch<16>(gather, src, idx, dst, bound, n, width, grid, sampled, st);
+        case 32: return launch<32>(gather, src, idx, dst, bound, n, width, grid, sampled, st);
+        case 64: return launch<64>(gather, src, idx, dst, bound, n, width, grid, sampled, st);
+        default: return launch<128>(gather, src, idx, dst, bound, n, width, grid, sampled, st);
     }
 }
 

@@ -41,16 +41,21 @@ namespace trv {
 //    2^21 121 / 104; 2^20 of 120 bytes 77 / 87, 2^21 180 / 149; 400 MiB of 132 bytes
 //    337 / 276, of 200 bytes 241 / 225 and, where half of them lie in order, 185 /
 //    225: wider than 136 bytes they stay plain.  The fetch alone they never take
-//    (`wide`: the row kernels' rows above 64 bytes, not packed ones).
+//    (kWideRows);
+//  - packed rows (packed.cu), whose plain pass is slower, gain from the fetch from 22
+//    MiB on (2^22 rows of 10 bytes 95 us, 107 without).
+enum RowKind { kStructRows, kWideRows, kPackedRows };
+constexpr uint64_t kPlainPackedBytes = uint64_t(22) << 20;
 constexpr uint64_t kPlainScatterBytes = uint64_t(40) << 20;
 constexpr uint64_t kOnePassBytes = uint64_t(64) << 20;
 constexpr uint64_t kPartBytes = uint64_t(56) << 20;
 constexpr uint64_t kMostParts = 24;
 constexpr uint32_t kWidestInParts = 136;
 
-inline int scatter_parts(uint32_t width, uint64_t n, uint64_t dst_n, bool sectors, bool wide) {
+inline int scatter_parts(uint32_t width, uint64_t n, uint64_t dst_n, bool sectors, RowKind kind) {
+    const bool wide = kind == kWideRows;
     const uint64_t bytes = dst_n * width;
-    if (n < 2 || bytes <= kPlainScatterBytes || 2 * n < dst_n) return 0;
+    if (n < 2 || bytes <= (kind == kPackedRows ? kPlainPackedBytes : kPlainScatterBytes) || 2 * n < dst_n) return 0;
     if (width % 32 == 0 && sectors) return 0;
     if (wide && (width > kWidestInParts || n < (uint64_t(1) << 21))) return 0;
     const uint64_t parts = bytes <= kOnePassBytes ? 1 : (bytes + kPartBytes - 1) / kPartBytes;
@@ -78,6 +83,32 @@ TRV_HOST_DEVICE inline int near_pairs(int row_bytes) { return row_bytes > 64 ? 1
 TRV_HOST_DEVICE inline bool sample_near(int a, int b, int row_bytes) {
     const long long d = (long long)b - a;
     return (d < 0 ? -d : d) * row_bytes <= kNearBytes;
+}
+
+// Rows of any width and alignment move in 4-byte words (packed.cu) where that
+// beats a thread per row moving bytes (flat.cu).  A word takes its bytes from at
+// most two rows, and words read past a row from at most two more: rows have at least
+// kLeastPackedWidth bytes, whatever pays.
+//
+// What pays, bytes / words in us.  Random rows: gathers of 29 bytes 6.5 / 2.8 for
+// 2^12, of 13 bytes 4.8 / 3.9 for 2^16, of 6 bytes 5.1 / 5.6 for 2^18 and 16.4 / 9.5
+// for 2^20; scatters of 13 bytes 4.9 / 2.4 for 2^12, of 6 / 8 / 10 bytes 5.9 / 4.3,
+// 7.0 / 3.6 and 8.1 / 4.3 for 2^16, 50 / 24, 68 / 12 and 84 / 24 for 2^20.  In order:
+// of 13 bytes 29.7 / 18.9 and 29.9 / 20.5 for 2^20, but the bytes of narrow rows meet
+// in the same sectors by themselves: gathers of 6 bytes 8.0 / 8.5 for 2^20, scatters
+// of 6 / 8 / 10 bytes 2.5 / 3.3, 2.2 / 3.4 and 2.8 / 3.8 for 2^16, 24 / 41, 29 / 44
+// and 51 / 56 for 2^22.  Long scatters of up to 8 bytes so go by words only where a
+// sample of the indices does not find them in order: both kernels are launched and
+// one leaves, which takes 2 to 3 us, more than shorter ones lose.
+enum PackedForm { kByBytes, kByWords, kBySample };
+constexpr uint32_t kLeastPackedWidth = 4, kMostPackedWidth = 1u << 20;
+inline PackedForm packed_form(bool gather, uint32_t width, uint64_t n) {
+    if (width < kLeastPackedWidth || width > kMostPackedWidth) return kByBytes;  // words would come out wrong
+    if (width < 6) return kByBytes;                                              // most words straddle rows
+    if (width >= 13) return kByWords;
+    if (gather) return n >= (1u << 19) ? kByWords : kByBytes;
+    if (n < (1u << 16)) return kByBytes;
+    return width <= 8 && n >= (1u << 20) ? kBySample : kByWords;
 }
 
 // Rows that a warp of the parts kernel takes at a time: its offsets inside such a
