@@ -20,6 +20,9 @@ int parts(unsigned width, unsigned long long n, unsigned long long dst_n, int se
                               width % 4 ? trv::kPackedRows : width > 64 ? trv::kWideRows : trv::kStructRows);
 }
 int packed(int gather, unsigned width, unsigned long long n) { return trv::packed_form(gather, width, n); }
+int rows_unroll(int gather, unsigned width, unsigned long long n) { return trv::rows_unroll(gather, width, n); }
+int struct_unroll(int gather, unsigned width, unsigned long long n) { return trv::struct_unroll(gather, width, n); }
+int default_unroll(unsigned width) { return trv::default_unroll(width); }
 unsigned least_packed() { return trv::kLeastPackedWidth; }
 // whether the sample of idx says that the rows lie in order
 int local(const int* idx, long long n, int row_bytes) {
@@ -44,7 +47,8 @@ def rules(tmp_path_factory):
     lib = ctypes.CDLL(str(d / "rules.so"))
     lib.most_pass_words.restype = ctypes.c_uint32
     lib.parts.argtypes = [ctypes.c_uint32, ctypes.c_uint64, ctypes.c_uint64, ctypes.c_int]
-    lib.packed.argtypes = [ctypes.c_int, ctypes.c_uint32, ctypes.c_uint64]
+    for f in (lib.packed, lib.rows_unroll, lib.struct_unroll):
+        f.argtypes = [ctypes.c_int, ctypes.c_uint32, ctypes.c_uint64]
     lib.local.argtypes = [ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int]
     return lib
 
@@ -110,3 +114,16 @@ def test_packed_words_only_where_they_are_right(rules):
     for width, n, scatter, gather in [(6, 1 << 12, 0, 0), (6, 1 << 18, 1, 0), (8, 1 << 20, 2, 1), (10, 1 << 20, 1, 1),
                                       (11, 1 << 16, 1, 0), (13, 16, 1, 1)]:
         assert (rules.packed(0, width, n), rules.packed(1, width, n)) == (scatter, gather), width
+
+
+def test_structs_per_lane_are_built(rules):
+    """Every choice is one of the unrolls built; a grid's structs per lane do not
+    depend on the length."""
+    for width in range(4, 65, 4):
+        assert rules.default_unroll(width) in (1, 2, 4, 8)
+        for n in (1, 1 << 16, (1 << 16) + 1, 1 << 22, 1 << 26):
+            for gather in (0, 1):
+                assert rules.rows_unroll(gather, width, n) in (1, 2, 4, 8)
+                assert rules.struct_unroll(gather, width, n) in (1, 2, 4, 8)
+    assert [rules.default_unroll(w) for w in (8, 16, 32, 36)] == [8, 4, 2, 1]
+    assert rules.struct_unroll(0, 8, 1 << 22) == 8 and rules.struct_unroll(1, 8, 1 << 22) == 4

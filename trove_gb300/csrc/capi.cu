@@ -133,16 +133,6 @@ int unroll_slot(int unroll) {
     return -1;
 }
 
-// Heuristic unroll when the caller gives none: about 16 words in flight per
-// lane (tuned by the autotuner when a cache entry exists).
-int default_unroll(unsigned width) {
-    const unsigned words = width / 4;
-    if (words <= 2) return 8;
-    if (words <= 4) return 4;
-    if (words <= 8) return 2;
-    return 1;
-}
-
 }  // namespace trv
 
 using namespace trv;
@@ -382,32 +372,6 @@ int32_t trv_copy_exit(void* dst, const void* src, uint64_t n, uint32_t width, ui
     return trv_copy_exit_ex(dst, src, n, width, modulus, &cfg, stream);
 }
 
-// Structs per lane of the row-form kernels when the caller gives none.  A call
-// of at most 2^16 structs does not fill the GPU (2048 warps at one struct per
-// lane): more structs per lane only lengthen each warp (4096 structs of 28
-// bytes: 1.79 us at 1, 1.93 at 2, 2.43 at 4).  Above, one or two 4- or 8-byte
-// words in flight per lane are too few (2^24 structs of 4 bytes: gather 99 us
-// at 1, 80 at 2, 79 at 4; 2^20 of 8 bytes: 8.7 / 8.1 / 8.0 us; 2^20 of 12 to
-// 24 bytes: 2-6 % faster at 2 than at 1), while from 28 bytes up one struct
-// per lane is as fast or faster (2^20 of 36 bytes: 16.1 us at 1, 17.0 at 2).
-// Scatters gain from 2 up to 8 bytes only (2^20 of 8 bytes: 8.8 / 7.8 us; of
-// 24 bytes: 23.3 / 23.8).
-static int rows_unroll(bool gather, uint32_t width, uint64_t n) {
-    if (n <= (uint64_t(1) << 16)) return 1;
-    if (gather) return width <= 8 ? 4 : width <= 24 ? 2 : 1;
-    return width <= 8 ? 2 : 1;
-}
-
-// The same for the struct kernels (coalesced_ptr and compiler-generated access),
-// whose loads and stores go through a struct to a lane: 2^23 structs of 4 bytes
-// 48.7 us at 1, 42.3 at 2, 41.1 at 4, 40.7 at 8; contiguous indices of 16 bytes
-// 53.1 / 48.2 / 45.1 at 1 / 2 / 4; of 12 bytes 58.1 / 49.9 / 48.3, but random
-// ones 86.9 / 86.3 / 90.2; from 28 bytes up 1 is as fast or faster.
-static int struct_unroll(uint32_t width, uint64_t n) {
-    if (n <= (uint64_t(1) << 16)) return 1;
-    return width == 4 ? 8 : width == 8 || width == 16 ? 4 : width <= 24 ? 2 : 1;
-}
-
 // L2 fetch hint of a gather's random loads.  A source larger than L2 is
 // fetched by 64-byte halves (policy 4): the rest of a 128-byte line would leave
 // L2 before another row of it is asked for.  A source that fits (112 MiB of 126)
@@ -503,8 +467,10 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
     if (!struct_width(width)) return TRV_ERR_UNSUPPORTED;
     if (!aligned(dst, 4) || !aligned(src, 4)) return TRV_ERR_MISALIGNED;
     const int u = c.unroll > 0                ? c.unroll
+                  : path == TRV_PATH_DIRECT || (path == TRV_PATH_WARP && grid_req != 0)
+                      ? default_unroll(width)
                   : path == TRV_PATH_WARP ? rows_unroll(gather, width, n)
-                                          : struct_unroll(width, n);
+                                          : struct_unroll(gather, width, n);
     const int slot = unroll_slot(u);
     if (slot < 0) return TRV_ERR_INVALID_ARGUMENT;
     const WidthOps* ops = ops_for_words(int(width / 4));

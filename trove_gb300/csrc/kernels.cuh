@@ -189,11 +189,88 @@ __global__ void __launch_bounds__(256, EXIT && !LOOP ? exit_blocks(S * U, U) : 1
 // issued before its stores.
 enum { MODE_COALESCED = 0, MODE_DIRECT = 1 };
 
-// LOOP as for copy_kernel: false, one chunk per warp (the default grid), without
-// the loop's registers: 34 instead of 48 at 36 bytes, 40 instead of 60 at 64, so
-// up to 56 warps an SM instead of 40.  2^23 structs in runs of 32, 36 bytes 145.5
-// -> 133.0 us, 64 bytes 199.3 -> 171.9.
 template <int S, int U, int MODE>
+__global__ void __launch_bounds__(256)
+gather_kernel(const aos<S>* __restrict__ src, long long src_n, const int* __restrict__ idx,
+              aos<S>* __restrict__ dst, long long n) {
+    const WarpGrid g;
+    constexpr int CH = 32 * U;
+    trove::coalesced_ptr<aos<S> > S_(const_cast<aos<S>*>(src));
+    trove::coalesced_ptr<aos<S> > D_(dst);
+    for (long long base = g.warp * CH; base < n; base += g.warps * CH) {
+        int id[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const long long i = base + u * 32 + g.lane;
+            id[u] = i < n ? __ldg(idx + i) : -1;
+        }
+        aos<S> v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (id[u] >= 0 && (long long)id[u] < src_n) {
+                if constexpr (MODE == MODE_COALESCED)
+                    v[u] = S_[id[u]];
+                else
+                    v[u] = src[id[u]];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const long long i = base + u * 32 + g.lane;
+            if (id[u] >= 0 && (long long)id[u] < src_n) {
+                if constexpr (MODE == MODE_COALESCED)
+                    D_[i] = v[u];
+                else
+                    dst[i] = v[u];
+            }
+        }
+    }
+}
+
+template <int S, int U, int MODE>
+__global__ void __launch_bounds__(256)
+scatter_kernel(const aos<S>* __restrict__ src, const int* __restrict__ idx, aos<S>* __restrict__ dst,
+               long long dst_n, long long n) {
+    const WarpGrid g;
+    constexpr int CH = 32 * U;
+    trove::coalesced_ptr<aos<S> > S_(const_cast<aos<S>*>(src));
+    trove::coalesced_ptr<aos<S> > D_(dst);
+    for (long long base = g.warp * CH; base < n; base += g.warps * CH) {
+        int id[U];
+        aos<S> v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const long long i = base + u * 32 + g.lane;
+            id[u] = i < n ? __ldg(idx + i) : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const long long i = base + u * 32 + g.lane;
+            if (i < n) {
+                if constexpr (MODE == MODE_COALESCED)
+                    v[u] = S_[i];
+                else
+                    v[u] = src[i];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (id[u] >= 0 && (long long)id[u] < dst_n) {
+                if constexpr (MODE == MODE_COALESCED)
+                    D_[id[u]] = v[u];
+                else
+                    dst[id[u]] = v[u];
+            }
+        }
+    }
+}
+
+// The default grid of coalesced_ptr: one chunk per warp, without the loop's
+// registers: 34 instead of 48 at 36 bytes, 40 instead of 60 at 64, so up to 56 warps
+// an SM instead of 40.  2^23 structs in runs of 32, 36 bytes 145.5 -> 133.0 us, 64
+// bytes 199.3 -> 171.9.  Compiler-generated access has the loop always: without it
+// 2^23 sorted structs of 24 bytes took 94 us at 4 to a lane instead of 80.
+template <int S, int U>
 __device__ __forceinline__ void gather_chunk(const aos<S>* __restrict__ src, long long src_n,
                                              const int* __restrict__ idx, aos<S>* __restrict__ dst, int rem, int lane) {
     trove::coalesced_ptr<aos<S> > S_(const_cast<aos<S>*>(src));
@@ -204,25 +281,15 @@ __device__ __forceinline__ void gather_chunk(const aos<S>* __restrict__ src, lon
     aos<S> v[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-        if (id[u] >= 0 && (long long)id[u] < src_n) {
-            if constexpr (MODE == MODE_COALESCED)
-                v[u] = S_[id[u]];
-            else
-                v[u] = src[id[u]];
-        }
+        if (id[u] >= 0 && (long long)id[u] < src_n) v[u] = S_[id[u]];
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-        if (id[u] >= 0 && (long long)id[u] < src_n) {
-            if constexpr (MODE == MODE_COALESCED)
-                D_[u * 32 + lane] = v[u];
-            else
-                dst[u * 32 + lane] = v[u];
-        }
+        if (id[u] >= 0 && (long long)id[u] < src_n) D_[u * 32 + lane] = v[u];
     }
 }
 
-template <int S, int U, int MODE>
+template <int S, int U>
 __device__ __forceinline__ void scatter_chunk(const aos<S>* __restrict__ src, const int* __restrict__ idx,
                                               aos<S>* __restrict__ dst, long long dst_n, int rem, int lane) {
     trove::coalesced_ptr<aos<S> > S_(const_cast<aos<S>*>(src));
@@ -233,48 +300,36 @@ __device__ __forceinline__ void scatter_chunk(const aos<S>* __restrict__ src, co
     for (int u = 0; u < U; ++u) id[u] = u * 32 + lane < rem ? __ldg(idx + u * 32 + lane) : -1;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-        if (u * 32 + lane < rem) {
-            if constexpr (MODE == MODE_COALESCED)
-                v[u] = S_[u * 32 + lane];
-            else
-                v[u] = src[u * 32 + lane];
-        }
+        if (u * 32 + lane < rem) v[u] = S_[u * 32 + lane];
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-        if (id[u] >= 0 && (long long)id[u] < dst_n) {
-            if constexpr (MODE == MODE_COALESCED)
-                D_[id[u]] = v[u];
-            else
-                dst[id[u]] = v[u];
-        }
+        if (id[u] >= 0 && (long long)id[u] < dst_n) D_[id[u]] = v[u];
     }
 }
 
-template <int S, int U, int MODE, bool LOOP>
+template <int S, int U>
 __global__ void __launch_bounds__(256)
-gather_kernel(const aos<S>* __restrict__ src, long long src_n, const int* __restrict__ idx,
-              aos<S>* __restrict__ dst, long long n) {
+gather_once_kernel(const aos<S>* __restrict__ src, long long src_n, const int* __restrict__ idx,
+                   aos<S>* __restrict__ dst, long long n) {
     const WarpGrid g;
     constexpr int CH = 32 * U;
-    for (long long base = g.warp * CH; base < n; base += g.warps * CH) {
-        const int rem = n - base < CH ? int(n - base) : CH;
-        gather_chunk<S, U, MODE>(src, src_n, idx + base, dst + base, rem, g.lane);
-        if (!LOOP) break;
-    }
+    const long long base = g.warp * CH;
+    if (base >= n) return;
+    const int rem = n - base < CH ? int(n - base) : CH;
+    gather_chunk<S, U>(src, src_n, idx + base, dst + base, rem, g.lane);
 }
 
-template <int S, int U, int MODE, bool LOOP>
+template <int S, int U>
 __global__ void __launch_bounds__(256)
-scatter_kernel(const aos<S>* __restrict__ src, const int* __restrict__ idx, aos<S>* __restrict__ dst,
-               long long dst_n, long long n) {
+scatter_once_kernel(const aos<S>* __restrict__ src, const int* __restrict__ idx, aos<S>* __restrict__ dst,
+                    long long dst_n, long long n) {
     const WarpGrid g;
     constexpr int CH = 32 * U;
-    for (long long base = g.warp * CH; base < n; base += g.warps * CH) {
-        const int rem = n - base < CH ? int(n - base) : CH;
-        scatter_chunk<S, U, MODE>(src + base, idx + base, dst, dst_n, rem, g.lane);
-        if (!LOOP) break;
-    }
+    const long long base = g.warp * CH;
+    if (base >= n) return;
+    const int rem = n - base < CH ? int(n - base) : CH;
+    scatter_chunk<S, U>(src + base, idx + base, dst, dst_n, rem, g.lane);
 }
 
 // ---- cache policies of the row-form kernels ----------------------------

@@ -13,6 +13,51 @@
 
 namespace trv {
 
+// ---- structs per lane --------------------------------------------------------
+
+// Heuristic unroll when the caller gives none: about 16 words in flight per
+// lane (tuned by the autotuner when a cache entry exists).
+inline int default_unroll(uint32_t width) {
+    const uint32_t words = width / 4;
+    if (words <= 2) return 8;
+    if (words <= 4) return 4;
+    if (words <= 8) return 2;
+    return 1;
+}
+
+// Structs per lane of the row-form kernels when the caller gives neither them nor a
+// grid (a grid's few warps want more in flight, default_unroll: 2^22 rows of 12 bytes
+// scattered by 152 blocks 113 us at 4, 146 at 1).  A call
+// of at most 2^16 structs does not fill the GPU (2048 warps at one struct per
+// lane): more structs per lane only lengthen each warp (4096 structs of 28
+// bytes: 1.79 us at 1, 1.93 at 2, 2.43 at 4).  Above, one or two 4- or 8-byte
+// words in flight per lane are too few (2^24 structs of 4 bytes: gather 99 us
+// at 1, 80 at 2, 79 at 4; 2^20 of 8 bytes: 8.7 / 8.1 / 8.0 us; 2^20 of 12 to
+// 24 bytes: 2-6 % faster at 2 than at 1), while from 28 bytes up one struct
+// per lane is as fast or faster (2^20 of 36 bytes: 16.1 us at 1, 17.0 at 2).
+// Scatters gain from 2 up to 8 bytes only (2^20 of 8 bytes: 8.8 / 7.8 us; of
+// 24 bytes: 23.3 / 23.8).
+inline int rows_unroll(bool gather, uint32_t width, uint64_t n) {
+    if (n <= (uint64_t(1) << 16)) return 1;
+    if (gather) return width <= 8 ? 4 : width <= 24 ? 2 : 1;
+    return width <= 8 ? 2 : 1;
+}
+
+// The same for coalesced_ptr access, whose loads and stores go through a struct to a
+// lane: 2^23 structs of 4 bytes 48.7 us at 1, 42.3 at 2, 41.1 at 4, 40.7 at 8;
+// contiguous indices of 16 bytes 53.1 / 48.2 / 45.1 at 1 / 2 / 4; of 12 bytes 58.1 /
+// 49.9 / 48.3, but random ones 86.9 / 86.3 / 90.2.  Scatters of 8 bytes in order gain
+// up to 8 (2^24: 51.1 at 4, 49.1 at 8); from 28 bytes up 1 is as fast or faster, but
+// for gathers of many 32-byte structs in runs (2^24: 196 us at 1, 190 at 2).
+// Compiler-generated access (DIRECT) stays with default_unroll: 2^24 sorted structs
+// of 28 bytes scattered in 298 us at 2, 344 at 1.
+inline int struct_unroll(bool gather, uint32_t width, uint64_t n) {
+    if (n <= (uint64_t(1) << 16)) return 1;
+    if (width <= 8) return width == 4 || !gather ? 8 : 4;
+    if (width == 32) return gather && n >= (uint64_t(1) << 22) ? 2 : 1;
+    return width == 16 ? 4 : width <= 24 ? 2 : 1;
+}
+
 // ---- scatters in parts (scatter_parts.cu) ----------------------------------
 
 // In how many parts a scatter writes its destination: 0, as one plain pass; 1,

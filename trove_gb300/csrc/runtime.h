@@ -39,7 +39,6 @@ int grid_for(const void* func, long long work_items, int items_per_block, int bl
 bool one_chunk_per_warp(long long n, int unroll, int requested, int* grid);
 
 int unroll_slot(int unroll);
-int default_unroll(unsigned width);
 
 // Runs an entry point's body so that no C++ exception crosses the C ABI.  The
 // only exceptions the host code can meet are failed allocations of its host

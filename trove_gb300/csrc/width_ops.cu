@@ -20,13 +20,17 @@ void launch_copy(const CopyArgs& a, int grid, int block, cudaStream_t st) {
 
 template <int U, int MODE>
 void launch_gather(const IndexArgs& a, int grid, int block, cudaStream_t st) {
-    auto* k = a.once ? &gather_kernel<S, U, MODE, false> : &gather_kernel<S, U, MODE, true>;
+    auto* k = &gather_kernel<S, U, MODE>;
+    if constexpr (MODE == MODE_COALESCED)
+        if (a.once) k = &gather_once_kernel<S, U>;
     k<<<grid, block, 0, st>>>(static_cast<const aos<S>*>(a.src), a.bound, a.idx, static_cast<aos<S>*>(a.dst), a.n);
 }
 
 template <int U, int MODE>
 void launch_scatter(const IndexArgs& a, int grid, int block, cudaStream_t st) {
-    auto* k = a.once ? &scatter_kernel<S, U, MODE, false> : &scatter_kernel<S, U, MODE, true>;
+    auto* k = &scatter_kernel<S, U, MODE>;
+    if constexpr (MODE == MODE_COALESCED)
+        if (a.once) k = &scatter_once_kernel<S, U>;
     k<<<grid, block, 0, st>>>(static_cast<const aos<S>*>(a.src), a.idx, static_cast<aos<S>*>(a.dst), a.bound, a.n);
 }
 
@@ -148,13 +152,13 @@ void fill_copy(CopyKernel (&row)[kUnrolls]) {
 template <int MODE, int k>
 IndexKernel gather_entry() {
     constexpr int U = unroll_for(k);
-    return {&launch_gather<U, MODE>, (const void*)&gather_kernel<S, U, MODE, true>};
+    return {&launch_gather<U, MODE>, (const void*)&gather_kernel<S, U, MODE>};
 }
 
 template <int MODE, int k>
 IndexKernel scatter_entry() {
     constexpr int U = unroll_for(k);
-    return {&launch_scatter<U, MODE>, (const void*)&scatter_kernel<S, U, MODE, true>};
+    return {&launch_scatter<U, MODE>, (const void*)&scatter_kernel<S, U, MODE>};
 }
 
 template <int MODE>
