@@ -23,6 +23,7 @@ int packed(int gather, unsigned width, unsigned long long n) { return trv::packe
 int rows_unroll(int gather, unsigned width, unsigned long long n) { return trv::rows_unroll(gather, width, n); }
 int struct_unroll(int gather, unsigned width, unsigned long long n) { return trv::struct_unroll(gather, width, n); }
 int default_unroll(unsigned width) { return trv::default_unroll(width); }
+int exit_unroll(unsigned width, unsigned long long bytes) { return trv::exit_unroll(width, bytes); }
 unsigned least_packed() { return trv::kLeastPackedWidth; }
 // whether the sample of idx says that the rows lie in order
 int local(const int* idx, long long n, int row_bytes) {
@@ -47,6 +48,7 @@ def rules(tmp_path_factory):
     lib = ctypes.CDLL(str(d / "rules.so"))
     lib.most_pass_words.restype = ctypes.c_uint32
     lib.parts.argtypes = [ctypes.c_uint32, ctypes.c_uint64, ctypes.c_uint64, ctypes.c_int]
+    lib.exit_unroll.argtypes = [ctypes.c_uint32, ctypes.c_uint64]
     for f in (lib.packed, lib.rows_unroll, lib.struct_unroll):
         f.argtypes = [ctypes.c_int, ctypes.c_uint32, ctypes.c_uint64]
     lib.local.argtypes = [ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int]
@@ -125,5 +127,7 @@ def test_structs_per_lane_are_built(rules):
             for gather in (0, 1):
                 assert rules.rows_unroll(gather, width, n) in (1, 2, 4, 8)
                 assert rules.struct_unroll(gather, width, n) in (1, 2, 4, 8)
+            assert rules.exit_unroll(width, n * width) in (1, 2, 4, 8)
     assert [rules.default_unroll(w) for w in (8, 16, 32, 36)] == [8, 4, 2, 1]
+    assert [rules.exit_unroll(16, mib << 20) for mib in (1, 16, 1024)] == [1, 4, 2]
     assert rules.struct_unroll(0, 8, 1 << 22) == 8 and rules.struct_unroll(1, 8, 1 << 22) == 4

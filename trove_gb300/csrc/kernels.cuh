@@ -33,16 +33,17 @@ enum Api { API_WARP = 0, API_BLOCK = 1, API_DIRECT = 2 };
 // divides w - (d - 1); and d = q * 2^k (q odd) divides x when x times q's inverse
 // modulo 2^32, rotated right by k, is at most (2^32 - 1) / d (Granlund and
 // Montgomery, "Division by Invariant Integers using Multiplication", section 9).
-// Five instructions where the remainder of a run-time d took about twenty of
-// the 84 that 32 structs of 12 bytes cost: 1 GiB of 4 bytes 311 -> 305 us, of 12
-// bytes 321 -> 309, of 20 bytes 316 -> 307, of 24 bytes 301 -> 298.  Structs of an
-// odd number of words from 36 bytes up are bound by DRAM either way and keep the
-// remainder (36 bytes 301.2 us, 302.0 by multiplication; 44 bytes 300.7 and 301.6;
-// 60 bytes 300.9 and 301.4), even ones gain from 32 bytes on (305.0 -> 303.1).
-template <int S>
+// Five instructions where the remainder of a run-time d takes about twenty, of the
+// 84 that 32 structs of 12 bytes cost: 1 GiB of 4 bytes 308.5 -> 305.2 us, of 12 bytes
+// 318.7 -> 306.4, of 20 bytes 313 -> 306.5, of 32 bytes 303.7 -> 301.8.  It pays for
+// lanes of few words, which are bound by instructions (exit_multiply).  Lanes of more
+// words wait for DRAM either way, and the multiplication's operands cost them
+// registers (12 bytes, 8 structs to a lane, 42 and 48: 314 -> 325 us; 28 bytes, 2 to a
+// lane, 32 and 40: 301 -> 308; 36 bytes 299.6 -> 300.5): they keep the remainder.
+template <bool MULTIPLY, int S>
 __device__ __forceinline__ bool exits(const aos<S>& v, const ExitTest& t) {
     const unsigned w = unsigned(v.head);
-    if (S >= 9 && S % 2 == 1) return w % (t.low + 1u) == t.low;
+    if constexpr (!MULTIPLY) return w % t.modulus == t.modulus - 1u;
     const unsigned x = (w - t.low) * t.inverse;
     return w >= t.low && __funnelshift_r(x, x, t.rotate) <= t.most;
 }
@@ -133,15 +134,20 @@ struct WarpGrid {
 // to 32+ registers and below full occupancy (2048 threads per SM), which is
 // where a one-chunk kernel gets its loads in flight.  LOOP = true serves
 // caller-chosen and persistent grids.
-// Resident blocks that the early-exit copy is built for, by the words of a lane:
-// up to 12 words fit 32 registers and 24 words 40 without spills, but ptxas takes
-// 38-48 where it may (1 GiB of 12 bytes, 4 structs to a lane, 326 us at 40
-// registers and 309 at 32; 24 bytes, 2 to a lane, 319 and 302).  One struct of 11
-// words and more to a lane is left alone: its 48 warps fill the memory system
-// (44 bytes 301.8 us, 303.6 at 64 warps).
-constexpr int exit_blocks(int words, int unroll) { return words <= (unroll > 1 ? 12 : 10) ? 8 : unroll > 1 && words <= 24 ? 6 : 1; }
+//
+// Resident blocks that the early-exit copy is built for, by the words of a lane: up
+// to 16 words fit 32 registers (of 12 bytes, 4 to a lane, with 8 bytes spilled), but
+// ptxas takes 34-48 where it may (1 GiB of 12 bytes, 4 structs to a lane, 326 us at 40
+// registers and 306 at 32; 24 bytes, 2 to a lane, 319 and 302).  One struct of more
+// than 8 words to a lane is left alone: fewer warps fill the memory system (44 bytes
+// 301.8 us, 303.6 at 64 warps).  0: as ptxas likes, which a bound of 1 is not (64
+// bytes 32 registers, 38 with it: 16 MiB 5.5 us and 6.1).
+template <int S, int U>
+constexpr int exit_blocks = S * U <= (U > 1 ? 16 : 8) ? 8 : 0;
+template <int S, int U>
+constexpr bool exit_multiply = S * U <= (U > 1 ? 12 : 8);
 
-template <int S, int U, int API, bool EXIT>
+template <int S, int U, int API, bool EXIT, bool MULTIPLY>
 __device__ __forceinline__ void copy_chunk(const aos<S>* __restrict__ src, aos<S>* __restrict__ dst, long long n,
                                            const ExitTest& test, long long base, int lane) {
     constexpr int CH = 32 * U;
@@ -151,7 +157,7 @@ __device__ __forceinline__ void copy_chunk(const aos<S>* __restrict__ src, aos<S
         for (int u = 0; u < U; ++u) v[u] = load_conv<S, API>(src, base + u * 32 + lane);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            if (!EXIT || !exits(v[u], test)) {
+            if (!EXIT || !exits<MULTIPLY>(v[u], test)) {
                 if constexpr (EXIT)
                     store_any<S, API>(dst, base + u * 32 + lane, v[u]);
                 else
@@ -164,23 +170,23 @@ __device__ __forceinline__ void copy_chunk(const aos<S>* __restrict__ src, aos<S
             const long long i = base + u * 32 + lane;
             if (i < n) {
                 const aos<S> v = src[i];
-                if (!EXIT || !exits(v, test)) dst[i] = v;
+                if (!EXIT || !exits<MULTIPLY>(v, test)) dst[i] = v;
             }
         }
     }
 }
 
 template <int S, int U, int API, bool EXIT, bool LOOP>
-__global__ void __launch_bounds__(256, EXIT && !LOOP ? exit_blocks(S * U, U) : 1) copy_kernel(const aos<S>* __restrict__ src, aos<S>* __restrict__ dst,
-                                                   long long n, ExitTest test) {
+__global__ void __launch_bounds__(256, EXIT && !LOOP ? exit_blocks<S, U> : 0)
+copy_kernel(const aos<S>* __restrict__ src, aos<S>* __restrict__ dst, long long n, ExitTest test) {
     const WarpGrid g;
     constexpr int CH = 32 * U;
     if constexpr (LOOP) {
         for (long long base = g.warp * CH; base < n; base += g.warps * CH)
-            copy_chunk<S, U, API, EXIT>(src, dst, n, test, base, g.lane);
+            copy_chunk<S, U, API, EXIT, false>(src, dst, n, test, base, g.lane);
     } else {
         const long long base = g.warp * CH;
-        if (base < n) copy_chunk<S, U, API, EXIT>(src, dst, n, test, base, g.lane);
+        if (base < n) copy_chunk<S, U, API, EXIT, exit_multiply<S, U>>(src, dst, n, test, base, g.lane);
     }
 }
 

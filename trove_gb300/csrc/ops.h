@@ -10,11 +10,12 @@ namespace trv {
 // Unroll factors offered (structs per lane per pass); index = log2(unroll).
 constexpr int kUnrolls = 4;  // 1, 2, 4, 8
 
-// The early-exit test w % d == d - 1 without a division (kernels.cuh, exits).
+// The early-exit test w % d == d - 1, and what it takes without a division
+// (kernels.cuh, exits).
 struct ExitTest {
-    unsigned low = 0, inverse = 1, rotate = 0, most = 0;
+    unsigned modulus = 1, low = 0, inverse = 1, rotate = 0, most = 0;
     ExitTest() = default;
-    explicit ExitTest(unsigned d) : low(d - 1), most(0xFFFFFFFFu / d) {  // d > 0
+    explicit ExitTest(unsigned d) : modulus(d), low(d - 1), most(0xFFFFFFFFu / d) {  // d > 0
         while (d % 2 == 0) {
             d /= 2;
             ++rotate;

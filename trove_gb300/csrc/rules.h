@@ -58,6 +58,21 @@ inline int struct_unroll(bool gather, uint32_t width, uint64_t n) {
     return width == 16 ? 4 : width <= 24 ? 2 : 1;
 }
 
+// Structs per lane of the early-exit copy when the caller gives none.  Up to 4
+// MiB the GPU is not full and more to a lane only lengthens each warp (1 MiB of
+// 12 bytes 1.74 us at 1, 1.94 at 2, 2.16 at 4).  Above, narrow structs need
+// several in flight (1 GiB of 4 bytes 770 / 446 / 326 / 305 us at 1 / 2 / 4 / 8;
+// of 8 bytes 442 / 324 / 304 / 306; of 12 bytes 380 / 351 / 309 / 322; of 16 bytes
+// 315 / 303 / 304, but 16 MiB 5.9 / 5.6 / 5.3) and from 24 bytes up one is as good as
+// two or better (24 bytes 298 / 302, 28 bytes 300 / 305).  20 bytes change over: 16
+// MiB 7.4 / 8.0, 128 MiB 41.8 / 41.5, 1 GiB 315 / 307.
+inline int exit_unroll(uint32_t width, uint64_t bytes) {
+    if (bytes <= (uint64_t(4) << 20)) return width == 4 ? 2 : 1;
+    if (width == 20) return bytes >= (uint64_t(128) << 20) ? 2 : 1;
+    if (width == 16) return bytes < (uint64_t(64) << 20) ? 4 : 2;
+    return width == 4 ? 8 : width <= 12 ? 4 : 1;
+}
+
 // ---- scatters in parts (scatter_parts.cu) ----------------------------------
 
 // In how many parts a scatter writes its destination: 0, as one plain pass; 1,
