@@ -24,6 +24,7 @@ int rows_unroll(int gather, unsigned width, unsigned long long n) { return trv::
 int struct_unroll(int gather, unsigned width, unsigned long long n) { return trv::struct_unroll(gather, width, n); }
 int default_unroll(unsigned width) { return trv::default_unroll(width); }
 int exit_unroll(unsigned width, unsigned long long bytes) { return trv::exit_unroll(width, bytes); }
+int layout_unroll(int to_soa, unsigned width, unsigned long long n) { return trv::layout_unroll(to_soa, width, n); }
 unsigned least_packed() { return trv::kLeastPackedWidth; }
 // whether the sample of idx says that the rows lie in order
 int local(const int* idx, long long n, int row_bytes) {
@@ -49,7 +50,7 @@ def rules(tmp_path_factory):
     lib.most_pass_words.restype = ctypes.c_uint32
     lib.parts.argtypes = [ctypes.c_uint32, ctypes.c_uint64, ctypes.c_uint64, ctypes.c_int]
     lib.exit_unroll.argtypes = [ctypes.c_uint32, ctypes.c_uint64]
-    for f in (lib.packed, lib.rows_unroll, lib.struct_unroll):
+    for f in (lib.packed, lib.rows_unroll, lib.struct_unroll, lib.layout_unroll):
         f.argtypes = [ctypes.c_int, ctypes.c_uint32, ctypes.c_uint64]
     lib.local.argtypes = [ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int]
     return lib
@@ -127,7 +128,11 @@ def test_structs_per_lane_are_built(rules):
             for gather in (0, 1):
                 assert rules.rows_unroll(gather, width, n) in (1, 2, 4, 8)
                 assert rules.struct_unroll(gather, width, n) in (1, 2, 4, 8)
+                assert rules.layout_unroll(gather, width, n) in (1, 2, 4, 8)
             assert rules.exit_unroll(width, n * width) in (1, 2, 4, 8)
     assert [rules.default_unroll(w) for w in (8, 16, 32, 36)] == [8, 4, 2, 1]
     assert [rules.exit_unroll(16, mib << 20) for mib in (1, 16, 1024)] == [1, 4, 2]
+    # fields' arrays aligned to sectors or not
+    assert [rules.layout_unroll(1, 64, (1 << 23) + k) for k in (0, 1, 4, 8)] == [1, 2, 2, 1]
+    assert [rules.layout_unroll(1, w, (1 << 25) + 1) for w in (32, 36, 40, 44, 48)] == [2, 1, 2, 1, 2]
     assert rules.struct_unroll(0, 8, 1 << 22) == 8 and rules.struct_unroll(1, 8, 1 << 22) == 4

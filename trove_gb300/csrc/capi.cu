@@ -517,21 +517,6 @@ int32_t trv_scatter(void* dst, uint64_t dst_n, const void* src, const int32_t* i
     return index_op(false, dst, src, dst_n, idx, n, width, nullptr, stream);
 }
 
-// The same for the layout conversions.  To SoA in us at 1 / 2 / 4 / 8: 512 MiB of
-// 4 bytes 366 / 214 / 159 / 153, of 8 bytes 215 / 161 / 154 / 153, of 12 bytes 183 /
-// 179 / 177 / 253 (32 MiB 13.9 / 13.9 / 14.6), of 28 bytes 158 / 162, of 64 bytes 185
-// / 170 (32 MiB 13.2 / 14.1).  From SoA: 512 MiB of 12 bytes 190 / 158 / 156, of 24
-// bytes 159 / 159 / 157, of 28 bytes 156 / 157, of 64 bytes 170 / 168.
-static int layout_unroll(bool to_soa, uint32_t width, uint64_t bytes) {
-    if (bytes <= (uint64_t(4) << 20)) return width == 4 ? 2 : 1;
-    if (width == 4) return 8;
-    if (to_soa) {
-        const bool large = bytes >= (uint64_t(256) << 20);
-        return width == 8 ? 4 : width <= 16 || (large && (width == 32 || width >= 40)) ? 2 : 1;
-    }
-    return width <= 12 ? 4 : width <= 24 ? 2 : 1;
-}
-
 static int32_t layout_op(bool to_soa, void* dst, const void* src, uint64_t n, uint32_t width, const trv_launch* cfg,
                          void* stream) {
     if (!size_ok(n, width)) return TRV_ERR_INVALID_ARGUMENT;
@@ -549,7 +534,7 @@ static int32_t layout_op(bool to_soa, void* dst, const void* src, uint64_t n, ui
             u = t.unroll;
             if (grid_req == 0) grid_req = t.grid;
         } else {
-            u = layout_unroll(to_soa, width, n * width);
+            u = layout_unroll(to_soa, width, n);
         }
     }
     const int slot = unroll_slot(u);

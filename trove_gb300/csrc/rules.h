@@ -73,6 +73,30 @@ inline int exit_unroll(uint32_t width, uint64_t bytes) {
     return width == 4 ? 8 : width <= 12 ? 4 : 1;
 }
 
+// The same for the layout conversions, in us at 1 / 2 / 4 / 8.  To SoA, 512 MiB of 4
+// bytes 366 / 214 / 159 / 153, of 8 bytes 216 / 161 / 154 / 154, of 12 bytes 183 / 179 /
+// 177 / 254 (32 MiB 13.9 / 13.9 / 14.6), 32 MiB of 16 bytes 11.7 / 10.7 / 10.3 / 10.7;
+// 1 GiB of 20 bytes 1 % faster at 2, shorter ones as fast or slower; 24 and 28 bytes
+// fastest at 1.  From 32 bytes on 1 too where the fields' arrays are aligned to
+// sectors (1 GiB of 32 / 36 / 44 / 48 / 64 bytes 307 / 304 / 324 / 322 / 311 at 1, 306
+// / 304 / 331 / 327 / 319 at 2).  Where they are not, a warp's 128 bytes of a field end
+// in a sector that the next warp's begin, and a warp of two such pieces saves one of
+// the two (352 / 320 / 344 / 364 / 398 at 1, 327 / 323 / 350 / 346 / 353 at 2; 40 / 52
+// / 56 / 60 bytes 325 / 335 / 345 / 350 and 317 / 331 / 323 / 336): from 64 MiB on, but
+// for 36 and 44 bytes, whose transpose holds more registers than it saves.  From SoA:
+// 512 MiB of 12 bytes 190 / 158 / 156, of 24 bytes 159 / 159 / 157, of 28 bytes 156 /
+// 157, but 16 MiB 5.1 / 4.7, of 32 bytes 5.1 / 4.6.
+inline int layout_unroll(bool to_soa, uint32_t width, uint64_t n) {
+    const uint64_t bytes = n * width, MiB = uint64_t(1) << 20;
+    if (bytes < 4 * MiB) return width == 4 ? 2 : 1;
+    if (width == 4) return 8;
+    if (!to_soa) return width <= 12 ? 4 : width <= 24 ? 2 : width <= 32 && bytes < 24 * MiB ? 2 : 1;
+    if (width == 8 || width == 16) return width == 8 ? 8 : 4;
+    if (width == 12) return bytes >= 256 * MiB ? 4 : 2;
+    if (width <= 28) return width == 20 && bytes >= 256 * MiB ? 2 : 1;
+    return n % 8 != 0 && bytes >= 64 * MiB && width != 36 && width != 44 ? 2 : 1;
+}
+
 // ---- scatters in parts (scatter_parts.cu) ----------------------------------
 
 // In how many parts a scatter writes its destination: 0, as one plain pass; 1,
