@@ -26,6 +26,17 @@ int default_unroll(unsigned width) { return trv::default_unroll(width); }
 int exit_unroll(unsigned width, unsigned long long bytes) { return trv::exit_unroll(width, bytes); }
 int layout_unroll(int to_soa, unsigned width, unsigned long long n) { return trv::layout_unroll(to_soa, width, n); }
 unsigned least_packed() { return trv::kLeastPackedWidth; }
+// tile bytes of each task (op, width, n); whether they make one wave
+int tiles(const long long* tasks, long long count, int blocks, int* bytes) {
+    const trv::TileRule rule([&](uint64_t k) {
+        return trv::TileTask{tasks[3 * k] == 0, uint32_t(tasks[3 * k + 1]), uint64_t(tasks[3 * k + 2])};
+    }, uint64_t(count), blocks);
+    for (long long k = 0; k < count; ++k) bytes[k] = rule.tile_bytes(int(tasks[3 * k]), uint32_t(tasks[3 * k + 1]));
+    return rule.one_wave();
+}
+int piece_rows(int blocks_per_sm, int wide, int row_bytes) {
+    return trv::piece_rows(trv::stage_bytes(blocks_per_sm), wide, row_bytes);
+}
 // whether the sample of idx says that the rows lie in order
 int local(const int* idx, long long n, int row_bytes) {
     int near = 0;
@@ -49,6 +60,7 @@ def rules(tmp_path_factory):
     lib = ctypes.CDLL(str(d / "rules.so"))
     lib.most_pass_words.restype = ctypes.c_uint32
     lib.parts.argtypes = [ctypes.c_uint32, ctypes.c_uint64, ctypes.c_uint64, ctypes.c_int]
+    lib.tiles.argtypes = [ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int, ctypes.c_void_p]
     lib.exit_unroll.argtypes = [ctypes.c_uint32, ctypes.c_uint64]
     for f in (lib.packed, lib.rows_unroll, lib.struct_unroll, lib.layout_unroll):
         f.argtypes = [ctypes.c_int, ctypes.c_uint32, ctypes.c_uint64]
@@ -136,3 +148,44 @@ def test_structs_per_lane_are_built(rules):
     assert [rules.layout_unroll(1, 64, (1 << 23) + k) for k in (0, 1, 4, 8)] == [1, 2, 2, 1]
     assert [rules.layout_unroll(1, w, (1 << 25) + 1) for w in (32, 36, 40, 44, 48)] == [2, 1, 2, 1, 2]
     assert rules.struct_unroll(0, 8, 1 << 22) == 8 and rules.struct_unroll(1, 8, 1 << 22) == 4
+
+
+def tiles_of(rules, tasks, blocks=608):
+    a = np.array(tasks, np.int64).reshape(-1, 3)
+    out = np.zeros(len(a), np.int32)
+    one = rules.tiles(a.ctypes.data, len(a), blocks, out.ctypes.data)
+    structs = np.maximum(out // a[:, 1] // 32 * 32, 32)
+    return bool(one), out, -(-a[:, 2] // structs)
+
+
+def test_tiles_of_a_batch(rules):
+    """A batch that can be one wave of tiles is one, whatever is left over of its
+    arrays; narrow rows get shorter tiles than wide ones; large batches get the largest
+    tiles, and nothing gets more than that."""
+    for op in (0, 1, 2):
+        for width in range(4, 65, 4):
+            for count, n in [(16, 1024), (16, 32768), (256, 512), (256, 2048), (100, 20000), (607, 999), (1, 1 << 18)]:
+                one, size, count_of = tiles_of(rules, [(op, width, n)] * count)
+                assert size.max() <= 65536 if one else (131072, 65536, 49152)[op]
+                if count * n * width <= 30 << 20:
+                    assert one and (count_of.sum() <= 608 or size[0] * (width + 48 * (op > 0)) <= 25000 * width)
+            one, size, _ = tiles_of(rules, [(op, width, 1 << 22)] * 40)
+            assert not one and size[0] == (131072, 65536, 49152)[op]
+    one, size, count_of = tiles_of(rules, [(1, 16, 8192)] * 256)  # 64 KiB and two to an array just fit
+    assert one and size[0] == 65536 and count_of.sum() == 512
+    _, size, _ = tiles_of(rules, [(1, 4, 30000), (1, 64, 30000)] * 20)
+    assert size[0] // 4 > size[1] // 64 and size[0] < size[1]
+    assert tiles_of(rules, [(1, 12, 0)] * 5)[0] and tiles_of(rules, [])[0]
+    assert tiles_of(rules, [(2, 64, 32)] * 50000)[2].max() == 1
+
+
+def test_staged_pieces_fit_their_memory(rules):
+    for blocks in (2, 4):
+        memory = 81408 if blocks == 2 else 40704
+        for width in range(4, 65, 4):
+            rows = rules.piece_rows(blocks, 0, width)
+            assert rows % 32 == 0 and rows >= 32 and 3 * rows * width + 4 * rows * 4 <= memory
+            if width % 16 == 0:
+                rows = rules.piece_rows(blocks, 1, width)
+                # the division of a word's number by words to a row holds for 12 bits
+                assert rows % 32 == 0 and rows >= 32 and 2 * rows * (width + 4) <= memory and rows * width // 16 <= 4096

@@ -21,6 +21,7 @@
 #include "batch.h"
 #include "fetch.cuh"
 #include "kernels.cuh"
+#include "rules.h"
 #include "runtime.h"
 #include "tma.cuh"
 #include "trove_gb300.h"
@@ -36,37 +37,31 @@ namespace {
 constexpr int kBulkChunk = 8 << 10;
 
 // Launch shapes of the persistent kernel: block size, resident blocks per SM
-// it is built for (hence the register budget), the staged gather / scatter
-// pieces with their index slots, and the copy ring's stages, which reuse the
-// pieces' memory.  128-thread blocks, 8 per SM, with 8 KiB pieces measured no
-// better than 256-thread ones (23.8 vs 22.9 ms for a 4096-array batch).
+// it is built for (hence the register budget), the staging memory of the gather and
+// scatter movers, and the copy ring's stages, which reuse that memory.  128-thread
+// blocks, 8 per SM, with 8 KiB pieces measured no better than 256-thread ones (23.8 vs
+// 22.9 ms for a 4096-array batch).
 //
-// The pieces' size is a balance of the two halves of an SM's 256 KiB.  Rows that
-// are copied by 4 or 8 bytes pass through L1, a 128-byte line for each row in
-// flight, so the more shared memory the blocks take, the fewer rows are in
-// flight; rows copied by 16 bytes go around L1 and are in flight in the pieces
-// alone.  2^24 rows of 12 / 20 / 64 bytes from sources of 2^19, us: 12 KiB pieces
-// with 1024 indices (212 KiB an SM, 28 KiB of L1) 264 / 328 / 348; these (163 and
-// 92) 150 / 180 / 333; 8 KiB with 416 (127 and 124) 147 / 176 / 369; 4 KiB with
-// 256 (100 and 156, but twice the barriers) 185 / 215 / 519.
-constexpr int kPieces = 3;      // staged pieces in shared memory (words of 4 and 8 bytes)
-constexpr int kIndexSlots = 4;  // index arrays of as many pieces
-
-template <int BLOCK, int MINB, int PIECE, int RING>
+// The memory is a balance of the two halves of an SM's 256 KiB.  Rows that are copied
+// by 4 or 8 bytes pass through L1, a 128-byte line for each row in flight, so the more
+// shared memory the blocks take, the fewer rows are in flight; rows copied by 16 bytes
+// go around L1 and are in flight in the pieces alone.  2^24 rows of 12 / 20 / 64 bytes
+// from sources of 2^19, us: with 212 KiB an SM (28 KiB of L1) 264 / 328 / 348; with
+// these 163 (and 92) 150 / 180 / 333; with 127 (and 124) 147 / 176 / 369; with 100 (and
+// 156, but twice the barriers) 185 / 215 / 519.  A tile divides it into pieces and
+// their indices by the width of its rows, so that neither lies idle: with the same
+// pieces and 480 indices for every width, 4-byte rows took 1.9 of a piece's 11 KB.
+template <int BLOCK, int MINB, int RING>
 struct Shape {
     static constexpr int block = BLOCK;
     static constexpr int warps = BLOCK / 32;
     static constexpr int minb = MINB;
-    static constexpr int piece = PIECE;     // bytes of one staged piece
-    static constexpr int idx_slots = 480;   // indices of one staged piece
-    static constexpr int wide_piece = kPieces * PIECE / 2;  // the same of the two pieces of 16-byte words
-    static constexpr int wide_slots = kIndexSlots * idx_slots / 2;
-    static constexpr int ring = RING;       // copy stages of kBulkChunk bytes
-    static constexpr int dyn_smem = kPieces * PIECE + kIndexSlots * idx_slots * int(sizeof(int));
-    static_assert(RING * kBulkChunk <= kPieces * PIECE, "the copy ring fits the piece buffers");
+    static constexpr int dyn_smem = stage_bytes(MINB);  // staging memory
+    static constexpr int ring = RING;                   // copy stages of kBulkChunk bytes
+    static_assert(RING * kBulkChunk <= dyn_smem, "the copy ring fits the staging memory");
 };
-using Shape2 = Shape<256, 2, 11008, 4>;  // 128 registers per thread
-using Shape4 = Shape<256, 4, 11008, 4>;  // 64 registers
+using Shape2 = Shape<256, 2, 4>;  // 128 registers per thread
+using Shape4 = Shape<256, 4, 4>;  // 64 registers
 
 // ---- per-tile movers (all warps of the CTA cooperate on one tile) --------
 
@@ -227,7 +222,7 @@ __device__ __forceinline__ void tile_index_rows(const V* src, V* dst, const int*
 // bytes (GB300s differ in their default, and the best size depends on the
 // struct width).
 //
-// Words of 4 and 8 bytes (tile_index_staged): three pieces of S::piece bytes
+// Words of 4 and 8 bytes (tile_index_staged): three pieces
 // rotate, two filling while one is written, with one barrier a piece.  A thread
 // copies word r of rows j, j + step, ...: r and its source column are fixed for
 // the whole tile, so a word costs its index from shared memory, an address and
@@ -296,20 +291,21 @@ __device__ __forceinline__ void cp_async_range(V* smem, const V* gmem, int bytes
 
 template <class S, typename V, bool GATHER, int PF>
 __device__ void tile_index_staged(const V* src, V* dst, const int* idx, long long bound64, long long first, int cnt,
-                                  int m, unsigned char* stage, int* s_idx, int* s_bad) {
+                                  int m, unsigned char* stage, int* s_bad) {
     const int tid = opaque_tid();
     const unsigned bound = bound64 > 0x80000000ll ? 0x80000000u : unsigned(bound64);
-    // structs per piece: a multiple of 32 that fits the buffer and the index slots
-    int per = (S::piece / int(sizeof(V))) / m / 32 * 32;
-    if (per > S::idx_slots) per = S::idx_slots;
+    const unsigned row_bytes = unsigned(m) * unsigned(sizeof(V));
+    // structs per piece: a multiple of 32, so many that the pieces and the index
+    // arrays fit the staging memory
+    const int per = piece_rows(S::dyn_smem, false, int(row_bytes));
+    int* s_idx = reinterpret_cast<int*>(stage + kPieces * per * int(row_bytes));
     const int pieces = (cnt + per - 1) / per;
     // this thread's word of a row, its first row, and the rows that the block's
     // threads cover together (the last few threads have no row where m does not
     // divide the block)
     const int step = S::block / m;
-    const int j0 = tid < step * m ? tid / m : S::idx_slots;
+    const int j0 = tid < step * m ? tid / m : S::dyn_smem;
     const int r = tid < step * m ? tid - tid / m * m : 0;
-    const unsigned row_bytes = unsigned(m) * unsigned(sizeof(V));
     idx += first;
     if (GATHER)
         dst += first * m;
@@ -318,8 +314,8 @@ __device__ void tile_index_staged(const V* src, V* dst, const int* idx, long lon
     const V* column = src + (GATHER ? r : 0);
     V* out_column = dst + (GATHER ? 0 : r);
     auto rows_of = [&](int p) { return cnt - p * per < per ? cnt - p * per : per; };
-    auto piece_at = [&](int p) { return reinterpret_cast<V*>(stage + (p % kPieces) * S::piece); };
-    auto index_at = [&](int p) { return s_idx + (p % kIndexSlots) * S::idx_slots; };
+    auto piece_at = [&](int p) { return reinterpret_cast<V*>(stage + (p % kPieces) * per * int(row_bytes)); };
+    auto index_at = [&](int p) { return s_idx + (p % kIndexSlots) * per; };
     auto issue_indices = [&](int p) {
         if (p < pieces) cp_async_range<S>(index_at(p), idx + p * per, rows_of(p) * 4, tid);
     };
@@ -436,19 +432,21 @@ __device__ void tile_index_staged(const V* src, V* dst, const int* idx, long lon
 // piece's indices are staged first (one coalesced read), invalid ones marked -1.
 template <class S, typename V, bool GATHER, int PF>
 __device__ void tile_index_wide(const V* src, V* dst, const int* idx, long long bound, long long first,
-                                  long long cnt, int m, unsigned char* stage, int* s_idx) {
-    constexpr int D = 2, kPiece = S::wide_piece, kSlots = S::wide_slots;
+                                  long long cnt, int m, unsigned char* stage) {
+    constexpr int D = kWidePieces;
     const int tid = opaque_tid();
-    // structs per piece: a multiple of 32 that fits the buffer and the index slots
-    int per = (kPiece / int(sizeof(V))) / m / 32 * 32;
-    if (per > kSlots) per = kSlots;
+    // structs per piece: a multiple of 32, so many that the pieces and their indices
+    // fit the staging memory
+    const int row_bytes = m * int(sizeof(V));
+    const int per = piece_rows(S::dyn_smem, true, row_bytes);
+    int* s_idx = reinterpret_cast<int*>(stage + D * per * row_bytes);
     // q / m for q < 2^12 and m <= 16 as a multiply and shift (exact there)
     const unsigned inv_m = (65536u + unsigned(m) - 1) / unsigned(m);
     const long long pieces = (cnt + per - 1) / per;
     auto issue = [&](long long p) {
         const int b = int(p % D);
-        V* buf = reinterpret_cast<V*>(stage + b * kPiece);
-        int* ix = s_idx + b * kSlots;
+        V* buf = reinterpret_cast<V*>(stage + b * per * row_bytes);
+        int* ix = s_idx + b * per;
         const long long base = first + p * per;
         const int n_here = int(cnt - p * per < per ? cnt - p * per : per);
         const int words = n_here * m;
@@ -471,8 +469,8 @@ __device__ void tile_index_wide(const V* src, V* dst, const int* idx, long long 
     };
     auto drain = [&](long long p) {
         const int b = int(p % D);
-        const V* buf = reinterpret_cast<const V*>(stage + b * kPiece);
-        const int* ix = s_idx + b * kSlots;
+        const V* buf = reinterpret_cast<const V*>(stage + b * per * row_bytes);
+        const int* ix = s_idx + b * per;
         const long long base = first + p * per;
         const int n_here = int(cnt - p * per < per ? cnt - p * per : per);
         const int words = n_here * m;
@@ -516,17 +514,17 @@ __device__ __forceinline__ void tile_index(const BatchTask& t, long long first, 
 
 template <class S, bool GATHER, int PF>
 __device__ __forceinline__ void tile_staged_pf(const BatchTask& t, long long first, int cnt, int m,
-                                               unsigned char* stage, int* s_idx, int* s_bad) {
+                                               unsigned char* stage, int* s_bad) {
     if (t.word_log2 == 4)
         tile_index_wide<S, uint4, GATHER, PF>(reinterpret_cast<const uint4*>(t.src), reinterpret_cast<uint4*>(t.dst),
-                                              t.idx, t.bound, first, cnt, m, stage, s_idx);
+                                              t.idx, t.bound, first, cnt, m, stage);
     else if (t.word_log2 == 3)
         tile_index_staged<S, uint2, GATHER, PF>(reinterpret_cast<const uint2*>(t.src), reinterpret_cast<uint2*>(t.dst),
-                                                t.idx, t.bound, first, cnt, m, stage, s_idx, s_bad);
+                                                t.idx, t.bound, first, cnt, m, stage, s_bad);
     else
         tile_index_staged<S, unsigned, GATHER, PF>(reinterpret_cast<const unsigned*>(t.src),
                                                    reinterpret_cast<unsigned*>(t.dst), t.idx, t.bound, first, cnt, m,
-                                                   stage, s_idx, s_bad);
+                                                   stage, s_bad);
 }
 
 // index_mode 2: staged with the context's fetch size; 3 / 4 (gathers): with
@@ -535,16 +533,16 @@ __device__ __forceinline__ void tile_staged_pf(const BatchTask& t, long long fir
 // 64-byte hint) are staged the same way: plain, or with the 64-byte hint.
 template <class S>
 __device__ __forceinline__ void tile_staged(const BatchTask& t, long long first, int cnt, unsigned char* stage,
-                                            int* s_idx, int* s_bad) {
+                                            int* s_bad) {
     const int m = t.words * 4 >> t.word_log2;
     if (t.op != TRV_OP_GATHER)
-        tile_staged_pf<S, false, 0>(t, first, cnt, m, stage, s_idx, s_bad);
+        tile_staged_pf<S, false, 0>(t, first, cnt, m, stage, s_bad);
     else if (t.index_mode == 3 || t.index_mode == 1)
-        tile_staged_pf<S, true, 64>(t, first, cnt, m, stage, s_idx, s_bad);
+        tile_staged_pf<S, true, 64>(t, first, cnt, m, stage, s_bad);
     else if (t.index_mode == 4)
-        tile_staged_pf<S, true, 128>(t, first, cnt, m, stage, s_idx, s_bad);
+        tile_staged_pf<S, true, 128>(t, first, cnt, m, stage, s_bad);
     else
-        tile_staged_pf<S, true, 0>(t, first, cnt, m, stage, s_idx, s_bad);
+        tile_staged_pf<S, true, 0>(t, first, cnt, m, stage, s_bad);
 }
 
 // Task of tile number `tile`: the last k with prefix[k] <= tile (tasks without
@@ -577,7 +575,6 @@ batch_kernel(const BatchTask* __restrict__ tasks, int ntasks, const long long* _
     __shared__ __align__(8) unsigned long long s_bar[S::ring];
     extern __shared__ __align__(128) unsigned char s_stage[];  // S::dyn_smem bytes
     __shared__ int s_bad[kIndexSlots];
-    int* s_idx = reinterpret_cast<int*>(s_stage + kPieces * S::piece);
     unsigned long long seq = 0;  // thread 0: bulk loads issued so far
     if (threadIdx.x == 0) {
         for (int k = 0; k < S::ring; ++k) mbar_init(&s_bar[k], 1);
@@ -646,7 +643,7 @@ batch_kernel(const BatchTask* __restrict__ tasks, int ntasks, const long long* _
             // the 128-register build: rows staged through shared memory, or
             // held in registers (index_mode 0 / 1)
             if (t.index_mode >= 2)
-                tile_staged<S>(t, first, int(cnt), s_stage, s_idx, s_bad);
+                tile_staged<S>(t, first, int(cnt), s_stage, s_bad);
             else if (t.op == TRV_OP_GATHER)
                 tile_index<S, true>(t, first, cnt);
             else
@@ -657,7 +654,7 @@ batch_kernel(const BatchTask* __restrict__ tasks, int ntasks, const long long* _
             // as well made it spill (456 bytes a thread) in every path, and
             // without them the 4096-array batch runs 21.32 instead of 22.22 ms
             // (its gathers 10.90 instead of 11.73 ms).
-            tile_staged<S>(t, first, int(cnt), s_stage, s_idx, s_bad);
+            tile_staged<S>(t, first, int(cnt), s_stage, s_bad);
         }
     }
 }

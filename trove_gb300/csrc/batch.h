@@ -39,16 +39,13 @@ struct TaskPlan {
                               // memory, 6 / 7 staged with the 64 / 128-byte hint
     int scatter_policy;       // 1 plain, 5 staged through shared memory
     int copy_bulk;            // copy tiles through the TMA bulk engine where aligned
+    int stage = 0;                // staging memory of a block: tiles are evened out to pieces and arrays; 0: left
     bool fetch_scatters = false;  // scatter destinations are fetched into L2 ahead of their rows
 };
 
 // Fills one task-table entry from a validated task; returns its tile count.
 long long plan_task(int op, uint32_t width, uint64_t n, uint64_t bound, const void* src, void* dst,
                     const int32_t* idx, const TaskPlan& p, BatchTask* d);
-
-// Tile size of a task of a batch that moves `bytes` bytes of structs in all on
-// `blocks` resident blocks, where nothing else chooses it.
-int fit_tile_bytes(int op, double bytes, int blocks);
 
 // Option checks shared by trv_batch_create and trv_batch_run_static.
 int check_batch_options(const trv_batch_options* opt);

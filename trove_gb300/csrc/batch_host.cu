@@ -9,6 +9,7 @@
 
 #include "autotune.h"
 #include "batch.h"
+#include "rules.h"
 #include "runtime.h"
 #include "trove_gb300.h"
 
@@ -69,29 +70,7 @@ int validate(const trv_task& t) {
     return TRV_OK;
 }
 
-// The largest tile when no tuned one exists: big enough to amortise the queue
-// step and the filling of the pieces, small enough that the tiles in flight, and
-// with them the sources and destinations in use, stay in L2, and that the last
-// ones balance across 152 SMs.  512 arrays of 1 K-4 M structs (14.9 GB) in us at
-// 24 / 32 / 48 / 64 / 128 KiB: copies 1013 / 1015 / 1020 / 1026 / 1032, gathers
-// 1479 / 1390 / 1356 / 1370 / 1508, scatters 510 / 513 / 523 / 538 / 672; all of
-// them 2844 with 128, 64 and 64 KiB and 2803 with these.
-int default_tile_bytes(int op) { return op == TRV_OP_SCATTER ? (24 << 10) : (48 << 10); }
-
 }  // namespace
-
-// A block takes about 25 us for a 64 KiB tile of gathered rows, so a batch that
-// comes to a few tiles a block is as long as its last ones: four tiles to each
-// resident block where the batch is that small, down to 8 KiB, below which the
-// queue step is felt.  Batches in us at 64 KiB (copies 128) / 2 / 4 / 8 to a block:
-// 87 arrays of 2-64 K structs 48.9 / 36.9 / 33.1 / 38.9, 343 of 0.5-64 K 68.4 /
-// 69.0 / 62.3 / 56.2, 16 of 4-32 K 26.6 / 12.3 / 12.3 / 12.3; 225 of 256-1024
-// 10.6 / 9.6 / 9.2 / 9.3 at 8 KiB and 10.3-10.4 at 4 KiB.
-int fit_tile_bytes(int op, double bytes, int blocks) {
-    const int most = default_tile_bytes(op), least = 8 << 10;
-    const double want = bytes / (4.0 * blocks);
-    return want >= most ? most : want <= least ? least : int(want) / 1024 * 1024;
-}
 
 // Tiles that fetch a scatter task's destination ahead of its rows: where rows
 // leave sectors partly written, each such write that misses L2 is filled from
@@ -99,11 +78,10 @@ int fit_tile_bytes(int op, double bytes, int blocks) {
 // than L2 the destination is seldom there when its turn comes.  2^24 scattered
 // rows in arrays of 2^19, plain / fetched in us: 8 bytes 185 / 121, 12 bytes 242 /
 // 146, 20 bytes 335 / 203, 36 bytes 463 / 302; arrays of 72 and 80 MiB 531 / 430
-// and 410 / 334, but of 144 MiB, which L2 does not hold, 628 / 641.  A batch of
-// little more than L2 only pays for the tiles (343 arrays, 124 MB of structs, 62.6
-// / 64.3 us; 60 arrays, 300 MB, 161.3 / 157.0).
+// and 410 / 334, but of 144 MiB, which L2 does not hold, 628 / 641.  Batches that fit
+// L2 only pay for the tiles; 343 scatters of 0.5-64 K rows (111 MB) 80 / 72.
 constexpr uint64_t kFetchLeast = uint64_t(256) << 10, kFetchMost = uint64_t(100) << 20;
-constexpr double kFetchBatchBytes = 200e6;  // bytes of structs in the batch
+constexpr double kFetchBatchBytes = 100e6;  // bytes of structs in the batch
 
 static int fetch_tiles(uint32_t width, uint64_t n, uint64_t bound, const void* dst) {
     const uint64_t bytes = bound * width;
@@ -135,6 +113,13 @@ long long plan_task(int op, uint32_t width, uint64_t n, uint64_t bound, const vo
                     : op == TRV_OP_SCATTER ? (p.scatter_policy == 5 ? 2 : 0)
                                            : 0;
     d->copy_bulk = p.copy_bulk;
+    if (p.stage && op != TRV_OP_COPY && n > 0) {
+        const int rows = piece_rows(p.stage, d->word_log2 == 4, int(width));
+        if (tile % rows * 25 <= tile) tile -= tile % rows;  // no last piece of a 25th of the tile or less
+        const long long tiles = ((long long)n + tile - 1) / tile;
+        if (tiles <= 16) tile = (((long long)n + tiles - 1) / tiles + 31) / 32 * 32;  // no short last tile of few
+        d->tile_structs = int(tile);
+    }
     d->fetch_tiles = op == TRV_OP_SCATTER && n > 0 && p.fetch_scatters ? fetch_tiles(width, n, bound, dst) : 0;
     return ((long long)n + tile - 1) / tile + d->fetch_tiles;
 }
@@ -158,17 +143,19 @@ int plan_batch(const trv_task* tasks, uint64_t count, const trv_batch_options* o
     uint64_t vote2 = 0, vote4 = 0, total = 0;
     double all = 0;  // bytes of structs, unchecked as yet
     for (uint64_t k = 0; k < count; ++k) all += double(tasks[k].n) * tasks[k].width;
+    for (uint64_t k = 0; k < count; ++k) {
+        const int rc = validate(tasks[k]);
+        if (rc != TRV_OK) return rc;
+    }
+    const int shape = (opt && opt->blocks_per_sm) ? opt->blocks_per_sm : 4;
+    const TileRule rule([&](uint64_t k) { return TileTask{tasks[k].op == TRV_OP_COPY, tasks[k].width, tasks[k].n}; },
+                        count, shape * device_info().sm_count);
     prefix[0] = 0;
     for (uint64_t k = 0; k < count; ++k) {
         const trv_task& t = tasks[k];
-        const int rc = validate(t);
-        if (rc != TRV_OK) return rc;
         TuneChoice c;
         const bool tuned = tune_lookup(TuneKey{SCOPE_BATCH, t.op, int(t.width), len_bucket(t.n)}, &c);
         TaskPlan p;
-        p.tile_bytes = (opt && opt->tile_bytes > 0) ? opt->tile_bytes
-                       : (tuned && c.tile_bytes > 0) ? c.tile_bytes
-                                                     : fit_tile_bytes(t.op, all, 4 * device_info().sm_count);
         // Gather and scatter rows are staged through shared memory with
         // cp.async unless chosen otherwise: on the 4096-array workload (4
         // blocks per SM) its gathers took 12.1 ms that way against 20.5 ms
@@ -182,6 +169,16 @@ int plan_batch(const trv_task* tasks, uint64_t count, const trv_batch_options* o
         p.scatter_policy = (opt && opt->scatter_policy) ? opt->scatter_policy
                            : (tuned && c.cache_policy)  ? c.cache_policy
                                                         : 5;
+        // Rows held in registers (the 2-block build, policies 1 and 4) move 512 at a
+        // time whatever the batch, and want the large tile of long tasks.
+        const int policy = t.op == TRV_OP_GATHER ? p.gather_policy : p.scatter_policy;
+        const bool held = shape == 2 && t.op != TRV_OP_COPY && (policy == 1 || policy == 4);
+        p.tile_bytes = (opt && opt->tile_bytes > 0) ? opt->tile_bytes
+                       : (tuned && c.tile_bytes > 0) ? c.tile_bytes
+                       : held                        ? kLargestTile[1]
+                                                     : rule.tile_bytes(t.op, t.width);
+        const bool chosen = !(opt && opt->tile_bytes > 0) && !(tuned && c.tile_bytes > 0);
+        p.stage = chosen && !held && !rule.one_wave() ? stage_bytes(shape) : 0;
         const int cp = (opt && opt->copy_path) ? opt->copy_path : (tuned && c.path) ? c.path : TRV_PATH_AUTO;
         p.copy_bulk = cp == TRV_PATH_VECTOR ? 0 : 1;
         p.fetch_scatters = all > kFetchBatchBytes;

@@ -169,6 +169,110 @@ TRV_HOST_DEVICE inline bool sample_near(int a, int b, int row_bytes) {
     return (d < 0 ? -d : d) * row_bytes <= kNearBytes;
 }
 
+// ---- tiles of a batch (batch.cu) -----------------------------------------------
+
+// Staging memory of a block of the batch kernel, by its resident blocks per SM, and
+// the rows of one staged piece: of 16-byte words two pieces and their indices fit it,
+// of 4- and 8-byte words three and four index arrays.  A piece of 16-byte words is at
+// most a whole number of words for each of 256 threads, four or eight (2^24 rows of 32
+// bytes in order 173 us in pieces of 512, 189 in pieces of 544).
+constexpr int kPieces = 3, kIndexSlots = 4, kWidePieces = 2;
+TRV_HOST_DEVICE constexpr int stage_bytes(int blocks_per_sm) { return blocks_per_sm == 2 ? 81408 : 40704; }
+TRV_HOST_DEVICE constexpr int piece_rows(int stage, bool wide, int row_bytes) {
+    const int fit = wide ? stage / (kWidePieces * (row_bytes + 4)) : stage / (kPieces * row_bytes + kIndexSlots * 4);
+    const int even = stage / stage_bytes(4) * 4 * 256 * 16 / row_bytes;
+    return (wide && even < fit ? even : fit) / 32 * 32;
+}
+
+// The largest tile of copies, gathers and scatters (by trv_op): big enough to amortise
+// the queue step and the filling of the pieces, small enough that the tiles in flight,
+// and with them the sources and destinations in use, stay in L2, and that the last
+// ones balance across 152 SMs.  512 arrays of 1 K-4 M structs (14.9 GB) in us at 24 /
+// 32 / 48 / 64 / 128 KiB: copies 1013 / 1015 / 1020 / 1026 / 1032, gathers 1479 / 1390 /
+// 1356 / 1370 / 1508, scatters 510 / 513 / 523 / 538 / 672.  220 scatters of 1 K-1 M
+// rows (1 GB) at 24 / 48 / 64 KiB: at random 501 / 477 / 479, in order 373 / 341 / 339.
+// 24 gathers of 2^19 rows of 64 bytes in order: 257 at 48 KiB, 251 at 64.  A tile
+// that is a little longer than whole pieces is cut to them (plan_task): of 16-byte rows
+// 64 KiB are 4096, four pieces of 992 and a fifth of 128.
+constexpr int kLargestTile[3] = {128 << 10, 64 << 10, 48 << 10};
+
+struct TileTask {
+    bool copy;
+    uint32_t width;
+    uint64_t n;
+};
+
+// Tile sizes of a batch where nothing else chooses them.  A tile takes a block about
+// 8 us before its first rows arrive, then 1.2 ns a row and 23 ps a byte (one array a
+// block, us: 16384 rows of 4 bytes 28, 1024 rows of 64 bytes 10), so rows of w bytes
+// weigh w + 48, and a batch of mixed widths is dealt out by weight: in bytes alone a
+// tile of narrow rows takes three times as long as one of wide rows.
+//
+// A batch that fits the resident blocks in one wave of tiles of at most 64 KiB gets
+// tiles that just do so, whatever is left over of each array counted: a second wave
+// of a few tiles costs as much as the first (256 arrays of 8192 rows of 16 bytes 24.7
+// us in one wave of 512 tiles, 28.8 in 1024 and 31.4 in 2560).  A larger one gets four
+// to a block, gathers two, up to the largest, so that the last ones are short (87
+// arrays of 2-64 K structs, 46 MB of gathers 57 us with the largest tile, 43 so);
+// copies, which take time by their bytes, not below 48 KiB.
+class TileRule {
+public:
+    static constexpr int kRowWeight = 48;
+    static constexpr double kLeastWork = 24 << 10;  // of a tile: less is lost in the queue step
+    static constexpr double kOneWaveBytes = 64 << 10;
+
+    template <typename TaskAt>  // TileTask TaskAt(k), k < count
+    TileRule(TaskAt&& at, uint64_t count, int blocks) {
+        double total = 0, most = 0;  // work, and the largest share of bytes in it
+        uint64_t arrays = 0;
+        for (uint64_t k = 0; k < count; ++k) {
+            const TileTask t = at(k);
+            if (!t.n) continue;
+            const double w = weight(t.copy, t.width);
+            total += double(t.n) * w;
+            most = most < t.width / w ? t.width / w : most;
+            ++arrays;
+        }
+        work_ = total / blocks < kLeastWork ? kLeastWork : total / blocks;
+        while (work_ * most <= kOneWaveBytes && (arrays <= uint64_t(blocks) || work_ == kLeastWork)) {
+            double tiles = 0;
+            for (uint64_t k = 0; k < count; ++k) {
+                const TileTask t = at(k);
+                const uint64_t each = structs(work_, t.copy, t.width);
+                tiles += double(t.n / each + (t.n % each != 0));
+            }
+            if (tiles <= blocks || work_ == kLeastWork) {
+                one_wave_ = true;
+                return;
+            }
+            const double over = tiles / blocks, limit = kOneWaveBytes / most;
+            if (work_ == limit) break;
+            work_ *= over > 1.25 ? 1.25 : over < 1.05 ? 1.05 : over;
+            if (work_ > limit) work_ = limit;  // the last try
+        }
+        work_ = total / blocks;
+    }
+
+    bool one_wave() const { return one_wave_; }
+
+    int tile_bytes(int op, uint32_t width) const {
+        const bool copy = op == 0;
+        if (one_wave_) return int(structs(work_, copy, width) * width);
+        const double bytes = work_ / (op == 1 ? 2 : 4) * width / weight(copy, width);
+        const double most = kLargestTile[op], least = copy ? 48 << 10 : kLeastWork * width / weight(copy, width);
+        return int(bytes >= most ? most : bytes <= least ? least : bytes);
+    }
+
+private:
+    static double weight(bool copy, uint32_t width) { return copy ? width : width + kRowWeight; }
+    static uint64_t structs(double work, bool copy, uint32_t width) {  // of a tile: whole warps, as plan_task rounds
+        const uint64_t s = uint64_t(work / weight(copy, width)) / 32 * 32;
+        return s < 32 ? 32 : s;
+    }
+    double work_ = 0;  // of a tile
+    bool one_wave_ = false;
+};
+
 // Rows of any width and alignment move in 4-byte words (packed.cu) where that
 // beats a thread per row moving bytes (flat.cu).  A word takes its bytes from at
 // most two rows, and words read past a row from at most two more: rows have at least

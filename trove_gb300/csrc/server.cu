@@ -34,6 +34,7 @@
 
 #include "autotune.h"
 #include "batch.h"
+#include "rules.h"
 #include "runtime.h"
 #include "trove_gb300.h"
 
@@ -295,8 +296,12 @@ struct trv_server {
             }
             const Tables h(s.h_tables, take), d(s.d_tables, take);
             long long tiles[2] = {0, 0};
-            double bytes[2] = {0, 0};
-            for (size_t k = 0; k < take; ++k) bytes[k < ns ? 0 : 1] += double(s.todo[k].first.n) * s.todo[k].first.width;
+            const auto task_at = [&](uint64_t k) {
+                const trv_request& r = s.todo[k].first;
+                return TileTask{r.op == TRV_OP_COPY, r.width, r.n};
+            };
+            const TileRule rule[2] = {TileRule(task_at, ns, grid),
+                                      TileRule([&](uint64_t k) { return task_at(ns + k); }, take - ns, grid_large)};
             for (size_t k = 0; k < take; ++k) {
                 const trv_request& r = s.todo[k].first;
                 const int grp = k < ns ? 0 : 1;
@@ -304,12 +309,14 @@ struct trv_server {
                 const bool tuned = tune_lookup(TuneKey{SCOPE_BATCH, r.op, int(r.width), len_bucket(r.n)}, &c);
                 const int tb = cfg.tile_bytes > 0 ? cfg.tile_bytes
                                : (tuned && c.tile_bytes > 0) ? c.tile_bytes
-                                                             : fit_tile_bytes(r.op, bytes[grp], grp ? grid_large : grid);
+                                                             : rule[grp].tile_bytes(r.op, r.width);
                 TaskPlan p;
                 p.tile_bytes = tb;
                 p.gather_policy = 7;  // rows staged through shared memory, 128-byte L2 fetches
                 p.scatter_policy = 5;
                 p.copy_bulk = 1;
+                if (cfg.tile_bytes <= 0 && !(tuned && c.tile_bytes > 0) && !rule[grp].one_wave())
+                    p.stage = stage_bytes(kServerBlocksPerSm);
                 const long long nt = plan_task(r.op, r.width, r.n, r.src_n, r.src, arena.base() + s.todo[k].second,
                                                r.idx, p, &h.tasks[k]);
                 h.prefix[k + size_t(grp)] = tiles[grp];
