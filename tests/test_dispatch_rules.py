@@ -34,6 +34,10 @@ int tiles(const long long* tasks, long long count, int blocks, int* bytes) {
     for (long long k = 0; k < count; ++k) bytes[k] = rule.tile_bytes(int(tasks[3 * k]), uint32_t(tasks[3 * k + 1]));
     return rule.one_wave();
 }
+int tuned_tile(int op, unsigned width, unsigned long long n, unsigned long long count, int tuned) {
+    const trv::TileRule rule([&](uint64_t) { return trv::TileTask{op == 0, width, n}; }, count, 608);
+    return rule.tile_bytes(op, width, tuned);
+}
 int piece_rows(int blocks_per_sm, int wide, int row_bytes) {
     return trv::piece_rows(trv::stage_bytes(blocks_per_sm), wide, row_bytes);
 }
@@ -61,6 +65,7 @@ def rules(tmp_path_factory):
     lib.most_pass_words.restype = ctypes.c_uint32
     lib.parts.argtypes = [ctypes.c_uint32, ctypes.c_uint64, ctypes.c_uint64, ctypes.c_int]
     lib.tiles.argtypes = [ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int, ctypes.c_void_p]
+    lib.tuned_tile.argtypes = [ctypes.c_int, ctypes.c_uint32, ctypes.c_uint64, ctypes.c_uint64, ctypes.c_int]
     lib.exit_unroll.argtypes = [ctypes.c_uint32, ctypes.c_uint64]
     for f in (lib.packed, lib.rows_unroll, lib.struct_unroll, lib.layout_unroll):
         f.argtypes = [ctypes.c_int, ctypes.c_uint32, ctypes.c_uint64]
@@ -189,3 +194,15 @@ def test_staged_pieces_fit_their_memory(rules):
                 rows = rules.piece_rows(blocks, 1, width)
                 # the division of a word's number by words to a row holds for 12 bits
                 assert rows % 32 == 0 and rows >= 32 and 2 * rows * (width + 4) <= memory and rows * width // 16 <= 4096
+
+
+def test_tuned_tiles_do_not_outgrow_a_small_batch(rules):
+    """A tuned tile is kept where the batch is large enough for the largest tiles, and
+    where it is smaller than the batch's own; 0 stands for none."""
+    for op in (0, 1, 2):
+        for width in (4, 20, 64):
+            own = rules.tuned_tile(op, width, 20000, 16, 0)
+            assert own < 65536
+            for tuned in (32 << 10, 64 << 10, 1 << 20):
+                assert rules.tuned_tile(op, width, 20000, 16, tuned) == min(own, tuned)
+                assert rules.tuned_tile(op, width, 1 << 22, 64, tuned) == tuned

@@ -177,7 +177,7 @@ static int32_t autotune_call_impl(int32_t op, uint32_t width, uint64_t n, void* 
         for (int u : {1, 2, 4, 8}) cands.push_back({TRV_PATH_WARP, u, 0, 0, 0, 0});
     } else if (op == TRV_OP_COPY) {
         for (int chunk : {16 << 10, 24 << 10}) cands.push_back({TRV_PATH_BULK, 0, 0, 0, chunk, 0});
-        for (int u : {2, 4, 8}) cands.push_back({TRV_PATH_VECTOR, u, 0, 0, 0, 0});
+        for (int u : {1, 2, 4, 8}) cands.push_back({TRV_PATH_VECTOR, u, 0, 0, 0, 0});
         if (width % 4 == 0 && width <= 64)
             for (int u : {1, 2, 4, 8}) cands.push_back({TRV_PATH_WARP, u, 0, 0, 0, 0});
     } else if (width % 4 == 0 && width <= 64) {
@@ -264,7 +264,7 @@ static int32_t autotune_batch_impl(const trv_task* tasks, uint64_t count, void* 
         const int op = std::get<0>(kv.first);
         // (tile_bytes, blocks per SM, gather / scatter policy, copy tile path)
         std::vector<std::tuple<int, int, int, int>> cands;
-        for (int tb : {32 << 10, 64 << 10, 128 << 10, 256 << 10, 1 << 20})
+        for (int tb : {0, 32 << 10, 64 << 10, 128 << 10, 256 << 10, 1 << 20})  // 0: the rule of untuned batches
             for (int bps : {2, 4})
                 for (int gp : {1, 4, 5, 6, 7})
                     for (int cpath : {TRV_PATH_AUTO, TRV_PATH_VECTOR}) {

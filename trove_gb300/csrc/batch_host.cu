@@ -174,9 +174,8 @@ int plan_batch(const trv_task* tasks, uint64_t count, const trv_batch_options* o
         const int policy = t.op == TRV_OP_GATHER ? p.gather_policy : p.scatter_policy;
         const bool held = shape == 2 && t.op != TRV_OP_COPY && (policy == 1 || policy == 4);
         p.tile_bytes = (opt && opt->tile_bytes > 0) ? opt->tile_bytes
-                       : (tuned && c.tile_bytes > 0) ? c.tile_bytes
-                       : held                        ? kLargestTile[1]
-                                                     : rule.tile_bytes(t.op, t.width);
+                       : held ? (tuned && c.tile_bytes > 0 ? c.tile_bytes : kLargestTile[1])
+                              : rule.tile_bytes(t.op, t.width, tuned ? c.tile_bytes : 0);
         const bool chosen = !(opt && opt->tile_bytes > 0) && !(tuned && c.tile_bytes > 0);
         p.stage = chosen && !held && !rule.one_wave() ? stage_bytes(shape) : 0;
         const int cp = (opt && opt->copy_path) ? opt->copy_path : (tuned && c.path) ? c.path : TRV_PATH_AUTO;

@@ -308,8 +308,7 @@ struct trv_server {
                 TuneChoice c;
                 const bool tuned = tune_lookup(TuneKey{SCOPE_BATCH, r.op, int(r.width), len_bucket(r.n)}, &c);
                 const int tb = cfg.tile_bytes > 0 ? cfg.tile_bytes
-                               : (tuned && c.tile_bytes > 0) ? c.tile_bytes
-                                                             : rule[grp].tile_bytes(r.op, r.width);
+                                                  : rule[grp].tile_bytes(r.op, r.width, tuned ? c.tile_bytes : 0);
                 TaskPlan p;
                 p.tile_bytes = tb;
                 p.gather_policy = 7;  // rows staged through shared memory, 128-byte L2 fetches
