@@ -85,7 +85,7 @@ typedef struct trv_launch {
                               3 as 1, random side kept in L2 (evict-last); 4 as 1, random-side
                               loads with a 64-byte L2 prefetch-size hint; 5 as 1, random-side
                               loads with a 128-byte L2 prefetch-size hint (gathers); 6 (scatters)
-                              the default: as 1, but onto destinations of 22 MiB to about
+                              the default: as 1, but onto destinations of 40 MiB to about
                               1.3 GiB structs that do not fill whole 32-byte sectors go after
                               the destination has been fetched into L2, in one pass or, above
                               64 MiB, in passes over 56 MiB parts of it, so that partial-sector

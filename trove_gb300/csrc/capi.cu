@@ -418,7 +418,8 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
         const bool sampled = form == kBySample;
         if (form != kByBytes) {
             if (parts == 1)
-                launch_fetch_destination(IndexArgs{src, dst, idx, (long long)n, (long long)bound, 1}, int(width), st);
+                launch_fetch_destination(IndexArgs{src, dst, idx, (long long)n, (long long)bound, 1}, int(width),
+                                         kPlainPackedBytes, st);
             launch_index_packed(gather, src, idx, dst, (long long)bound, (long long)n, int(width),
                                 grid_req > 0 ? grid_req : grid_req < 0 ? cap : 0, sampled, st);
         }
@@ -488,7 +489,7 @@ static int32_t index_op(bool gather, void* dst, const void* src, uint64_t bound,
             const int wb = kp == &ops->scatter_rows[0][slot] ? ops->rows_word_bytes : 4;
             launch_scatter_passes(wb, a, int(width) / wb, parts, st);
         } else {
-            launch_fetch_destination(a, int(width), st);
+            launch_fetch_destination(a, int(width), kPlainScatterBytes, st);
             k.launch(a, grid, 256, st);
         }
         return check_launch();

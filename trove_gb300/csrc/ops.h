@@ -5,6 +5,8 @@
 
 #include <cuda_runtime.h>
 
+#include <cstdint>
+
 namespace trv {
 
 // Unroll factors offered (structs per lane per pass); index = log2(unroll).
@@ -85,9 +87,10 @@ bool launch_wide_rows(bool gather, int word_bytes, const IndexArgs& a, int m, cu
 
 // Scatter onto a large destination (scatter_parts.cu), any width that is a multiple
 // of 4 bytes, n >= 2: in `passes` parts of the destination (one launch), or the
-// fetch of the destination into L2 ahead of a scatter in one pass.
+// fetch of the destination into L2 ahead of a scatter in one pass, unless the rows
+// lie within `plain` bytes of it.
 void launch_scatter_passes(int word_bytes, const IndexArgs& a, int m, int passes, cudaStream_t st);
-void launch_fetch_destination(const IndexArgs& a, int row_bytes, cudaStream_t st);
+void launch_fetch_destination(const IndexArgs& a, int row_bytes, uint64_t plain, cudaStream_t st);
 
 // Defined in width_ops.cu, one specialisation per translation unit.
 template <int S>

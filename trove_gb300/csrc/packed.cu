@@ -165,13 +165,14 @@ gather_packed_kernel(const unsigned char* __restrict__ src, unsigned bound, cons
 // One warp: kRows source rows, each as the `slots` aligned words of its
 // destination row; slot k of a row that starts c bytes past a 4-byte boundary
 // holds its bytes 4k - c to 4k - c + 3.
-template <int kRows>
+template <int kRows, bool SAMPLED>
 __global__ void __launch_bounds__(32 * kWarps)
 scatter_packed_kernel(const unsigned char* __restrict__ src, const int* __restrict__ idx,
-                      unsigned char* __restrict__ dst, unsigned bound, long long n, int width, bool sampled) {
+                      unsigned char* __restrict__ dst, unsigned bound, long long n, int width) {
     __shared__ int s_id[kWarps][kRows];
     const int lane = int(threadIdx.x & 31u), warp = int(threadIdx.x >> 5);
-    if (sampled && IndexSample(idx, n, lane).rows_adjoin(width)) return;
+    if constexpr (SAMPLED)
+        if (IndexSample(idx, n, lane).rows_adjoin(width)) return;
     const unsigned char* hi = src + n * (long long)width;
     const int slots = (width + 6) / 4;
     const int step_j = 32 / slots, step_k = 32 % slots;
@@ -251,8 +252,10 @@ static void launch(bool gather, const void* src, const int* idx, void* dst, long
     }
     if (gather)
         gather_packed_kernel<ROWS><<<grid, 32 * kWarps, 0, st>>>(s, clamp_bound(bound), idx, d, n, width);
+    else if (ROWS == 128 && sampled)
+        scatter_packed_kernel<128, true><<<grid, 32 * kWarps, 0, st>>>(s, idx, d, clamp_bound(bound), n, width);
     else
-        scatter_packed_kernel<ROWS><<<grid, 32 * kWarps, 0, st>>>(s, idx, d, clamp_bound(bound), n, width, sampled);
+        scatter_packed_kernel<ROWS, false><<<grid, 32 * kWarps, 0, st>>>(s, idx, d, clamp_bound(bound), n, width);
 }
 
 // Rows to a warp, 8 to 128.  More rows to a warp waste less on its start and its
@@ -282,7 +285,7 @@ static int rows_to_a_warp(int width, long long n) {
 
 void launch_index_packed(bool gather, const void* src, const int* idx, void* dst, long long bound, long long n,
                          int width, int grid, bool sampled, cudaStream_t st) {
-    switch (rows_to_a_warp(width, n)) {
+    switch (sampled ? 128 : rows_to_a_warp(width, n)) {
         case 8: return launch<8>(gather, src, idx, dst, bound, n, width, grid, sampled, st);
         case 16: return launch<16>(gather, src, idx, dst, bound, n, width, grid, sampled, st);
         case 32: return launch<32>(gather, src, idx, dst, bound, n, width, grid, sampled, st);

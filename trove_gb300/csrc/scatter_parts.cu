@@ -50,12 +50,12 @@ __device__ __forceinline__ int ld_once(const int* p, unsigned long long pol) {
 // Ahead of a one-pass scatter: what the sampled indices span of the destination.
 __global__ void __launch_bounds__(256)
 fetch_destination_kernel(const unsigned char* dst, unsigned bound, const int* __restrict__ idx, long long n,
-                         int row_bytes) {
+                         int row_bytes, unsigned long long plain) {
     const IndexSample sample(idx, n, int(threadIdx.x & 31u));
     if (sample.local(row_bytes)) return;
     unsigned first, rows;
     sample.span(bound, first, rows);
-    if (rows * (unsigned long long)unsigned(row_bytes) <= kPlainScatterBytes) return;
+    if (rows * (unsigned long long)unsigned(row_bytes) <= plain) return;  // L2 holds them as it is
     const unsigned long long p = reinterpret_cast<unsigned long long>(dst) + first * (unsigned long long)unsigned(row_bytes);
     fetch_part(p, p + rows * (unsigned long long)unsigned(row_bytes), blockIdx.x, gridDim.x);
 }
@@ -255,9 +255,9 @@ void launch_passes(const IndexArgs& a, int m, int passes, cudaStream_t st) {
 }
 }  // namespace
 
-void launch_fetch_destination(const IndexArgs& a, int row_bytes, cudaStream_t st) {
+void launch_fetch_destination(const IndexArgs& a, int row_bytes, uint64_t plain, cudaStream_t st) {
     fetch_destination_kernel<<<kFetchBlocks, 256, 0, st>>>(static_cast<const unsigned char*>(a.dst), unsigned(a.bound > 0x80000000ll ? 0x80000000ll : a.bound),
-                                                           a.idx, a.n, row_bytes);
+                                                           a.idx, a.n, row_bytes, plain);
 }
 
 void launch_scatter_passes(int word_bytes, const IndexArgs& a, int m, int passes, cudaStream_t st) {
