@@ -95,6 +95,8 @@ def parse():
                         "or 'none'")
     p.add_argument("--sub-cpu-seconds", type=float, default=3.0,
                    help="CPU-baseline seconds of each sub-record")
+    p.add_argument("--details", default=None, metavar="FILE",
+                   help="also write the full record (every kernel, every sub-record) there")
     p.add_argument("--no-check", action="store_true")
     p.add_argument("--no-tune", action="store_true")
     p.add_argument("--array-mib", type=int, default=ARRAY_BYTES >> 20,
@@ -1560,6 +1562,33 @@ def free_device(torch, dev):
     torch.cuda.empty_cache()
 
 
+SUMMARY_LIMIT = 3000  # characters of the result line
+
+
+def summary(line):
+    """The result line: the record without its per-kernel tables, each sub-record
+    by its headline figures, and no notes where they make it too long to be read
+    back whole from the end of a log (the full record is some 50 KB)."""
+    keep = {k: v for k, v in line.items() if k not in ("kernels", "details", "ceiling", "reference_gpu")}
+    keep["config"] = {k: v for k, v in line["config"].items() if k != "structs_per_width"}
+    details = line.get("details") or {}
+    if "targets" in details:
+        keep["targets"] = {k: {"ratio": t["ratio"], "met": t["met"]} if "ratio" in t else
+                           {"gbs": t["slowest_kernel_gbs"], "met": t["met"]} for k, t in details["targets"].items()}
+    if "configs" in details:
+        keep["configs"] = {name: {k: rec[k] for k in ("value", "ms_per_step", "bit_exact", "p50_ms", "p99_ms")
+                                  if rec.get(k) is not None} for name, rec in details["configs"].items()}
+    for name in ("cpu_baseline", "roofline", "configs", "targets"):
+        if len(json.dumps(keep)) <= SUMMARY_LIMIT:
+            break
+        rec = keep.get(name)
+        if name in ("configs", "targets"):
+            keep.pop(name, None)
+        elif isinstance(rec, dict):
+            keep[name] = {k: v for k, v in rec.items() if not isinstance(v, (str, dict, list)) or k in ("kind", "unit")}
+    return keep
+
+
 def run_trove(args, world, rank, local):
     import torch
 
@@ -1598,7 +1627,9 @@ def run_trove(args, world, rank, local):
         line["gpu_launches"] += sum(r.get("gpu_launches") or 0 for r in subs.values())
         line["details"]["targets"] = targets(line, subs)
     if rank == 0:
-        print(json.dumps(line), flush=True)
+        if args.details:
+            Path(args.details).write_text(json.dumps(line) + "\n")
+        print(json.dumps(summary(line)), flush=True)
 
 
 def main():
