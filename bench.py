@@ -1562,7 +1562,7 @@ def free_device(torch, dev):
     torch.cuda.empty_cache()
 
 
-SUMMARY_LIMIT = 3000  # characters of the result line
+SUMMARY_LIMIT = 2800  # characters of the result line
 
 
 def summary(line):
