@@ -171,9 +171,10 @@ def test_tiles_of_a_batch(rules):
         for width in range(4, 65, 4):
             for count, n in [(16, 1024), (16, 32768), (256, 512), (256, 2048), (100, 20000), (607, 999), (1, 1 << 18)]:
                 one, size, count_of = tiles_of(rules, [(op, width, n)] * count)
-                assert size.max() <= 65536 if one else (131072, 65536, 49152)[op]
+                assert size.max() <= (65536 if one else (131072, 65536, 49152)[op])
                 if count * n * width <= 30 << 20:
-                    assert one and (count_of.sum() <= 608 or size[0] * (width + 48 * (op > 0)) <= 25000 * width)
+                    assert one and count_of.sum() <= 608
+            assert tiles_of(rules, [(op, width, 512 if op else 8192 // width // 32 * 32)] * 256)[2].max() == 1
             one, size, _ = tiles_of(rules, [(op, width, 1 << 22)] * 40)
             assert not one and size[0] == (131072, 65536, 49152)[op]
     one, size, count_of = tiles_of(rules, [(1, 16, 8192)] * 256)  # 64 KiB and two to an array just fit

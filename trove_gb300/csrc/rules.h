@@ -218,8 +218,10 @@ struct TileTask {
 class TileRule {
 public:
     static constexpr int kRowWeight = 48;
-    static constexpr double kLeastWork = 24 << 10;  // of a tile: less is lost in the queue step
     static constexpr double kOneWaveBytes = 64 << 10;
+    // A shorter tile loses more in the queue step than it gains (256 arrays of 512 rows
+    // 8.4 us in one tile each, 10.4 in two).
+    static constexpr uint32_t kLeastRows = 512, kLeastCopyBytes = 8 << 10;
 
     template <typename TaskAt>  // TileTask TaskAt(k), k < count
     TileRule(TaskAt&& at, uint64_t count, int blocks) {
@@ -233,15 +235,16 @@ public:
             most = most < t.width / w ? t.width / w : most;
             ++arrays;
         }
-        work_ = total / blocks < kLeastWork ? kLeastWork : total / blocks;
-        while (work_ * most <= kOneWaveBytes && (arrays <= uint64_t(blocks) || work_ == kLeastWork)) {
+        work_ = total / blocks;
+        if (!arrays) one_wave_ = true;
+        while (!one_wave_ && arrays <= uint64_t(blocks) && work_ * most <= kOneWaveBytes) {
             double tiles = 0;
             for (uint64_t k = 0; k < count; ++k) {
                 const TileTask t = at(k);
                 const uint64_t each = structs(work_, t.copy, t.width);
                 tiles += double(t.n / each + (t.n % each != 0));
             }
-            if (tiles <= blocks || work_ == kLeastWork) {
+            if (tiles <= blocks) {
                 one_wave_ = true;
                 return;
             }
@@ -268,15 +271,15 @@ public:
         const bool copy = op == 0;
         if (one_wave_) return int(structs(work_, copy, width) * width);
         const double bytes = work_ / (op == 1 ? 2 : 4) * width / weight(copy, width);
-        const double most = kLargestTile[op], least = copy ? 48 << 10 : kLeastWork * width / weight(copy, width);
+        const double most = kLargestTile[op], least = copy ? 48 << 10 : kLeastRows * width;
         return int(bytes >= most ? most : bytes <= least ? least : bytes);
     }
 
 private:
     static double weight(bool copy, uint32_t width) { return copy ? width : width + kRowWeight; }
     static uint64_t structs(double work, bool copy, uint32_t width) {  // of a tile: whole warps, as plan_task rounds
-        const uint64_t s = uint64_t(work / weight(copy, width)) / 32 * 32;
-        return s < 32 ? 32 : s;
+        const uint64_t s = uint64_t(work / weight(copy, width)), least = copy ? kLeastCopyBytes / width : kLeastRows;
+        return (s < least ? least : s) / 32 * 32;
     }
     double work_ = 0;  // of a tile
     bool one_wave_ = false;
