@@ -511,9 +511,10 @@ def test_scatter_orders_of_indices(cuda, width, mib):
     wide[::3] = (torch.randperm(bound // 2, device="cuda") + bound // 4)[:(n + 2) // 3]
     few = torch.full((n,), bound, device="cuda", dtype=torch.int64)
     few[7] = bound - 1
+    tenths = torch.where(torch.rand(n, device="cuda") < 0.9, torch.full_like(order, bound), torch.randperm(bound, device="cuda")[:n])
     for name, idx in (("order", order), ("runs", torch.cat([runs, order[runs.numel():]])),
                       ("random", torch.randperm(bound, device="cuda")[:n]), ("inside", inside), ("wide", wide),
-                      ("few", few)):
+                      ("few", few), ("tenths", tenths), ("tenths in order", torch.where(tenths < bound, order, tenths))):
         idx = idx.to(torch.int32)
         ok = (idx >= 0) & (idx < bound)
         expect = torch.full((bound, width), SENTINEL, dtype=torch.uint8, device="cuda")

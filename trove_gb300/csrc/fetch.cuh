@@ -29,6 +29,11 @@ struct IndexSample {
         const long long d = (long long)b - a;
         return __popc(__ballot_sync(0xFFFFFFFFu, (d < 0 ? -d : d) * row_bytes <= 64)) >= 20;
     }
+    // Whether half of the sampled indices or fewer lie below `bound`.
+    __device__ __forceinline__ bool mostly_skipped(unsigned bound) const {
+        return __popc(__ballot_sync(0xFFFFFFFFu, unsigned(a) < bound)) +
+                   __popc(__ballot_sync(0xFFFFFFFFu, unsigned(b) < bound)) <= kSamples;
+    }
     // The rows [first, first + rows) that the sampled indices below `bound` lie in.
     __device__ __forceinline__ void span(unsigned bound, unsigned& first, unsigned& rows) const {
         const bool va = unsigned(a) < bound, vb = unsigned(b) < bound;

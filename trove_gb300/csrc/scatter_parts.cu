@@ -96,7 +96,7 @@ struct PassPlan {
 // where the first blocks work).  On fewer rows, slabs would come to hardly more
 // than a wave of blocks, and all blocks take kOrderRows rows to a warp (200 MiB of
 // sorted rows of 80 bytes 83 us in slabs, 68 so, 66 plain).
-constexpr int kOrderRows = 128;
+constexpr int kOrderRows = 128, kOrderWideRows = 64;
 constexpr int kBodyBlocks = 2048;  // blocks that move a part's structs, at most (launch_passes)
 
 template <typename V, int G>
@@ -107,7 +107,7 @@ __device__ __forceinline__ void scatter_in_order(const V* __restrict__ src, cons
     const unsigned each = slabs && sizeof(V) > 4 ? plan.passes : 1u;
     const unsigned c = blockIdx.x / each, blocks = slabs ? plan.body : gridDim.x;
     if (c * each != blockIdx.x || c >= blocks) return;
-    const int rows = slabs ? kSlab : kOrderRows;
+    const int rows = slabs ? kSlab : m * int(sizeof(V)) > 64 ? kOrderWideRows : kOrderRows;
     const int step_j = 32 / m, step_r = 32 % m;
     for (long long base = ((long long)c * kPassWarps + warp) * rows; base < n;
          base += (long long)blocks * kPassWarps * rows) {
@@ -158,34 +158,42 @@ scatter_passes_kernel(const V* __restrict__ src, const int* __restrict__ idx, V*
     int* to = s_to[warp];
     const unsigned long long pol = l2_evict_first_policy();
     const int step_j = 32 / m, step_r = 32 % m;
-    if (sample.local(int(row)) || spanned * row <= kPlainScatterBytes) {
+    unsigned lo = 0, rows = plan.bound, c;
+    if (sample.mostly_skipped(plan.bound)) {
+        // One pass over everything, by lists of the valid rows: the source of the others
+        // is not read (2^22 rows of 80 bytes, nine in ten skipped: 58 us, 84 where it is).
+        const unsigned each = sizeof(V) > 4 ? plan.passes : 1u;
+        c = blockIdx.x / each;
+        if (c * each != blockIdx.x || c >= plan.body) return;
+    } else if (sample.local(int(row)) || spanned * row <= kPlainScatterBytes) {
         scatter_in_order<V, G>(src, idx, dst, n, m, plan, to, pol, lane, warp);
         return;
-    }
-    const unsigned pass = blockIdx.x / (plan.fetch + plan.body);
-    unsigned c = blockIdx.x - pass * (plan.fetch + plan.body);
-    unsigned passes = plan.passes, step = plan.rows_per_pass;
-    if (spanned < plan.bound / 4 * 3) {
-        // All of the sample within three quarters of the destination (of 64 rows at
-        // random, one time in a million): as many parts as those rows need, the
-        // outer ones with what lies outside.
-        passes = (spanned + plan.rows_per_pass - 1) / plan.rows_per_pass;
-        if (pass >= passes) return;
-        step = (spanned + passes - 1) / passes;
     } else {
-        first = 0;
+        const unsigned pass = blockIdx.x / (plan.fetch + plan.body);
+        c = blockIdx.x - pass * (plan.fetch + plan.body);
+        unsigned passes = plan.passes, step = plan.rows_per_pass;
+        if (spanned < plan.bound / 4 * 3) {
+            // All of the sample within three quarters of the destination (of 64 rows at
+            // random, one time in a million): as many parts as those rows need, the
+            // outer ones with what lies outside.
+            passes = (spanned + plan.rows_per_pass - 1) / plan.rows_per_pass;
+            if (pass >= passes) return;
+            step = (spanned + passes - 1) / passes;
+        } else {
+            first = 0;
+        }
+        lo = first + pass * step;
+        unsigned end = plan.bound - lo < step ? plan.bound : lo + step;
+        if (c < plan.fetch) {
+            const unsigned long long p = reinterpret_cast<unsigned long long>(dst);
+            fetch_part(p + lo * row, p + end * row, c, plan.fetch);
+            return;
+        }
+        if (pass == 0) lo = 0;
+        if (pass == passes - 1) end = plan.bound;
+        rows = end - lo;
+        c -= plan.fetch;
     }
-    unsigned lo = first + pass * step;
-    unsigned end = plan.bound - lo < step ? plan.bound : lo + step;
-    if (c < plan.fetch) {
-        const unsigned long long p = reinterpret_cast<unsigned long long>(dst);
-        fetch_part(p + lo * row, p + end * row, c, plan.fetch);
-        return;
-    }
-    if (pass == 0) lo = 0;
-    if (pass == passes - 1) end = plan.bound;
-    const unsigned rows = end - lo;
-    c -= plan.fetch;
     unsigned short* at = s_at[warp];
     for (long long base = ((long long)c * kPassWarps + warp) * kSlab; base < n;
          base += (long long)plan.body * kPassWarps * kSlab) {
