@@ -12,8 +12,8 @@
 //
 // One thread per row moving bytes was bound by its load / store instructions,
 // each touching 32 rows: 2^22 rows of 13 bytes, gather 153 us (10 % of DRAM's
-// rate) -> 46, scatter 446 -> 113; of 47 bytes 1252 -> 137 and 1604 -> 252.
-// What is left is the instructions of the joins, about 30 a word.
+// rate) -> 45, scatter 435 -> 114; of 47 bytes 1235 -> 138 and 1567 -> 267.
+// What is left is the instructions of the joins, about 80 for a warp's 32 words.
 #include <cuda_runtime.h>
 #include <stdint.h>
 

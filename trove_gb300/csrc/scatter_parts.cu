@@ -1,7 +1,7 @@
 // Scatters onto large destinations.
 //
 // A row that does not fill whole 32-byte sectors is a partial-sector write.
-// Scattered over a destination of more than about 22 MiB, each one makes L2
+// Scattered over a destination that L2 does not hold yet, each one makes L2
 // fill the rest of its sector from DRAM at the rate of random accesses, and
 // over one larger than L2 the sector leaves before its other rows arrive and
 // is filled and written again.  Two remedies:
@@ -73,9 +73,9 @@ fetch_destination_kernel(const unsigned char* dst, unsigned bound, const int* __
 // to leave L2, which keeps the part being written.
 //
 // Bound by DRAM: 2^24 random rows of 12 bytes in four passes move about 1.35 GB
-// in 233 us (one pass of the row-form kernel 544 us, three passes of it over
-// 64 MiB parts 380 us); of 24 bytes 406 us (one pass 717), of 48 bytes 682 us
-// (1147), of 60 bytes 916 us (1358).
+// in 230 us (one pass of the row-form kernel 544 us, three passes of it over
+// 64 MiB parts 380 us); of 24 bytes 406 us (one pass 717), of 48 bytes 680 us
+// (1143), of 60 bytes 888 us (1509).
 constexpr int kPassWarps = 8;
 
 struct PassPlan {
